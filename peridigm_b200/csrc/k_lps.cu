@@ -29,6 +29,7 @@
 
 #include <cub/cub.cuh>
 
+#include "fp64_math.cuh"
 #include "pd_internal.cuh"
 
 namespace pdb {
@@ -655,13 +656,46 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
 // K2: damage + dilatation, FP64, the reference's operation order:
 //   rel = (|Y|-|X|)/|X| > s_c                     (CriticalStretchDamageModel.cpp:147-158)
 //   theta += 3*omega*(1-d)*|X|*e*V_j/m_i           (material_utilities.cxx:284)
-// Writes ab64[i] = (theta, 3K/m - alpha/3, alpha) (elastic.cxx:99,119).
+// Writes ab64[i] = (theta, q = 3K/m - alpha/3, alpha, theta*q) (elastic.cxx:99,119).
 // ---------------------------------------------------------------------------
-template <int TPO>
-__global__ void __launch_bounds__(kBlock) k_dilatation_fp64(
+//
+// A lane takes its bonds a batch at a time: loads, gathers, then straight-line
+// arithmetic (fp64_math.cuh) with broken and absent bonds masked. The
+// quotients and roots round as the reference's do (results bit for bit those
+// of the built-in functions). One rare branch redoes a batch with the built-in
+// functions (operands out of range); another runs the break test, only for
+// batches with a bond past s_gate = s_min (1 - 1e-12), below every critical
+// stretch of the body by more than the roundings of the comparison.
+// Bound: latency of the gathers (64 B per bond here, 80 B in the force pass)
+// and of the FP64 chains, so resident warps count for more than bonds in
+// flight per lane: one bond per batch and 4 blocks per SM (64 registers) is the
+// fastest. 131x97x21 points, 27.5 M bonds: dilatation 318 -> 230 us, force
+// 522 -> 293 us (2 bonds per batch 248 and 399 us; 5 blocks 255 and 396 us).
+#ifndef PD_F64_DIL_BATCH
+#define PD_F64_DIL_BATCH 1
+#endif
+#ifndef PD_F64_FORCE_BATCH
+#define PD_F64_FORCE_BATCH 1
+#endif
+#ifndef PD_F64_DIL_MINB
+#define PD_F64_DIL_MINB 4
+#endif
+#ifndef PD_F64_FORCE_MINB
+#define PD_F64_FORCE_MINB 4
+#endif
+
+// 32-byte record of a point (read-only during the pass).
+__device__ __forceinline__ double4 ld_f64x4_nc(const double4* p) {
+  double4 r;
+  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+
+template <int TPO, bool ONE>
+__global__ void __launch_bounds__(kBlock, PD_F64_DIL_MINB) k_dilatation_fp64(
     int64_t n, const int64_t* __restrict__ row, const int32_t* __restrict__ col, uint8_t* __restrict__ dmg,
     const double4* __restrict__ xv, const double4* __restrict__ st, const double4* __restrict__ pt,
-    const double* __restrict__ sc, const double* __restrict__ hp, int influence, int damage_on,
+    const double* __restrict__ sc, const double* __restrict__ hp, int influence, int damage_on, double s_gate,
     double4* __restrict__ ab64, double* __restrict__ theta_out, double* __restrict__ node_damage, int pair) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = g / TPO;
@@ -670,45 +704,84 @@ __global__ void __launch_bounds__(kBlock) k_dilatation_fp64(
   double th = 0.0;
   int broken = 0;
   int64_t b0 = 0, b1 = 0;
-  double m = 1.0;
   if (valid) {
     b0 = row[i];
     b1 = row[i + 1];
     const double4 xi = xv[i];
     const double4 yi = st[i];
-    m = pt[i].x;
+    const double m = pt[i].x;
+    const bool m_in = root_in_range(m);  // m and 1/m far from the ends of the range
+    const double rm = __drcp_rn(m);
     const double s_c = damage_on ? sc[i] : -1.0;
+    const double gate = damage_on ? s_gate : INFINITY;
     const double h = hp[i];
-    for (int64_t b = b0 + lane; b < b1; b += TPO) {
-      const int d = dmg[b];  // bit 0: this half broken, bit 1: the partner's half
-      if ((d & 3) == 3) {
-        broken++;
-        continue;
+    constexpr int K = PD_F64_DIL_BATCH;
+    int dn[K];  // bit 0: this half broken, bit 1: the partner's half
+    int32_t jn[K];
+    auto next = [&](int64_t b) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const bool in = b + k * TPO < b1;
+        dn[k] = in ? dmg[b + k * TPO] : kDummyBond | 3;
+        jn[k] = in ? col[b + k * TPO] : (int32_t)i;
       }
-      const int32_t j = col[b];
-      const double4 xj = xv[j];
-      const double4 yj = st[j];
-      const double zeta = __dsqrt_rn(sq3_rn(__dsub_rn(xj.x, xi.x), __dsub_rn(xj.y, xi.y), __dsub_rn(xj.z, xi.z)));
-      const double dY = __dsqrt_rn(sq3_rn(__dsub_rn(yj.x, yi.x), __dsub_rn(yj.y, yi.y), __dsub_rn(yj.z, yi.z)));
-      // this half's test with s_c,i; the partner's with s_c,j (the same test
-      // on both halves when the critical stretch is one along every bond)
-      const double scj = pair && damage_on ? sc[j] : s_c;
-      bool brk = false, brkp = false;
-      if ((s_c >= 0.0 && !(d & 1)) || (scj >= 0.0 && !(d & 2))) {
-        const double rel = __ddiv_rn(__dsub_rn(dY, zeta), zeta);
-        brk = !(d & 1) && s_c >= 0.0 && rel > s_c;
-        brkp = !(d & 2) && scj >= 0.0 && rel > scj;
+    };
+    next(b0 + lane);
+    for (int64_t b = b0 + lane; b < b1; b += K * TPO) {
+      int d[K];
+      int32_t j[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) d[k] = dn[k], j[k] = jn[k];
+      next(b + K * TPO);
+      double4 xj[K], yj[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) xj[k] = ld_f64x4_nc(xv + j[k]), yj[k] = ld_f64x4_nc(st + j[k]);
+      double zz[K], yy[K], zeta[K], e[K], q[K];
+      auto term = [&](double zt, double ex, double V) {  // 3.0*omega*(1.0-d)*d*e*cellVolume with d = 0
+        const double om3 = ONE ? 3.0 : __dmul_rn(3.0, omega_d(influence, zt, h));
+        return __dmul_rn(__dmul_rn(__dmul_rn(om3, zt), ex), V);
+      };
+      bool odd = !m_in, hot = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const bool live = (d[k] & 3) != 3;
+        const double z2 = sq3_rn(__dsub_rn(xj[k].x, xi.x), __dsub_rn(xj[k].y, xi.y), __dsub_rn(xj[k].z, xi.z));
+        const double y2 = sq3_rn(__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z));
+        zz[k] = live ? z2 : 1.0;
+        yy[k] = live ? y2 : 1.0;
+        zeta[k] = root_d(zz[k]).root;
+        e[k] = __dsub_rn(root_d(yy[k]).root, zeta[k]);
+        q[k] = quotient_d(term(zeta[k], e[k], xj[k].w), m, rm);
+        odd |= !root_in_range(zz[k]) || !root_in_range(yy[k]);
       }
-      if (brk || brkp) dmg[b] = (uint8_t)(d | (brk ? 1 : 0) | (brkp ? 2 : 0));
-      if ((d & 1) || brk) {
-        broken++;
-        continue;
+      if (odd)
+        for (int k = 0; k < K; ++k) {
+          zeta[k] = __dsqrt_rn(zz[k]);
+          e[k] = __dsub_rn(__dsqrt_rn(yy[k]), zeta[k]);
+          q[k] = __ddiv_rn(term(zeta[k], e[k], xj[k].w), m);
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) hot |= e[k] > gate * zeta[k];
+      if (hot)
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          // this half's test with s_c,i; the partner's with s_c,j (the same test
+          // on both halves when the critical stretch is one along every bond)
+          if ((d[k] & 3) == 3) continue;
+          const double scj = pair ? sc[j[k]] : s_c;
+          const double rel = __ddiv_rn(e[k], zeta[k]);
+          const bool brk = !(d[k] & 1) && s_c >= 0.0 && rel > s_c;
+          const bool brkp = !(d[k] & 2) && scj >= 0.0 && rel > scj;
+          if (brk || brkp) {
+            d[k] |= (brk ? 1 : 0) | (brkp ? 2 : 0);
+            dmg[b + k * TPO] = (uint8_t)d[k];
+          }
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        broken += (d[k] & (kDummyBond | 1)) == 1 ? 1 : 0;
+        if (!(d[k] & 1)) th = __dadd_rn(th, q[k]);
       }
-      const double e = __dsub_rn(dY, zeta);
-      const double om = omega_d(influence, zeta, h);
-      // 3.0*omega*(1.0-d)*d*e*cellVolume/m with d = 0
-      double t = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(3.0, om), zeta), e), xj.w);
-      th = __dadd_rn(th, __ddiv_rn(t, m));
     }
   }
   th = group_sum<TPO>(th);
@@ -717,7 +790,7 @@ __global__ void __launch_bounds__(kBlock) k_dilatation_fp64(
     const double4 p = pt[i];
     const double alpha = __ddiv_rn(__dmul_rn(15.0, p.z), p.x);
     const double q = __dsub_rn(__ddiv_rn(__dmul_rn(3.0, p.y), p.x), __ddiv_rn(alpha, 3.0));
-    ab64[i] = make_double4(th, q, alpha, 0.0);
+    ab64[i] = make_double4(th, q, alpha, __dmul_rn(th, q));
     theta_out[i] = th;
     node_damage[i] = (b1 > b0) ? (double)broken / (double)(b1 - b0) : 0.0;
   }
@@ -903,8 +976,9 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_BOND_MINB) k_forc
 //   own term  +  (t_ij*Y)/|Y| * V_j      (elastic.cxx:121-127)
 //   neighbor  -  (t_ji*(-Y))/|Y| * V_j   (elastic.cxx:128-130 from j's loop)
 // ---------------------------------------------------------------------------
-template <int TPO>
-__global__ void __launch_bounds__(kBlock) k_force_fp64(int64_t n, const int64_t* __restrict__ row,
+// Batches as in k_dilatation_fp64; the six quotients of a bond share 1/|Y|.
+template <int TPO, bool ONE>
+__global__ void __launch_bounds__(kBlock, PD_F64_FORCE_MINB) k_force_fp64(int64_t n, const int64_t* __restrict__ row,
                                                        const int32_t* __restrict__ col,
                                                        const uint8_t* __restrict__ dmg,
                                                        const double4* __restrict__ xv,
@@ -922,36 +996,79 @@ __global__ void __launch_bounds__(kBlock) k_force_fp64(int64_t n, const int64_t*
   if (valid) {
     xi = xv[i];
     const double4 yi = st[i];
-    const double4 ai = ab64[i];  // (theta, q, alpha)
+    const double4 ai = ab64[i];  // (theta, q, alpha, theta*q)
     const double hi = hp[i];
     const int64_t b1 = row[i + 1];
-    for (int64_t b = row[i] + lane; b < b1; b += TPO) {
-      const int d = dmg[b];  // bit 0: t_ij's half broken, bit 1: t_ji's
-      if ((d & 3) == 3) continue;
-      const int32_t j = col[b];
-      const double4 xj = xv[j];
-      const double4 yj = st[j];
-      const double4 aj = ab64[j];
-      const double zeta = __dsqrt_rn(sq3_rn(__dsub_rn(xj.x, xi.x), __dsub_rn(xj.y, xi.y), __dsub_rn(xj.z, xi.z)));
-      const double Yx = __dsub_rn(yj.x, yi.x), Yy = __dsub_rn(yj.y, yi.y), Yz = __dsub_rn(yj.z, yi.z);
-      const double dY = __dsqrt_rn(sq3_rn(Yx, Yy, Yz));
-      const double e = __dsub_rn(dY, zeta);
-      const double om_i = omega_d(influence, zeta, hi);
-      const double om_j = influence == PD_INFLUENCE_ONE ? 1.0 : omega_d(influence, zeta, hp[j]);
-      const double ti = __dadd_rn(__dmul_rn(__dmul_rn(__dmul_rn(om_i, ai.x), ai.y), zeta),
-                                  __dmul_rn(__dmul_rn(om_i, ai.z), e));
-      const double tj = __dadd_rn(__dmul_rn(__dmul_rn(__dmul_rn(om_j, aj.x), aj.y), zeta),
-                                  __dmul_rn(__dmul_rn(om_j, aj.z), e));
-      const double V = xj.w;
-      if (!(d & 1)) {
-        fx = __dadd_rn(fx, __dmul_rn(__ddiv_rn(__dmul_rn(ti, Yx), dY), V));
-        fy = __dadd_rn(fy, __dmul_rn(__ddiv_rn(__dmul_rn(ti, Yy), dY), V));
-        fz = __dadd_rn(fz, __dmul_rn(__ddiv_rn(__dmul_rn(ti, Yz), dY), V));
+    constexpr int K = PD_F64_FORCE_BATCH;
+    for (int64_t b = row[i] + lane; b < b1; b += K * TPO) {
+      int d[K];  // bit 0: t_ij's half broken, bit 1: t_ji's
+      int32_t j[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const bool in = b + k * TPO < b1;
+        d[k] = in ? dmg[b + k * TPO] & 3 : 3;
+        j[k] = in ? col[b + k * TPO] : (int32_t)i;
       }
-      if (!(d & 2)) {
-        fx = __dsub_rn(fx, __dmul_rn(__ddiv_rn(__dmul_rn(tj, -Yx), dY), V));
-        fy = __dsub_rn(fy, __dmul_rn(__ddiv_rn(__dmul_rn(tj, -Yy), dY), V));
-        fz = __dsub_rn(fz, __dmul_rn(__ddiv_rn(__dmul_rn(tj, -Yz), dY), V));
+      double4 xj[K], yj[K], aj[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        xj[k] = ld_f64x4_nc(xv + j[k]), yj[k] = ld_f64x4_nc(st + j[k]);
+        if (ONE) {  // with omega = 1 the products theta*q of the points are the bond's
+          const double2 a = __ldg(reinterpret_cast<const double2*>(ab64 + j[k]) + 1);
+          aj[k] = make_double4(0.0, 0.0, a.x, a.y);
+        } else {
+          aj[k] = ld_f64x4_nc(ab64 + j[k]);
+        }
+      }
+      double zz[K], yy[K];
+      double fi[K][3], fj[K][3];  // (t Y)/|Y| of the two halves
+      auto state = [&](const double4& a, double om, double zeta, double e) {
+        return ONE ? __dadd_rn(__dmul_rn(a.w, zeta), __dmul_rn(a.z, e))
+                   : __dadd_rn(__dmul_rn(__dmul_rn(__dmul_rn(om, a.x), a.y), zeta), __dmul_rn(__dmul_rn(om, a.z), e));
+      };
+      auto om_i = [&](double zeta) { return ONE ? 1.0 : omega_d(influence, zeta, hi); };
+      auto om_j = [&](int k, double zeta) { return ONE ? 1.0 : omega_d(influence, zeta, hp[j[k]]); };
+      bool odd = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double Y[3] = {__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z)};
+        const double z2 = sq3_rn(__dsub_rn(xj[k].x, xi.x), __dsub_rn(xj[k].y, xi.y), __dsub_rn(xj[k].z, xi.z));
+        const double y2 = sq3_rn(Y[0], Y[1], Y[2]);
+        zz[k] = d[k] != 3 ? z2 : 1.0;
+        yy[k] = d[k] != 3 ? y2 : 1.0;
+        odd |= !root_in_range(zz[k]) || !root_in_range(yy[k]);
+        const RootD r = root_d(yy[k]);
+        const double zeta = root_d(zz[k]).root, e = __dsub_rn(r.root, zeta), rd = recip_d(r.root, r.inv);
+        const double ti = state(ai, om_i(zeta), zeta, e), tj = state(aj[k], om_j(k, zeta), zeta, e);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          fi[k][c] = quotient_d(__dmul_rn(ti, Y[c]), r.root, rd);
+          fj[k][c] = quotient_d(__dmul_rn(tj, Y[c]), r.root, rd);
+        }
+      }
+      if (odd)
+        for (int k = 0; k < K; ++k) {
+          const double Y[3] = {__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z)};
+          const double zeta = __dsqrt_rn(zz[k]), dY = __dsqrt_rn(yy[k]), e = __dsub_rn(dY, zeta);
+          const double ti = state(ai, om_i(zeta), zeta, e), tj = state(aj[k], om_j(k, zeta), zeta, e);
+          for (int c = 0; c < 3; ++c) {
+            fi[k][c] = __ddiv_rn(__dmul_rn(ti, Y[c]), dY);
+            fj[k][c] = __ddiv_rn(__dmul_rn(tj, Y[c]), dY);
+          }
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double V = xj[k].w;
+        if (!(d[k] & 1)) {
+          fx = __dadd_rn(fx, __dmul_rn(fi[k][0], V));
+          fy = __dadd_rn(fy, __dmul_rn(fi[k][1], V));
+          fz = __dadd_rn(fz, __dmul_rn(fi[k][2], V));
+        }
+        if (!(d[k] & 2)) {  // - (t_ji*(-Y))/|Y| * V_j, the signs folded (exact)
+          fx = __dadd_rn(fx, __dmul_rn(fj[k][0], V));
+          fy = __dadd_rn(fy, __dmul_rn(fj[k][1], V));
+          fz = __dadd_rn(fz, __dmul_rn(fj[k][2], V));
+        }
       }
     }
   }
@@ -979,20 +1096,23 @@ __global__ void __launch_bounds__(kBlock) k_force_fp64(int64_t n, const int64_t*
 __device__ __forceinline__ void ldcs_f64x4(const double* p, double* o) {
   asm("ld.global.cs.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p));
 }
-// 32-byte record of a point (read-only during the pass).
-__device__ __forceinline__ double4 ld_f64x4_nc(const double4* p) {
-  double4 r;
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
-  return r;
-}
 __device__ __forceinline__ double2 ld_f64x2_nc(const double4* p) {
   return __ldg(reinterpret_cast<const double2*>(p));
 }
 
 // Walks lane `lane` of owner i through its bonds of the sliced stream (the
-// order of sell_walk): body(X0, X1, X2, damage byte, neighbor (y, V),
-// neighbor (A, B) (zeros unless AB), the bond's damage byte in the stream,
-// row offset r - lane).
+// order of sell_walk), PD_F64S_BATCH (full blocks) or three (the tail) bonds
+// to a call: body(count, X planes, damage bytes, neighbors' (y, V), neighbors'
+// (A, B) (zeros unless AB), the first bond's damage byte in the stream, the
+// step to the next, the first bond's row offset r - lane, that of the next
+// being 4 more).
+#ifndef PD_F64S_BATCH
+#define PD_F64S_BATCH 4
+#endif
+template <int K>
+struct Count {
+  static constexpr int value = K;
+};
 template <bool AB, typename Body>
 __device__ __forceinline__ void sell_walk64(int64_t i, int lane, const int64_t* __restrict__ soff,
                                             const int32_t* __restrict__ col, uint8_t* __restrict__ dmg,
@@ -1016,41 +1136,58 @@ __device__ __forceinline__ void sell_walk64(int64_t i, int lane, const int64_t* 
     ldcs_f64x4(px + 256, X2);
     double4 yj[4];
     double2 aj[4];
+    int d[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       yj[k] = ld_f64x4_nc(st + jv[k]);
       aj[k] = AB ? ld_f64x2_nc(ab + jv[k]) : make_double2(0.0, 0.0);
+      d[k] = (int)((dw >> (8 * k)) & 0xffu);
     }
     uint8_t* pb = reinterpret_cast<uint8_t*>(pd);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) body(X0[k], X1[k], X2[k], (int)((dw >> (8 * k)) & 0xffu), yj[k], aj[k], pb + k, 16 * b + 4 * k);
+    for (int k = 0; k < 4; k += PD_F64S_BATCH)
+      body(Count<PD_F64S_BATCH>(), X0 + k, X1 + k, X2 + k, d + k, yj + k, aj + k, pb + k, 1, 16 * b + 4 * k);
   }
   const int T = G - 4 * F;
   if (T > 0) {  // tail groups: masked, one slot per lane per group
     const int64_t t0 = 32 * (so + 4 * F) + l32;
     const double* pt = bx + 96 * (so + 4 * F) + l32;
+    double X0[3], X1[3], X2[3];
+    double4 yj[3];
+    double2 aj[3];
+    int d[3], j[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const bool in = k < T;
-      const int32_t j = in ? __ldcs(col + t0 + 32 * k) : (int32_t)i;
-      const int d = in ? (int)dmg[t0 + 32 * k] : kDummyBond;
-      const double X0 = in ? __ldcs(pt + 96 * k) : 1.0;
-      const double X1 = in ? __ldcs(pt + 96 * k + 32) : 0.0;
-      const double X2 = in ? __ldcs(pt + 96 * k + 64) : 0.0;
-      const double4 yj = ld_f64x4_nc(st + j);
-      const double2 aj = AB ? ld_f64x2_nc(ab + j) : make_double2(0.0, 0.0);
-      body(X0, X1, X2, d, yj, aj, dmg + t0 + 32 * k, 16 * F + 4 * k);
+      j[k] = in ? __ldcs(col + t0 + 32 * k) : (int32_t)i;
+      d[k] = in ? (int)dmg[t0 + 32 * k] : kDummyBond;
+      X0[k] = in ? __ldcs(pt + 96 * k) : 1.0;
+      X1[k] = in ? __ldcs(pt + 96 * k + 32) : 0.0;
+      X2[k] = in ? __ldcs(pt + 96 * k + 64) : 0.0;
     }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      yj[k] = ld_f64x4_nc(st + j[k]);
+      aj[k] = AB ? ld_f64x2_nc(ab + j[k]) : make_double2(0.0, 0.0);
+    }
+    body(Count<3>(), X0, X1, X2, d, yj, aj, dmg + t0, 32, 16 * F);
   }
 }
 
 // Damage + dilatation. The break test is the reference's
 // rel = (|Y| - |X|)/|X| > s_c (CriticalStretchDamageModel.cpp:155-158), run
-// only for bonds with e > s_gate |X|, s_gate = s_min (1 - 1e-12) below every
-// critical stretch of the body by more than the roundings of e/|X| and
-// s_gate |X|, so that no bond the reference breaks skips it.
+// only for batches with a bond of e > s_gate |X|, s_gate = s_min (1 - 1e-12)
+// below every critical stretch of the body by more than the roundings of
+// e/|X| and s_gate |X|, so that no bond the reference breaks skips it. The
+// arithmetic of a batch is straight-line (fp64_math.cuh), out-of-range roots
+// (root_in_range) in one rare branch; a padding slot gathers its own owner
+// (Y = 0) and takes |Y| = 1 there, its terms masked. With the built-in
+// functions' branches gone, the chains of a block's 4 bonds overlap:
+// 160x160x40 points, 109 M bonds, dilatation 869 -> 667 us (5 blocks per SM; 4
+// 728, 6 704), force 938 -> 823 us (4 blocks; 3 902, 5 923); 2 or 1 bonds to a
+// batch are slower in both.
 #ifndef PD_F64S_DIL_MINB
-#define PD_F64S_DIL_MINB 4
+#define PD_F64S_DIL_MINB 5
 #endif
 #ifndef PD_F64S_FORCE_MINB
 #define PD_F64S_FORCE_MINB 4
@@ -1073,36 +1210,57 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
     const int64_t b0 = row[i];
     len = (int)(row[i + 1] - b0);
     const double4 yi = ld_f64x4_nc(st + i);
-    const double s_c = damage_on ? sc[i] : -1.0;
+    const double gate = damage_on ? s_gate : INFINITY;
     uint8_t* cdm = dmg_csr + b0 + lane;  // the lane's bonds in the canonical CSR damage
-    auto body = [&](double X0, double X1, double X2, int d, const double4& yj, const double2&, uint8_t* pdm,
-                    int r) {
+    auto body = [&](auto count, const double* X0, const double* X1, const double* X2, int* d, const double4* yj,
+                    const double2*, uint8_t* pdm, int step, int r) {
+      constexpr int K = decltype(count)::value;
       // |X|, |Y| and e in the reference's operation order: the break test
       // sees the reference's stretch bit for bit
-      const double Yx = __dsub_rn(yj.x, yi.x), Yy = __dsub_rn(yj.y, yi.y), Yz = __dsub_rn(yj.z, yi.z);
-      const double zeta = __dsqrt_rn(sq3_rn(X0, X1, X2));
-      const double e = __dsub_rn(__dsqrt_rn(sq3_rn(Yx, Yy, Yz)), zeta);
-      const bool own_ok = (d & 5) == 0;  // own half intact (and a real bond)
-      bool brk = false, brkp = false;
-      if (damage_on && e > s_gate * zeta) {
-        const double rel = __ddiv_rn(e, zeta);
-        brk = own_ok && s_c >= 0.0 && rel > s_c;
-        if (PAIR) {
-          if ((d & 6) == 0) {
-            const double scj = __ldg(sc + __ldg(col + (pdm - dmg)));
-            brkp = scj >= 0.0 && rel > scj;
+      double zz[K], yy[K], zeta[K], e[K];
+      bool odd = false, hot = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double y2 = sq3_rn(__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z));
+        zz[k] = sq3_rn(X0[k], X1[k], X2[k]);
+        yy[k] = (d[k] & kDummyBond) ? 1.0 : y2;
+        zeta[k] = root_d(zz[k]).root;
+        e[k] = __dsub_rn(root_d(yy[k]).root, zeta[k]);
+        odd |= !root_in_range(zz[k]) || !root_in_range(yy[k]);
+      }
+      if (odd)
+        for (int k = 0; k < K; ++k) {
+          zeta[k] = __dsqrt_rn(zz[k]);
+          e[k] = __dsub_rn(__dsqrt_rn(yy[k]), zeta[k]);
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) hot |= e[k] > gate * zeta[k];
+      if (hot) {
+        const double s_c = sc[i];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const double rel = __ddiv_rn(e[k], zeta[k]);
+          const bool brk = (d[k] & 5) == 0 && s_c >= 0.0 && rel > s_c;
+          bool brkp = brk;
+          if (PAIR) {
+            brkp = false;
+            if ((d[k] & 6) == 0) {
+              const double scj = __ldg(sc + __ldg(col + (pdm + k * step - dmg)));
+              brkp = scj >= 0.0 && rel > scj;
+            }
           }
-        } else {
-          brkp = brk;
+          if (brk || brkp) {
+            d[k] |= (brk ? 1 : 0) | (brkp ? 2 : 0);
+            pdm[k * step] = (uint8_t)d[k];
+            cdm[r + 4 * k] = (uint8_t)d[k];  // the CSR copy stays canonical
+          }
         }
       }
-      if (brk || brkp) {
-        const uint8_t nd = (uint8_t)(d | (brk ? 1 : 0) | (brkp ? 2 : 0));
-        *pdm = nd;
-        cdm[r] = nd;  // the CSR copy stays canonical
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        broken += d[k] & 1;
+        th = fma((d[k] & 5) == 0 ? yj[k].w * zeta[k] : 0.0, e[k], th);  // V_j |X| e
       }
-      broken += ((d & 1) || brk) ? 1 : 0;
-      th = fma((own_ok && !brk) ? yj.w * zeta : 0.0, e, th);  // V_j |X| e
     };
     sell_walk64<false>(i, lane, soff, col, dmg, bx, st, nullptr, body);
   }
@@ -1141,22 +1299,37 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_FORCE_MINB) k_force_f64s(
   if (valid) {
     const double4 yi = ld_f64x4_nc(st + i);
     const double2 ai = ld_f64x2_nc(ab64 + i);
-    auto body = [&](double X0, double X1, double X2, int d, const double4& yj, const double2& aj, uint8_t*, int) {
-      const double Yx = __dsub_rn(yj.x, yi.x), Yy = __dsub_rn(yj.y, yi.y), Yz = __dsub_rn(yj.z, yi.z);
-      const double zeta = __dsqrt_rn(sq3_rn(X0, X1, X2));
-      const double dY = __dsqrt_rn(sq3_rn(Yx, Yy, Yz));
-      const double e = __dsub_rn(dY, zeta);
-      double a = ai.x + aj.x, b = ai.y + aj.y;
-      if (d != 0) {  // a broken half or a padding slot (both intact is the common case)
-        const bool own_live = (d & 5) == 0, part_live = PAIR ? (d & 6) == 0 : own_live;
-        a = (own_live ? ai.x : 0.0) + (part_live ? aj.x : 0.0);
-        b = (own_live ? ai.y : 0.0) + (part_live ? aj.y : 0.0);
+    auto body = [&](auto count, const double* X0, const double* X1, const double* X2, const int* d, const double4* yj,
+                    const double2* aj, uint8_t*, int, int) {
+      constexpr int K = decltype(count)::value;
+      double zz[K], yy[K], w[K];
+      auto weight = [&](int k, double zeta, double dY) {  // V_j (t_ij + t_ji) of the intact halves
+        const bool own_live = (d[k] & 5) == 0, part_live = PAIR ? (d[k] & 6) == 0 : own_live;
+        const double a = (own_live ? ai.x : 0.0) + (part_live ? aj[k].x : 0.0);
+        const double b = (own_live ? ai.y : 0.0) + (part_live ? aj[k].y : 0.0);
+        return fma(zeta, a, __dsub_rn(dY, zeta) * b) * yj[k].w;
+      };
+      bool odd = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double y2 = sq3_rn(__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z));
+        zz[k] = sq3_rn(X0[k], X1[k], X2[k]);
+        yy[k] = (d[k] & kDummyBond) ? 1.0 : y2;
+        odd |= !root_in_range(zz[k]) || !root_in_range(yy[k]);
+        const RootD ry = root_d(yy[k]);
+        w[k] = quotient_d(weight(k, root_d(zz[k]).root, ry.root), ry.root, recip_d(ry.root, ry.inv));
       }
-      // a padding slot gathers its own owner (Y = 0): no term, and no 0/0
-      const double w = (d & kDummyBond) ? 0.0 : fma(zeta, a, e * b) * yj.w / dY;
-      fx = fma(w, Yx, fx);
-      fy = fma(w, Yy, fy);
-      fz = fma(w, Yz, fz);
+      if (odd)
+        for (int k = 0; k < K; ++k) {
+          const double dY = __dsqrt_rn(yy[k]);
+          w[k] = weight(k, __dsqrt_rn(zz[k]), dY) / dY;
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        fx = fma(w[k], __dsub_rn(yj[k].x, yi.x), fx);
+        fy = fma(w[k], __dsub_rn(yj[k].y, yi.y), fy);
+        fz = fma(w[k], __dsub_rn(yj[k].z, yi.z), fz);
+      }
     };
     uint8_t* dm = const_cast<uint8_t*>(dmg);  // not written by this pass
     sell_walk64<true>(i, lane, soff, col, dm, bx, st, ab64, body);
@@ -1624,6 +1797,23 @@ static inline unsigned grid_split(int64_t n, int tpo) {
     default: KERNEL<32, false><<<GRID, BLOCK, 0, c->stream>>>(__VA_ARGS__); break;   \
   }
 
+#define PD_DISPATCH_TPO_ONE(tpo, KERNEL, GRID, ...)                                  \
+  if (c->influence == PD_INFLUENCE_ONE) {                                            \
+    switch (tpo) {                                                                   \
+      case 4: KERNEL<4, true><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break;   \
+      case 8: KERNEL<8, true><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break;   \
+      case 16: KERNEL<16, true><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break; \
+      default: KERNEL<32, true><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break; \
+    }                                                                                \
+  } else {                                                                           \
+    switch (tpo) {                                                                   \
+      case 4: KERNEL<4, false><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break;  \
+      case 8: KERNEL<8, false><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break;  \
+      case 16: KERNEL<16, false><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break; \
+      default: KERNEL<32, false><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break; \
+    }                                                                                \
+  }
+
 #define PD_DISPATCH_TPO(tpo, KERNEL, GRID, ...)                                      \
   switch (tpo) {                                                                     \
     case 4: KERNEL<4><<<GRID, kBlock, 0, c->stream>>>(__VA_ARGS__); break;           \
@@ -2004,8 +2194,8 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
                     c->pt.p, c->sc.p, c->hp.p, c->influence, sp.damage_on, c->ab64.p, c->theta.p, c->node_damage.p,
                     ipair);
   } else {
-    PD_DISPATCH_TPO(tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->pt.p,
-                    c->sc.p, c->hp.p, c->influence, sp.damage_on, c->ab64.p, c->theta.p, c->node_damage.p, ipair);
+    PD_DISPATCH_TPO_ONE(tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->pt.p,
+                    c->sc.p, c->hp.p, c->influence, sp.damage_on, c->sc_gate64, c->ab64.p, c->theta.p, c->node_damage.p, ipair);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -2048,7 +2238,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
     PD_DISPATCH_TPO(tpo, k_force_lin_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->ab64.p,
                     c->pt.p, c->hp.p, c->influence, E);
   } else {
-    PD_DISPATCH_TPO(tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->ab64.p,
+    PD_DISPATCH_TPO_ONE(tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->ab64.p,
                     c->pt.p, c->hp.p, c->influence, E);
   }
   if (ev) cudaEventRecord(ev[2], c->stream);
@@ -2099,15 +2289,15 @@ cudaError_t launch_fp64_eval_at(pd_ctx* c, const double4* y4, double4* ab, doubl
                                 double* f_out) {
   if (c->n == 0) return cudaSuccess;
   const unsigned grid = grid_for(c->n, c->tpo);
-  PD_DISPATCH_TPO(c->tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, c->pt.p,
-                  c->sc.p, c->hp.p, c->influence, 0, ab, theta, nd, 0);
+  PD_DISPATCH_TPO_ONE(c->tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, c->pt.p,
+                      c->sc.p, c->hp.p, c->influence, 0, c->sc_gate64, ab, theta, nd, 0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   EpiArgs E{};
   E.mode = EVAL_ONLY;
   E.f_out = f_out;
   E.status = c->status.p;
-  PD_DISPATCH_TPO(c->tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, ab, c->pt.p, c->hp.p,
+  PD_DISPATCH_TPO_ONE(c->tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, ab, c->pt.p, c->hp.p,
                   c->influence, E);
   return cudaGetLastError();
 }
