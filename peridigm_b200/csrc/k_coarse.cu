@@ -44,6 +44,7 @@
 #include <vector>
 
 #include "cells.cuh"
+#include "cg.cuh"
 #include "pd_internal.cuh"
 
 namespace pdb {
@@ -588,8 +589,10 @@ __global__ void __launch_bounds__(kRestrictT) k_coarse_restrict(int64_t nagg, co
 
 // y = A x with the FP32 copy of the inverse, FP64 products and sums (warp per
 // row, four entries per lane per load: the row's order of terms is fixed).
+// ctl (may be null): a CG solve that has ended makes the kernel return.
 __global__ void k_coarse_gemv_f(int nc, const float* __restrict__ A, const double* __restrict__ x,
-                                double* __restrict__ y) {
+                                double* __restrict__ y, const CgCtl* __restrict__ ctl) {
+  if (ctl && ctl->state) return;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (i >= nc) return;
@@ -836,6 +839,120 @@ __global__ void k_rigid_prolong(int64_t n, const int32_t* __restrict__ agg_of, c
 }
 
 // ---------------------------------------------------------------------------
+// CG iteration with the two-level preconditioner (k_qs.cu): the vector updates
+// ride on the restriction (each point belongs to one aggregate) and the dot
+// products on the prolongation.
+// ---------------------------------------------------------------------------
+// The rigid coarse vector of raw mode sums m (translations, then the rotations
+// about z, x, y): rc = T^T m, the orthonormal modes' products. The sums of an
+// aggregate's points are taken over the raw modes (9 operations per point
+// instead of the 108 of forming the orthonormal modes there).
+template <int MODES, bool FIRST>
+__global__ void __launch_bounds__(kRestrictT) k_cg_restrict(const int32_t* __restrict__ agg_cell,
+                                                            const int64_t* __restrict__ cstart,
+                                                            const int32_t* __restrict__ sorted,
+                                                            const double* __restrict__ center,
+                                                            const double* __restrict__ Tm,
+                                                            const double4* __restrict__ xv, double inv_side,
+                                                            const double4* __restrict__ w,
+                                                            const double* __restrict__ q, double* __restrict__ x,
+                                                            double* __restrict__ r, double* __restrict__ rc,
+                                                            const CgCtl* __restrict__ ctl) {
+  __shared__ double sh[MODES][kRestrictT / 32];
+  if (!FIRST && ctl->state) return;
+  const double alpha = FIRST ? 0.0 : ctl->rz / ctl->pq;
+  const int64_t I = blockIdx.x;
+  const int cell = agg_cell[I];
+  double acc[MODES];
+#pragma unroll
+  for (int k = 0; k < MODES; ++k) acc[k] = 0.0;
+  double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+  if (MODES == 6) c0 = center[4 * I], c1 = center[4 * I + 1], c2 = center[4 * I + 2];
+  for (int64_t t = cstart[cell] + threadIdx.x; t < cstart[cell + 1]; t += kRestrictT) {
+    const int64_t p = sorted[t];
+    double rv[3] = {r[3 * p], r[3 * p + 1], r[3 * p + 2]};
+    if (!FIRST) {
+      const double4 d = w[p];
+      const double dv[3] = {d.x, d.y, d.z};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        rv[k] -= alpha * q[3 * p + k];
+        r[3 * p + k] = rv[k];
+        x[3 * p + k] += alpha * dv[k];
+      }
+    }
+    // (r is zero at prescribed dofs, which no mode moves)
+    acc[0] += rv[0];
+    acc[1] += rv[1];
+    acc[2] += rv[2];
+    if (MODES == 6) {
+      const double4 xp = xv[p];
+      const double d0 = (xp.x - c0) * inv_side, d1 = (xp.y - c1) * inv_side, d2 = (xp.z - c2) * inv_side;
+      acc[3] += d0 * rv[1] - d1 * rv[0];
+      acc[4] += d1 * rv[2] - d2 * rv[1];
+      acc[5] += d2 * rv[0] - d0 * rv[2];
+    }
+  }
+  cg_block_sum<MODES, kRestrictT>(acc, sh);
+  if (MODES == 3) {
+    if (threadIdx.x == 0) rc[3 * I] = acc[0], rc[3 * I + 1] = acc[1], rc[3 * I + 2] = acc[2];
+  } else if (threadIdx.x < 6) {
+    double s = 0.0;
+#pragma unroll
+    for (int l = 0; l < 6; ++l) s += Tm[36 * I + 6 * l + threadIdx.x] * acc[l];
+    rc[6 * I + threadIdx.x] = s;
+  }
+}
+
+// z = P_bj r + P0 zc on the free dofs, r.z and r.r, and the scalars.
+template <int MODES, bool FIRST>
+__global__ void __launch_bounds__(256) k_cg_prolong(int64_t n, const int32_t* __restrict__ agg_of,
+                                                    const double* __restrict__ center, const double* __restrict__ Tm,
+                                                    const double4* __restrict__ xv, double inv_side,
+                                                    const uint8_t* __restrict__ fixed, const double* __restrict__ zc,
+                                                    const double* __restrict__ dinv, const double* __restrict__ r,
+                                                    double* __restrict__ z, double* __restrict__ partial,
+                                                    CgCtl* __restrict__ ctl) {
+  if (!FIRST && ctl->state) return;
+  double s[2] = {0.0, 0.0};
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t I = agg_of[i];
+    const double rv[3] = {r[3 * i], r[3 * i + 1], r[3 * i + 2]};
+    double cv[3];
+    if (MODES == 3) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cv[c] = zc[3 * I + c];
+    } else {
+      double y[6];
+      const double* T = Tm + 36 * I;
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        y[l] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) y[l] += T[6 * l + k] * zc[6 * I + k];
+      }
+      const double4 xp = xv[i];
+      const double d0 = (xp.x - center[4 * I]) * inv_side, d1 = (xp.y - center[4 * I + 1]) * inv_side,
+                   d2 = (xp.z - center[4 * I + 2]) * inv_side;
+      cv[0] = y[0] - d1 * y[3] + d2 * y[5];
+      cv[1] = y[1] + d0 * y[3] - d2 * y[4];
+      cv[2] = y[2] + d1 * y[4] - d0 * y[5];
+    }
+    const uint8_t f = fixed[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double* d = dinv + 9 * i + 3 * c;
+      double zv = d[0] * rv[0] + d[1] * rv[1] + d[2] * rv[2];
+      if (!((f >> c) & 1)) zv += cv[c];
+      z[3 * i + c] = zv;
+      s[0] += rv[c] * zv;
+      s[1] += rv[c] * rv[c];
+    }
+  }
+  if (cg_grid_sum<2, 256>(s, partial, &ctl->ticket[1]) && threadIdx.x == 0) cg_scalars(ctl, s[0], s[1], FIRST);
+}
+
+// ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 static CoarseState* co_state(pd_ctx* c) {
@@ -1030,7 +1147,7 @@ static int co_apply(pd_ctx* c, const T* r, double* z, const uint8_t* fixed, doub
     const double inv_side = 1.0 / s->g.cell;
     k_rigid_restrict<T><<<ga, kRestrictT, 0, c->stream>>>(s->nagg, s->agg_cell.p, s->cstart.p, s->sorted.p,
                                                           s->center.p, s->T.p, c->xv.p, fixed, inv_side, r, s->rc.p);
-    k_coarse_gemv_f<<<gv, 256, 0, c->stream>>>(s->nc, s->Af.p, s->rc.p, s->zc.p);
+    k_coarse_gemv_f<<<gv, 256, 0, c->stream>>>(s->nc, s->Af.p, s->rc.p, s->zc.p, nullptr);
     k_rigid_prolong<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, s->agg_of.p, s->center.p, s->T.p, c->xv.p,
                                                                         fixed, inv_side, s->zc.p, scale, z);
     PD_CUDA_TRY(c, cudaGetLastError());
@@ -1038,7 +1155,7 @@ static int co_apply(pd_ctx* c, const T* r, double* z, const uint8_t* fixed, doub
   }
   k_coarse_restrict<T><<<ga, kRestrictT, 0, c->stream>>>(s->nagg, s->agg_cell.p, s->cstart.p, s->sorted.p, r,
                                                          s->rc.p);
-  k_coarse_gemv_f<<<gv, 256, 0, c->stream>>>(s->nc, s->Af.p, s->rc.p, s->zc.p);
+  k_coarse_gemv_f<<<gv, 256, 0, c->stream>>>(s->nc, s->Af.p, s->rc.p, s->zc.p, nullptr);
   k_coarse_prolong<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, s->agg_of.p, s->zc.p, scale, fixed, z);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;
@@ -1049,6 +1166,33 @@ int coarse_apply_add(pd_ctx* c, const double* r, double* z, const uint8_t* fixed
 }
 int coarse_apply_add_f(pd_ctx* c, const float* r, double* z, const uint8_t* fixed, double scale) {
   return co_apply(c, r, z, fixed, scale);
+}
+
+template <int MODES, bool FIRST>
+static void launch_cg_update(pd_ctx* c, const double4* w, const double* q, double* x, double* r, double* z,
+                             const double* dinv, const uint8_t* fixed, double* partial, CgCtl* ctl, unsigned blocks) {
+  CoarseState* s = c->coarse;
+  const double inv_side = 1.0 / s->g.cell;
+  k_cg_restrict<MODES, FIRST><<<(unsigned)s->nagg, kRestrictT, 0, c->stream>>>(
+      s->agg_cell.p, s->cstart.p, s->sorted.p, s->center.p, s->T.p, c->xv.p, inv_side, w, q, x, r, s->rc.p, ctl);
+  k_coarse_gemv_f<<<(unsigned)(((int64_t)s->nc * 32 + 255) / 256), 256, 0, c->stream>>>(s->nc, s->Af.p, s->rc.p,
+                                                                                        s->zc.p, FIRST ? nullptr : ctl);
+  k_cg_prolong<MODES, FIRST><<<blocks, 256, 0, c->stream>>>(c->n, s->agg_of.p, s->center.p, s->T.p, c->xv.p, inv_side,
+                                                            fixed, s->zc.p, dinv, r, z, partial, ctl);
+}
+
+int coarse_cg_update(pd_ctx* c, const double4* w, const double* q, double* x, double* r, double* z, const double* dinv,
+                     const uint8_t* fixed, double* partial, CgCtl* ctl, bool first, unsigned blocks) {
+  CoarseState* s = c->coarse;
+  if (!s || !s->have_op) {
+    c->err = "coarse operator not built";
+    return PD_ERR_STATE;
+  }
+  auto* f = s->modes == 6 ? (first ? &launch_cg_update<6, true> : &launch_cg_update<6, false>)
+                          : (first ? &launch_cg_update<3, true> : &launch_cg_update<3, false>);
+  f(c, w, q, x, r, z, dinv, fixed, partial, ctl, blocks);
+  PD_CUDA_TRY(c, cudaGetLastError());
+  return PD_OK;
 }
 
 // Aggregate of every point (device, n) of the current coarse space.

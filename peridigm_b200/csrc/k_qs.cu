@@ -27,6 +27,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cg.cuh"
 #include "pd_internal.cuh"
 
 namespace pdb {
@@ -37,6 +38,10 @@ constexpr int kQsTpo = 8;
 #define PD_QS_BATCH 4
 #endif
 constexpr int kQsBatch = PD_QS_BATCH;  // bonds per lane in flight in the tangent passes
+#ifndef PD_QS_WIDE
+#define PD_QS_WIDE 16384
+#endif
+constexpr int64_t kQsWide = PD_QS_WIDE;  // bodies up to this size: 32 lanes per point in the tangent passes
 constexpr int kRedBlocks = 296;  // 2 x 148 SMs: fixed, so reductions are deterministic
 
 struct QsState {
@@ -64,6 +69,12 @@ struct QsState {
   double jk = 1.0, jm = 0.0;
   DBuf<double> v2;  // implicit dynamics: velocity predictor
   DBuf<double> cg_b, cg_x0;  // learned-preconditioner CG: right-hand side and restart point (kept, not reallocated)
+  DBuf<CgCtl> ctl;           // scalars and state of the running solve
+  CgReport* report = nullptr;      // its progress, in mapped pinned memory
+  CgReport* report_dev = nullptr;
+  ~QsState() {
+    if (report) cudaFreeHost(report);
+  }
 };
 
 __device__ __forceinline__ double qs_omega(int kind, double zeta, double h) {
@@ -76,10 +87,10 @@ __device__ __forceinline__ double qs_omega(int kind, double zeta, double h) {
   return exp(-(zeta * zeta) / (h * h * 0.16));
 }
 
-template <typename T>
+template <int TPO = kQsTpo, typename T>
 __device__ __forceinline__ T qs_group_sum(T v) {
 #pragma unroll
-  for (int o = kQsTpo / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = TPO / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -190,13 +201,17 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_bond_geom(int64_t n, const int6
 }
 
 // Tangent pass 1 on the geometry: w[i].w = q_i dtheta_i = 3 (q_i/m_i) sum_j V_j om zeta yh.(w_j - w_i)
+// (a solve that has ended makes the kernel return)
+template <int TPO>
 __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_g(int64_t n, const int64_t* __restrict__ row,
                                                           const int32_t* __restrict__ col,
                                                           const double4* __restrict__ g,
                                                           const double4* __restrict__ ab,
-                                                          const double4* __restrict__ pt, double4* __restrict__ w) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kQsTpo;
-  const int lane = threadIdx.x & (kQsTpo - 1);
+                                                          const double4* __restrict__ pt, double4* __restrict__ w,
+                                                          const CgCtl* __restrict__ ctl) {
+  if (ctl->state) return;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / TPO;
+  const int lane = threadIdx.x & (TPO - 1);
   const bool valid = i < n;
   double acc = 0.0;
   if (valid) {
@@ -205,30 +220,31 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_g(int64_t n, const int64
     int64_t b = row[i] + lane;
     // batches of kQsBatch bonds per lane: stream loads, then gathers, then the
     // sums in bond order (the same order as one bond at a time)
-    for (; b + (kQsBatch - 1) * kQsTpo < b1; b += kQsBatch * kQsTpo) {
+    for (; b + (kQsBatch - 1) * TPO < b1; b += kQsBatch * TPO) {
       double4 gb[kQsBatch], wj[kQsBatch];
       int32_t j[kQsBatch];
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * kQsTpo], j[k] = col[b + k * kQsTpo];
+      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * TPO], j[k] = col[b + k * TPO];
 #pragma unroll
       for (int k = 0; k < kQsBatch; ++k) wj[k] = w[j[k]];
 #pragma unroll
       for (int k = 0; k < kQsBatch; ++k)
         acc += gb[k].w * (gb[k].x * (wj[k].x - wi.x) + gb[k].y * (wj[k].y - wi.y) + gb[k].z * (wj[k].z - wi.z));
     }
-    for (; b < b1; b += kQsTpo) {
+    for (; b < b1; b += TPO) {
       const double4 gb = g[b];
       const double4 wj = w[col[b]];
       acc += gb.w * (gb.x * (wj.x - wi.x) + gb.y * (wj.y - wi.y) + gb.z * (wj.z - wi.z));
     }
   }
-  acc = qs_group_sum(acc);
+  acc = qs_group_sum<TPO>(acc);
   if (valid && lane == 0) w[i].w = 3.0 * (ab[i].y / pt[i].x) * acc;
 }
 
 // Tangent pass 2 on the geometry: q = K p = -V d f (prescribed rows: q = p), or
-// (jm rho I + jk K) p for implicit dynamics; block partials of p.q
+// (jm rho I + jk K) p for implicit dynamics; p.q goes to ctl->pq
 //   V_j [dT yh + (T/|Y|)(dw - yh de)] = c2 (q dth_i + q dth_j) yh + V_j om (a_i + a_j) de yh + V_j T/|Y| (dw - yh de)
+template <int TPO>
 __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* __restrict__ row,
                                                       const int32_t* __restrict__ col,
                                                       const double4* __restrict__ g,
@@ -237,10 +253,10 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
                                                       const double4* __restrict__ w,
                                                       const uint8_t* __restrict__ fixed, double* __restrict__ q,
                                                       double* __restrict__ partial, const double4* __restrict__ pt,
-                                                      double jk, double jm) {
-  __shared__ double spq[kQsBlock];
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kQsTpo;
-  const int lane = threadIdx.x & (kQsTpo - 1);
+                                                      double jk, double jm, CgCtl* __restrict__ ctl) {
+  if (ctl->state) return;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / TPO;
+  const int lane = threadIdx.x & (TPO - 1);
   const bool valid = i < n;
   double d0 = 0.0, d1 = 0.0, d2 = 0.0;
   double4 wi = make_double4(0, 0, 0, 0);
@@ -256,22 +272,22 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
       d1 += sy * gb.y + cb.x * w1;
       d2 += sy * gb.z + cb.x * w2;
     };
-    for (; b + (kQsBatch - 1) * kQsTpo < b1; b += kQsBatch * kQsTpo) {  // batched as in k_qs_dtheta_g
+    for (; b + (kQsBatch - 1) * TPO < b1; b += kQsBatch * TPO) {  // batched as in k_qs_dtheta_g
       double4 gb[kQsBatch], wj[kQsBatch];
       double2 cb[kQsBatch];
       int32_t j[kQsBatch];
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * kQsTpo], cb[k] = gc[b + k * kQsTpo], j[k] = col[b + k * kQsTpo];
+      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * TPO], cb[k] = gc[b + k * TPO], j[k] = col[b + k * TPO];
 #pragma unroll
       for (int k = 0; k < kQsBatch; ++k) wj[k] = w[j[k]];
 #pragma unroll
       for (int k = 0; k < kQsBatch; ++k) bond(gb[k], cb[k], wj[k]);
     }
-    for (; b < b1; b += kQsTpo) bond(g[b], gc[b], w[col[b]]);
+    for (; b < b1; b += TPO) bond(g[b], gc[b], w[col[b]]);
   }
-  d0 = qs_group_sum(d0);
-  d1 = qs_group_sum(d1);
-  d2 = qs_group_sum(d2);
+  d0 = qs_group_sum<TPO>(d0);
+  d1 = qs_group_sum<TPO>(d1);
+  d2 = qs_group_sum<TPO>(d2);
   double pq = 0.0;
   if (valid && lane < 3) {
     const double d = lane == 0 ? d0 : (lane == 1 ? d1 : d2);
@@ -282,13 +298,8 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
     q[3 * i + lane] = out;
     pq = p * out;
   }
-  spq[threadIdx.x] = pq;
-  __syncthreads();
-  for (int o = kQsBlock / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) spq[threadIdx.x] += spq[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = spq[0];
+  double sum[1] = {pq};
+  if (cg_grid_sum<1, kQsBlock>(sum, partial, &ctl->ticket[0]) && threadIdx.x == 0) ctl->pq = sum[0];
 }
 
 // Inverse 3x3 diagonal blocks of K (prescribed rows/columns set to identity).
@@ -373,16 +384,12 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_block_diag(int64_t n, const int
   }
 }
 
-// z = P r (block Jacobi or identity); optional partial sums of r.z and r.r.
+// z = P r (block Jacobi)
 __global__ void k_qs_precond(int64_t n, const double* __restrict__ dinv, const double* __restrict__ r,
-                             double* __restrict__ z, int use_bj) {
+                             double* __restrict__ z) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double r0 = r[3 * i], r1 = r[3 * i + 1], r2 = r[3 * i + 2];
-  if (!use_bj) {
-    z[3 * i] = r0, z[3 * i + 1] = r1, z[3 * i + 2] = r2;
-    return;
-  }
   const double* d = dinv + 9 * i;
   z[3 * i] = d[0] * r0 + d[1] * r1 + d[2] * r2;
   z[3 * i + 1] = d[3] * r0 + d[4] * r1 + d[5] * r2;
@@ -445,20 +452,14 @@ __global__ void k_qs_update_p(int64_t n, const double* __restrict__ scal, const 
   w[i] = p;
 }
 
+// The learned preconditioner's scalars. scal: [0] r.z, [1] p.q, [3] beta,
+// [4] r.r; red: [0] z.r, [2] r.r of the new residual, [4] z.q. what 0:
+// scal[1] = p.q; else beta = max(0, z_new.(r_new - r_old)/rz_old) with
+// z_new.r_old = z_new.r_new + alpha z_new.q (Polak-Ribiere).
 __global__ void k_qs_set_scalars(double* scal, const double* red, int what) {
-  // scal: [0] r.z, [1] p.q, [3] beta, [4] r.r; red: [0] z.r, [2] r.r of the new
-  // residual, [4] z.q (flexible only).
-  // what 0: scal[1] = p.q ; what 1: beta = rz_new/rz_old (Fletcher-Reeves on the
-  // preconditioned residual); what 2: flexible beta = max(0, z_new.(r_new -
-  // r_old)/rz_old) with z_new.r_old = z_new.r_new + alpha z_new.q (Polak-Ribiere).
   if (threadIdx.x != 0) return;
   if (what == 0) {
     scal[1] = red[0];
-  } else if (what == 1) {
-    const double rz_new = red[0];
-    scal[3] = rz_new / scal[0];
-    scal[0] = rz_new;
-    scal[4] = red[2];
   } else {
     const double rz_old = scal[0];
     const double alpha = __ddiv_rn(rz_old, scal[1]);
@@ -508,11 +509,84 @@ __global__ void k_qs_finish(int64_t m, double inv_dt, const double* __restrict__
   v[k] = du[k] * inv_dt;
 }
 
+// One CG iteration after the tangent passes, without a coarse level:
+//   x += alpha p, r -= alpha q, z = P r (block Jacobi, or P = I), r.z, r.r
+// with alpha = r.z / p.q, and the iteration's scalars from the last block.
+// FIRST: the start of a solve (x and r as they are). One launch where the
+// update, the preconditioner, the dot products, their reduction and the
+// scalars were one each, with a copy of |r|^2 to the host.
+template <bool FIRST>
+__global__ void __launch_bounds__(kQsBlock) k_cg_update(int64_t n, const double4* __restrict__ w,
+                                                        const double* __restrict__ q, double* __restrict__ x,
+                                                        double* __restrict__ r, double* __restrict__ z,
+                                                        const double* __restrict__ dinv, int use_bj,
+                                                        double* __restrict__ partial, CgCtl* __restrict__ ctl) {
+  if (!FIRST && ctl->state) return;
+  const double alpha = FIRST ? 0.0 : ctl->rz / ctl->pq;
+  double s[2] = {0.0, 0.0};
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double rv[3] = {r[3 * i], r[3 * i + 1], r[3 * i + 2]};
+    if (!FIRST) {
+      const double4 p = w[i];
+      const double pv[3] = {p.x, p.y, p.z};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        rv[c] -= alpha * q[3 * i + c];
+        r[3 * i + c] = rv[c];
+        x[3 * i + c] += alpha * pv[c];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double zc = rv[c];
+      if (use_bj) {
+        const double* d = dinv + 9 * i + 3 * c;
+        zc = d[0] * rv[0] + d[1] * rv[1] + d[2] * rv[2];
+      }
+      z[3 * i + c] = zc;
+      s[0] += rv[c] * zc;
+      s[1] += rv[c] * rv[c];
+    }
+  }
+  if (cg_grid_sum<2, kQsBlock>(s, partial, &ctl->ticket[1]) && threadIdx.x == 0) cg_scalars(ctl, s[0], s[1], FIRST);
+}
+
+// p = z + beta p (p = z at the start, where the previous direction may be unset)
+__global__ void k_cg_direction(int64_t n, const double* __restrict__ z, double4* __restrict__ w, int first,
+                               const CgCtl* __restrict__ ctl) {
+  if (ctl->state) return;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double beta = ctl->beta;
+  const double z0 = z[3 * i], z1 = z[3 * i + 1], z2 = z[3 * i + 2];
+  if (first) {
+    w[i] = make_double4(z0, z1, z2, 0.0);
+  } else {
+    const double4 p = w[i];
+    w[i] = make_double4(z0 + beta * p.x, z1 + beta * p.y, z2 + beta * p.z, p.w);
+  }
+}
+
+// The start of a solve (state, tolerance, where the report goes).
+__global__ void k_cg_begin(CgCtl* ctl, double tol, long long max_it, CgReport* report) {
+  ctl->state = CG_RUNNING;
+  ctl->ticket[0] = ctl->ticket[1] = 0;
+  ctl->tol = tol;
+  ctl->max_it = max_it;
+  ctl->it = 0;
+  ctl->report = report;
+}
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 static unsigned g1(int64_t m) { return (unsigned)((m + kQsBlock - 1) / kQsBlock); }
-static unsigned gt(int64_t n) { return (unsigned)((n * kQsTpo + kQsBlock - 1) / kQsBlock); }
+static unsigned gt(int64_t n, int tpo = kQsTpo) { return (unsigned)((n * tpo + kQsBlock - 1) / kQsBlock); }
+// Blocks of the CG vector kernels: enough to fill the chip, few enough that
+// the last block adds their sums quickly.
+static unsigned gv(int64_t n) { return std::min(g1(n), 4u * 148u); }
+// Lanes per point of the tangent passes.
+static int qs_lanes(int64_t n) { return n <= kQsWide ? 32 : kQsTpo; }
 
 static int qs_alloc(pd_ctx* c) {
   if (!c->qs) c->qs = new QsState();
@@ -526,7 +600,13 @@ static int qs_alloc(pd_ctx* c) {
   PD_CUDA_TRY(c, s->nd.alloc(n));
   for (auto* b : {&s->f, &s->r, &s->du, &s->x, &s->z, &s->q, &s->pred}) PD_CUDA_TRY(c, b->alloc(3 * n));
   PD_CUDA_TRY(c, s->dinv.alloc(9 * n));
-  PD_CUDA_TRY(c, s->partial.alloc(3 * (size_t)std::max<int64_t>(kRedBlocks, gt(n)) + 8));
+  PD_CUDA_TRY(c, s->partial.alloc(3 * (size_t)std::max<int64_t>(kRedBlocks, gt(n, qs_lanes(n))) + 8));
+  PD_CUDA_TRY(c, s->ctl.alloc(1));
+  PD_CUDA_TRY(c, dzero(c, s->ctl.p, s->ctl.bytes()));
+  if (!s->report) {
+    PD_CUDA_TRY(c, cudaHostAlloc((void**)&s->report, sizeof(CgReport), cudaHostAllocMapped));
+    PD_CUDA_TRY(c, cudaHostGetDevicePointer((void**)&s->report_dev, s->report, 0));
+  }
   PD_CUDA_TRY(c, s->scal.alloc(16));
   PD_CUDA_TRY(c, s->fixed.alloc(n));
   PD_CUDA_TRY(c, dzero(c, s->pred.p, s->pred.bytes()));
@@ -563,15 +643,14 @@ static int qs_residual(pd_ctx* c, double* l2, double* linf) {
   return PD_OK;
 }
 
-// z = M r: block Jacobi, plus the coarse correction (two-level), plus the
-// network's correction (learned).
-static int qs_apply_precond(pd_ctx* c, int precond, const double* r, double* z) {
+// z = M r of the learned preconditioner: block Jacobi, the network's
+// correction and, where it is on, the coarse one.
+static int qs_apply_learned(pd_ctx* c, const double* r, double* z) {
   QsState* s = c->qs;
-  k_qs_precond<<<g1(c->n), kQsBlock, 0, c->stream>>>(c->n, s->dinv.p, r, z, precond != PD_PRECOND_NONE);
+  k_qs_precond<<<g1(c->n), kQsBlock, 0, c->stream>>>(c->n, s->dinv.p, r, z);
   PD_CUDA_TRY(c, cudaGetLastError());
-  if (precond == PD_PRECOND_MPNN) TRY_RC(mpnn_apply_add(c, r, z));
-  if (s->coarse_on && (precond == PD_PRECOND_MPNN || precond == PD_PRECOND_TWO_LEVEL))
-    TRY_RC(coarse_apply_add(c, r, z, s->fixed.p));
+  TRY_RC(mpnn_apply_add(c, r, z));
+  if (s->coarse_on) TRY_RC(coarse_apply_add(c, r, z, s->fixed.p));
   return PD_OK;
 }
 
@@ -593,15 +672,30 @@ static int qs_geometry(pd_ctx* c) {
   return PD_OK;
 }
 
-static int qs_tangent(pd_ctx* c) {
+template <int TPO>
+static void launch_tangent(pd_ctx* c) {
   QsState* s = c->qs;
   const int64_t n = c->n;
+  k_qs_dtheta_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->abq.p, c->pt.p,
+                                                             s->w.p, s->ctl.p);
+  k_qs_df_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->gco.p, c->xv.p, s->w.p,
+                                                         s->fixed.p, s->q.p, s->partial.p, c->pt.p, s->jk, s->jm,
+                                                         s->ctl.p);
+}
+
+static int qs_tangent(pd_ctx* c) {
   TRY_RC(qs_geometry(c));
-  k_qs_dtheta_g<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->abq.p, c->pt.p, s->w.p);
-  k_qs_df_g<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->gco.p, c->xv.p, s->w.p,
-                                               s->fixed.p, s->q.p, s->partial.p, c->pt.p, s->jk, s->jm);
+  if (qs_lanes(c->n) == 32) launch_tangent<32>(c);
+  else launch_tangent<kQsTpo>(c);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;
+}
+
+// Outside a solve the passes must not see the last one's end.
+static int qs_tangent_alone(pd_ctx* c) {
+  QsState* s = c->qs;
+  k_cg_begin<<<1, 1, 0, c->stream>>>(s->ctl.p, 0.0, 0, s->report_dev);
+  return qs_tangent(c);
 }
 
 // Preconditioned CG on K x = r (Belos BlockCG in the reference). Flexible
@@ -622,8 +716,9 @@ static void k_qs_pack_x(int64_t n, QsState* s, pd_ctx* c) {
   k_qs_x_to_w<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->x.p, s->w.p);
 }
 
-static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out,
-                     bool* stalled);
+static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out);
+static int qs_cg_flexible(pd_ctx* c, double rel_tol, int max_it, int* iters, double* rel_out, bool* stalled);
+constexpr int kCgAhead = 3;  // iterations the host launches ahead of the last one reported
 
 // CG with the learned preconditioner first and 3x3 block Jacobi (the
 // reference's "Block 3x3") as the fallback: when the flexible iteration
@@ -633,10 +728,7 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
 static int qs_cg(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out) {
   QsState* s = c->qs;
   const int64_t m = 3 * c->n;
-  if (precond != PD_PRECOND_MPNN) {
-    bool stalled = false;
-    return qs_cg_run(c, precond, rel_tol, max_it, iters, rel_out, &stalled);
-  }
+  if (precond != PD_PRECOND_MPNN) return qs_cg_run(c, precond, rel_tol, max_it, iters, rel_out);
   if (s->cg_b.count < (size_t)m) PD_CUDA_TRY(c, s->cg_b.alloc(m));
   if (s->cg_x0.count < (size_t)m) PD_CUDA_TRY(c, s->cg_x0.alloc(m));
   DBuf<double>& b = s->cg_b;
@@ -645,13 +737,13 @@ static int qs_cg(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters,
   bool stalled = false;
   int its = 0;
   double rel = 0.0;
-  int rc = qs_cg_run(c, PD_PRECOND_MPNN, rel_tol, max_it, &its, &rel, &stalled);
+  int rc = qs_cg_flexible(c, rel_tol, max_it, &its, &rel, &stalled);
   if (rc != PD_OK && rc != PD_ERR_NOT_CONVERGED && rc != PD_ERR_NONFINITE) return rc;
   TRY_RC(mpnn_check_status(c));
   // true residual r = b - K x
   const int64_t n = c->n;
   k_qs_pack_x(n, s, c);
-  TRY_RC(qs_tangent(c));
+  TRY_RC(qs_tangent_alone(c));
   k_qs_true_residual<<<g1(m), kQsBlock, 0, c->stream>>>(m, b.p, s->q.p, s->r.p);
   k_qs_dots<<<kRedBlocks, kQsBlock, 0, c->stream>>>(m, s->r.p, s->r.p, b.p, s->partial.p);
   k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, kRedBlocks, 3, 0, s->scal.p + 8);
@@ -680,7 +772,7 @@ static int qs_cg(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters,
   const double tol2 = (std::isfinite(true_rel) && true_rel > 0) ? std::min(1.0, rel_tol / true_rel) : rel_tol;
   int its2 = 0;
   double rel2 = 0.0;
-  rc = qs_cg_run(c, PD_PRECOND_BLOCK_JACOBI, tol2, max_it, &its2, &rel2, &stalled);
+  rc = qs_cg_run(c, PD_PRECOND_BLOCK_JACOBI, tol2, max_it, &its2, &rel2);
   k_qs_axpy<<<g1(m), kQsBlock, 0, c->stream>>>(m, 1.0, x0.p, s->x.p);
   PD_CUDA_TRY(c, cudaGetLastError());
   *iters = its + its2;
@@ -688,18 +780,16 @@ static int qs_cg(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters,
   return rc;
 }
 
-static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out,
-                     bool* stalled) {
+// CG with the learned preconditioner (flexible beta), one host read per iteration.
+static int qs_cg_flexible(pd_ctx* c, double rel_tol, int max_it, int* iters, double* rel_out, bool* stalled) {
   QsState* s = c->qs;
   const int64_t n = c->n, m = 3 * n;
-  const bool flexible = precond == PD_PRECOND_MPNN;
-  const int every =
-      (precond == PD_PRECOND_BLOCK_JACOBI || precond == PD_PRECOND_TWO_LEVEL) ? mpnn_capture_every(c) : 0;
   double best = 1.0;
   int best_it = 0;
   *stalled = false;
   PD_CUDA_TRY(c, cudaMemsetAsync(s->x.p, 0, s->x.bytes(), c->stream));
-  TRY_RC(qs_apply_precond(c, precond, s->r.p, s->z.p));
+  k_cg_begin<<<1, 1, 0, c->stream>>>(s->ctl.p, 0.0, 0, s->report_dev);
+  TRY_RC(qs_apply_learned(c, s->r.p, s->z.p));
   // scal: [0] rz, [1] pq, [3] beta, [4] rr
   k_qs_dots<<<kRedBlocks, kQsBlock, 0, c->stream>>>(m, s->r.p, s->z.p, s->z.p, s->partial.p);
   k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, kRedBlocks, 3, 0, s->scal.p + 8);
@@ -715,49 +805,130 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
   k_qs_update_p<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->scal.p, s->z.p, s->w.p, 1);
   double rel = 1.0;
   int it = 0;
-  if (every > 0) TRY_RC(mpnn_snapshot(c, s->r.p, s->x.p));
   while (it < max_it) {
     TRY_RC(qs_tangent(c));
-    k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, (int)gt(n), 1, 0, s->scal.p + 8);
-    k_qs_set_scalars<<<1, 32, 0, c->stream>>>(s->scal.p, s->scal.p + 8, 0);
+    k_qs_set_scalars<<<1, 32, 0, c->stream>>>(s->scal.p, &s->ctl.p->pq, 0);
     k_qs_axpy2<<<g1(m), kQsBlock, 0, c->stream>>>(m, s->scal.p, s->w.p, s->q.p, s->x.p, s->r.p);
-    TRY_RC(qs_apply_precond(c, precond, s->r.p, s->z.p));
+    TRY_RC(qs_apply_learned(c, s->r.p, s->z.p));
     k_qs_dots<<<kRedBlocks, kQsBlock, 0, c->stream>>>(m, s->r.p, s->z.p, s->z.p, s->partial.p);
     k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, kRedBlocks, 3, 0, s->scal.p + 8);
-    if (flexible) {  // z_new.q for beta = z_new.(r_new - r_old)/rz_old, r_old = r_new + alpha q
-      k_qs_dots<<<kRedBlocks, kQsBlock, 0, c->stream>>>(m, s->z.p, s->q.p, s->q.p, s->partial.p);
-      k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, kRedBlocks, 3, 0, s->scal.p + 12);
-    }
-    k_qs_set_scalars<<<1, 32, 0, c->stream>>>(s->scal.p, s->scal.p + 8, flexible ? 2 : 1);
+    // z_new.q for beta = z_new.(r_new - r_old)/rz_old, r_old = r_new + alpha q
+    k_qs_dots<<<kRedBlocks, kQsBlock, 0, c->stream>>>(m, s->z.p, s->q.p, s->q.p, s->partial.p);
+    k_qs_reduce<<<1, kQsBlock, 0, c->stream>>>(s->partial.p, kRedBlocks, 3, 0, s->scal.p + 12);
+    k_qs_set_scalars<<<1, 32, 0, c->stream>>>(s->scal.p, s->scal.p + 8, 1);
     double rr;  // the only host read of the iteration: |r|^2 for the stopping test
     PD_CUDA_TRY(c, cudaMemcpyAsync(&rr, s->scal.p + 4, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     rel = std::sqrt(rr) / r0;
     ++it;
     if (!std::isfinite(rel)) {
-      if (every > 0) mpnn_drop_snapshots(c);
       c->err = "CG diverged (non-finite residual)";
       return PD_ERR_NONFINITE;
     }
     if (rel <= rel_tol) break;
-    if (every > 0 && it % every == 0) TRY_RC(mpnn_snapshot(c, s->r.p, s->x.p));
-    if (flexible) {  // stall: no 10x decrease of the residual over 60 iterations
-      if (rel < 0.1 * best) best = rel, best_it = it;
-      if (it - best_it > 60) {
-        *stalled = true;
-        break;
-      }
+    // stall: no 10x decrease of the residual over 60 iterations
+    if (rel < 0.1 * best) best = rel, best_it = it;
+    if (it - best_it > 60) {
+      *stalled = true;
+      break;
     }
     k_qs_update_p<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->scal.p, s->z.p, s->w.p, 0);
   }
   PD_CUDA_TRY(c, cudaGetLastError());
-  if (every > 0) {
-    if (rel <= rel_tol) TRY_RC(mpnn_commit_snapshots(c, s->x.p, s->dinv.p));
-    else mpnn_drop_snapshots(c);
-  }
   *iters = it;
   *rel_out = rel;
   return rel <= rel_tol ? PD_OK : PD_ERR_NOT_CONVERGED;
+}
+
+// Waits until the solve has reported `it` iterations or its end. The report
+// is written by kernels already in the stream: the wait ends with them (or
+// with their error, or when the stream is idle and nothing was reported).
+static int cg_wait(pd_ctx* c, long long it, CgReport* out) {
+  const volatile CgReport* h = c->qs->report;
+  bool idle = false;
+  for (unsigned spin = 0;; ++spin) {
+    const CgReport word = *h;
+    if (word != ~0ull && ((word & 7) != CG_RUNNING || (long long)(word >> 3) >= it)) {
+      *out = word;
+      return PD_OK;
+    }
+    if (idle) {
+      c->err = "the CG solve stopped without a report";
+      return PD_ERR_CUDA;
+    }
+    if ((spin & 1023u) == 1023u) {
+      const cudaError_t e = cudaStreamQuery(c->stream);
+      if (e == cudaSuccess) idle = true;  // one more look at the report
+      else if (e != cudaErrorNotReady) PD_CUDA_TRY(c, e);
+    }
+  }
+}
+
+// CG with a fixed preconditioner (none, block Jacobi, two-level): the scalars
+// and the stopping test stay on the device, and the host runs kCgAhead
+// iterations ahead of the last one reported. Launches after the end of the
+// solve return at once.
+static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out) {
+  QsState* s = c->qs;
+  const int64_t n = c->n;
+  const int every = mpnn_capture_every(c) && precond != PD_PRECOND_NONE ? mpnn_capture_every(c) : 0;
+  const int ahead = every > 0 ? 0 : kCgAhead;  // training pairs are taken at the reported iterate
+  const bool coarse = s->coarse_on && precond == PD_PRECOND_TWO_LEVEL;
+  const int use_bj = precond != PD_PRECOND_NONE;
+  auto update = [&](bool first) -> int {
+    if (coarse)
+      return coarse_cg_update(c, s->w.p, s->q.p, s->x.p, s->r.p, s->z.p, s->dinv.p, s->fixed.p, s->partial.p, s->ctl.p,
+                              first, gv(n));
+    if (first)
+      k_cg_update<true><<<gv(n), kQsBlock, 0, c->stream>>>(n, s->w.p, s->q.p, s->x.p, s->r.p, s->z.p, s->dinv.p,
+                                                           use_bj, s->partial.p, s->ctl.p);
+    else
+      k_cg_update<false><<<gv(n), kQsBlock, 0, c->stream>>>(n, s->w.p, s->q.p, s->x.p, s->r.p, s->z.p, s->dinv.p,
+                                                            use_bj, s->partial.p, s->ctl.p);
+    return PD_OK;
+  };
+  *(volatile CgReport*)s->report = ~0ull;  // (no kernel of an earlier solve is in flight: each ends with a wait for the stream)
+  PD_CUDA_TRY(c, cudaMemsetAsync(s->x.p, 0, s->x.bytes(), c->stream));
+  k_cg_begin<<<1, 1, 0, c->stream>>>(s->ctl.p, rel_tol, max_it, s->report_dev);
+  TRY_RC(update(true));
+  k_cg_direction<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->z.p, s->w.p, 1, s->ctl.p);
+  if (every > 0) TRY_RC(mpnn_snapshot(c, s->r.p, s->x.p));
+  CgReport at = 0;
+  int rc = PD_OK;
+  for (int it = 1; it <= max_it; ++it) {
+    rc = qs_tangent(c);
+    if (rc == PD_OK) rc = update(false);
+    PD_CUDA_TRY(c, cudaGetLastError());
+    if (rc == PD_OK) rc = cg_wait(c, it - ahead, &at);
+    if (rc != PD_OK || (at & 7) != CG_RUNNING) break;
+    if (every > 0 && it % every == 0) TRY_RC(mpnn_snapshot(c, s->r.p, s->x.p));
+    k_cg_direction<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->z.p, s->w.p, 0, s->ctl.p);
+  }
+  if (rc == PD_OK && (at & 7) == CG_RUNNING) rc = cg_wait(c, max_it, &at);
+  // (the copy also ends the launches beyond the last iteration, which must not
+  // reach into the next solve's report)
+  const cudaError_t e = d2h(c, rel_out, &s->ctl.p->rel, sizeof(double));
+  if (rc != PD_OK) {
+    if (every > 0) mpnn_drop_snapshots(c);
+    return rc;
+  }
+  PD_CUDA_TRY(c, e);
+  const int state = (int)(at & 7);
+  *iters = (int)(at >> 3);
+  if (state == CG_NONFINITE) {
+    if (every > 0) mpnn_drop_snapshots(c);
+    c->err = "CG diverged (non-finite residual)";
+    return PD_ERR_NONFINITE;
+  }
+  if (state == CG_ZERO_RHS) {
+    if (every > 0) mpnn_drop_snapshots(c);
+    return PD_OK;
+  }
+  if (every > 0) {
+    if (state == CG_CONVERGED) TRY_RC(mpnn_commit_snapshots(c, s->x.p, s->dinv.p));
+    else mpnn_drop_snapshots(c);
+  }
+  return state == CG_CONVERGED ? PD_OK : PD_ERR_NOT_CONVERGED;
 }
 
 __global__ void k_qs_pack_w(int64_t n, const double* __restrict__ w, const uint8_t* __restrict__ fixed,
@@ -807,7 +978,7 @@ int qs_tangent_apply(pd_ctx* c, const double* u_dev, const double* w_dev, double
   QsState* s = c->qs;
   const int64_t n = c->n;
   k_qs_pack_w<<<g1(n), kQsBlock, 0, c->stream>>>(n, w_dev, s->fixed.p, s->w.p);
-  TRY_RC(qs_tangent(c));
+  TRY_RC(qs_tangent_alone(c));
   k_qs_fixed_rows<<<g1(n), kQsBlock, 0, c->stream>>>(n, w_dev, s->fixed.p, s->q.p);
   PD_CUDA_TRY(c, cudaMemcpyAsync(kw_dev, s->q.p, 3 * n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
   return PD_OK;
@@ -866,7 +1037,7 @@ int qs_apply_K(pd_ctx* c, const double* w_dev, double* kw_dev) {
   QsState* s = c->qs;
   const int64_t n = c->n;
   k_qs_pack_w<<<g1(n), kQsBlock, 0, c->stream>>>(n, w_dev, s->fixed.p, s->w.p);
-  TRY_RC(qs_tangent(c));
+  TRY_RC(qs_tangent_alone(c));
   k_qs_fixed_rows<<<g1(n), kQsBlock, 0, c->stream>>>(n, w_dev, s->fixed.p, s->q.p);
   PD_CUDA_TRY(c, cudaMemcpyAsync(kw_dev, s->q.p, 3 * n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
   return PD_OK;
@@ -1285,8 +1456,7 @@ int implicit_run(pd_ctx* c, double dt, double t0, int64_t nsteps, const pd_impli
       }
       int its = 0;
       double rel = 0.0;
-      bool stalled = false;
-      const int r2 = qs_cg_run(c, precond, o->cg_relative_tolerance, o->max_cg_iterations, &its, &rel, &stalled);
+      const int r2 = qs_cg_run(c, precond, o->cg_relative_tolerance, o->max_cg_iterations, &its, &rel);
       if (r2 != PD_OK && r2 != PD_ERR_NOT_CONVERGED) {  // a CG that stops short is used as it is (:3870-3872)
         rc = r2;
         break;

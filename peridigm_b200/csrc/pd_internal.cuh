@@ -329,6 +329,12 @@ int coarse_build(pd_ctx* c, const double4* y, const double4* ab, const uint8_t* 
                  double* assembled);
 int coarse_apply_add(pd_ctx* c, const double* r, double* z, const uint8_t* fixed);
 int coarse_apply_add_f(pd_ctx* c, const float* r, double* z, const uint8_t* fixed, double scale);
+// One CG iteration's vector work with the two-level preconditioner (after the
+// tangent passes): x, r and z = P_bj r + P0 Ac^-1 P0^T r, the dot products and
+// the scalars. first: the start of a solve. blocks: of the point kernels.
+struct CgCtl;
+int coarse_cg_update(pd_ctx* c, const double4* w, const double* q, double* x, double* r, double* z, const double* dinv,
+                     const uint8_t* fixed, double* partial, CgCtl* ctl, bool first, unsigned blocks);
 int coarse_aggregates(pd_ctx* c, int32_t* agg_dev);
 int coarse_copy_inverse(pd_ctx* c, double* dst_dev);
 int64_t coarse_size(const pd_ctx* c);

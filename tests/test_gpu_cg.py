@@ -1,0 +1,71 @@
+"""The conjugate-gradient loop that keeps its scalars on the device.
+
+* Tangent products of both lane counts (32 lanes per point up to 16384 points,
+  8 above) against the oracle's linearization: 1e-11 relative, the bound of
+  the tangent tests.
+* The iteration limit: CG stops at exactly max_cg iterations although the host
+  runs ahead of the device, and the solution is the limited one, not a later
+  iterate: a second solve with the same limit repeats it bit for bit.
+* A converged load step leaves a force residual below the Newton tolerance.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from peridigm_b200 import Context, PDError, _lib, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims", [(7, 6, 5), (32, 32, 16), (33, 31, 17)])
+def test_tangent_product_of_both_lane_counts(dims):
+    x, vol = workloads.lattice(*dims, 1.0e-3, jitter=0.05, seed=2)
+    h, K, mu = 3.015e-3, 130.0e9, 78.0e9
+    rng = np.random.default_rng(5)
+    u, w = rng.normal(0, 1e-6, x.size), rng.normal(0, 1.0, x.size)
+    row, col = O.neighbor_search(x, h)
+    ref = -np.repeat(vol, 3) * O.lps_jv(x, x + u, vol, row, col, K, mu, h, w)
+    with Context(precision="fp64") as ctx:
+        ctx.set_points(x, vol)
+        ctx.set_horizons([h])
+        ctx.build_bonds()
+        ctx.material(K, mu, 7800.0)
+        kw = ctx.jacobian_apply(u, w)
+    assert np.linalg.norm(kw - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+def _step(ctx, precond, max_cg, max_newton, tol):
+    st = _lib.Stats()
+    ctx.set_state(np.zeros(3 * ctx.n), np.zeros(3 * ctx.n))
+    try:
+        ctx.qs_load_step(0.0, 0.05, newton_tolerance=tol, cg_relative_tolerance=1e-12, max_newton=max_newton,
+                         max_cg=max_cg, preconditioner=precond, use_predictor=False, stats=st)
+    except PDError as e:
+        assert "Newton" in str(e)
+    return st, ctx.field("Displacement")
+
+
+@pytest.mark.parametrize("precond,modes", [("none", 3), ("block_jacobi", 3), ("two_level", 3), ("two_level", 6)])
+def test_iteration_limit_and_convergence(precond, modes):
+    w = workloads.qs_cube(n=13, jitter=0.05, load_steps=4)
+    with Context(precision="fp64") as ctx:
+        workloads.setup_context(ctx, w)
+        ctx.coarse_modes(modes)
+        for limit in (1, 2, 7):
+            st, u = _step(ctx, precond, limit, 1, -1e-12)
+            assert st.newton_iterations == 1 and st.cg_iterations == limit
+            st, u2 = _step(ctx, precond, limit, 1, -1e-12)
+            assert st.cg_iterations == limit and np.array_equal(u, u2)
+        st, u = _step(ctx, precond, 4000, 20, -1e-9)
+        f = ctx.field("Force_Density") * np.repeat(w["vol"], 3)
+    free = np.ones(len(f), bool)
+    for bc in w["bcs"]:
+        free[3 * bc["points"] + bc["coordinate"]] = False
+    row, col = O.neighbor_search(w["x"], w["horizon"])
+    start = np.zeros(len(f))  # the prescribed increment alone: the scale of a relative tolerance
+    for bc in w["bcs"]:
+        start[3 * bc["points"] + bc["coordinate"]] = 0.05 * bc["a"]
+    r0 = O.eval_model(w["x"], w["x"] + start, w["vol"], row, col, w["K"], w["mu"], w["horizon"])["force"]
+    r0 = (r0 * np.repeat(w["vol"], 3))[free]
+    metric = lambda r: np.linalg.norm(r) + 20.0 * np.abs(r).max()  # noqa: E731
+    assert metric(f[free]) <= 1.01e-9 * metric(r0)
