@@ -41,6 +41,12 @@ struct ContactState {
   DBuf<int32_t> ccol;
   int64_t npairs = 0;
   bool have_list = false;
+  // the points that have a pair, and their number (device), from the last
+  // search: the force pass of a step visits them alone
+  DBuf<int32_t> active;
+  DBuf<int> n_active;
+  DBuf<double4> pos_s;   // search positions in cell order
+  bool fc_follows = false;  // the context's contact force is zero at the points without a pair
   // search temporaries kept between searches (grown only): a search between
   // steps then allocates and frees no device memory, whose driver calls can
   // wait behind other processes' queries of the device
@@ -87,104 +93,150 @@ __global__ void k_contact_positions(int64_t n, const double4* __restrict__ xv, c
   }
 }
 
-// One warp per point; FILL = false counts, FILL = true writes the row.
+// The search positions cell by cell.
+__global__ void k_sorted_positions(int64_t n, const int32_t* __restrict__ sorted_idx, const double4* __restrict__ pos,
+                                   double4* __restrict__ pos_s) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < n) pos_s[s] = pos[sorted_idx[s]];
+}
+
+// Eight lanes per point over the 9 rows of 3 cells around its own: the three
+// cells of a row are one run of the sorted points, read in order. FILL = false
+// counts, FILL = true writes the row (most points have no pair and leave at
+// once). A cell is little wider than the search radius and holds a few points:
+// a warp to a point, cell by cell, had 3 of 32 lanes at work (two bodies of
+// 814,000 points: count 3.33 -> 0.29 ms, fill 3.83 -> 0.02 ms).
 template <bool FILL>
-__global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4* __restrict__ pos, Grid g,
+__global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4* __restrict__ pos,
+                                                       const double4* __restrict__ pos_s, Grid g,
                                                        const int64_t* __restrict__ cell_start,
                                                        const int32_t* __restrict__ sorted_idx, double r_search,
                                                        const int64_t* __restrict__ brow,
                                                        const int32_t* __restrict__ bcol, int64_t* __restrict__ counts,
                                                        const int64_t* __restrict__ crow, int32_t* __restrict__ ccol) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 7, shift = threadIdx.x & 24;
+  const unsigned group = 0xffu << shift;
+  if (i >= n) return;  // the lanes of a point leave together
+  if (FILL && crow[i + 1] == crow[i]) return;
   const double4 pi = pos[i];
   const double R2 = __dmul_rn(r_search, r_search);
   const int c0 = cell_coord(g, pi.x, 0), c1 = cell_coord(g, pi.y, 1), c2 = cell_coord(g, pi.z, 2);
+  const int x0 = max(c0 - 1, 0), x1 = min(c0 + 1, g.dims[0] - 1);
   int64_t cnt = 0;
   int64_t base = FILL ? crow[i] : 0;
-  for (int zc = c2 - 1; zc <= c2 + 1; ++zc) {
-    if (zc < 0 || zc >= g.dims[2]) continue;
-    for (int yc = c1 - 1; yc <= c1 + 1; ++yc) {
-      if (yc < 0 || yc >= g.dims[1]) continue;
-      for (int xc = c0 - 1; xc <= c0 + 1; ++xc) {
-        if (xc < 0 || xc >= g.dims[0]) continue;
-        const int64_t q = ((int64_t)zc * g.dims[1] + yc) * g.dims[0] + xc;
-        const int64_t s0 = cell_start[q], s1 = cell_start[q + 1];
-        for (int64_t s = s0; s < s1; s += 32) {
-          bool hit = false;
-          int32_t j = -1;
-          if (s + lane < s1) {
+  for (int zc = max(c2 - 1, 0); zc <= min(c2 + 1, g.dims[2] - 1); ++zc)
+    for (int yc = max(c1 - 1, 0); yc <= min(c1 + 1, g.dims[1] - 1); ++yc) {
+      const int64_t q = ((int64_t)zc * g.dims[1] + yc) * g.dims[0];
+      const int64_t s0 = cell_start[q + x0], s1 = cell_start[q + x1 + 1];
+      for (int64_t s = s0; s < s1; s += 8) {
+        bool hit = false;
+        int32_t j = -1;
+        if (s + lane < s1) {
+          const double4 pj = pos_s[s + lane];
+          if (sq3(__dsub_rn(pj.x, pi.x), __dsub_rn(pj.y, pi.y), __dsub_rn(pj.z, pi.z)) <= R2) {
             j = sorted_idx[s + lane];
-            if (j != i) {
-              const double4 pj = pos[j];
-              hit = sq3(__dsub_rn(pj.x, pi.x), __dsub_rn(pj.y, pi.y), __dsub_rn(pj.z, pi.z)) <= R2 &&
-                    !in_row(brow, bcol, i, j);
-            }
+            hit = j != i && !in_row(brow, bcol, i, j);
           }
-          const unsigned m = __ballot_sync(0xffffffffu, hit);
-          if (FILL) {
-            if (hit) ccol[base + __popc(m & ((1u << lane) - 1u))] = j;
-            base += __popc(m);
-          } else {
-            cnt += __popc(m);
-          }
+        }
+        const unsigned m = (__ballot_sync(group, hit) >> shift) & 0xffu;
+        if (FILL) {
+          if (hit) ccol[base + __popc(m & ((1u << lane) - 1u))] = j;
+          base += __popc(m);
+        } else {
+          cnt += __popc(m);
         }
       }
     }
-  }
   if (!FILL && lane == 0) counts[i] = cnt;
 }
 
-// Contact force density on each point (gather over its contact list).
-__global__ void __launch_bounds__(256) k_contact_force(int64_t n, const int64_t* __restrict__ crow,
-                                                      const int32_t* __restrict__ ccol,
-                                                      const double* __restrict__ y, const double* __restrict__ v,
+// The points with a pair (their order does not matter to the force pass).
+__global__ void k_contact_active(int64_t n, const int64_t* __restrict__ crow, int32_t* __restrict__ active,
+                                 int* __restrict__ n_active) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && crow[i + 1] > crow[i]) active[atomicAdd(n_active, 1)] = (int32_t)i;
+}
+
+// Where the current coordinates come from: an array y [3n], the FP64 records,
+// or x + u (split contexts), formed where they are needed.
+struct ContactCoords {
+  const double* y;
+  const double4* st;
+  const double4* xv;
+  const double* u;
+  __device__ __forceinline__ void at(int64_t i, double& a, double& b, double& c) const {
+    if (y) {
+      a = y[3 * i], b = y[3 * i + 1], c = y[3 * i + 2];
+    } else if (st) {
+      const double4 p = st[i];
+      a = p.x, b = p.y, c = p.z;
+    } else {
+      const double4 x = xv[i];
+      a = __dadd_rn(x.x, u[3 * i]), b = __dadd_rn(x.y, u[3 * i + 1]), c = __dadd_rn(x.z, u[3 * i + 2]);
+    }
+  }
+};
+
+// Contact force density on each point that has a pair (gather over its
+// contact list); the force of the others stays zero from the search on. Only
+// the coordinates of the pairs are formed: a pass over all points for them and
+// one for the forces were 26 us a step at 814,000 points, this one is 4.
+__global__ void __launch_bounds__(128) k_contact_force(const int* __restrict__ n_active,
+                                                      const int32_t* __restrict__ active,
+                                                      const int64_t* __restrict__ crow,
+                                                      const int32_t* __restrict__ ccol, ContactCoords Y,
+                                                      const double* __restrict__ v,
                                                       const double4* __restrict__ xv,
                                                       const double* __restrict__ kappa, double r_contact,
                                                       double friction, double* __restrict__ fc,
                                                       int* __restrict__ status) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double yi0 = y[3 * i], yi1 = y[3 * i + 1], yi2 = y[3 * i + 2];
-  const double vi0 = v[3 * i], vi1 = v[3 * i + 1], vi2 = v[3 * i + 2];
-  const double rc2 = __dmul_rn(r_contact, r_contact);
-  const double ki = kappa[i];
-  double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-  for (int64_t b = crow[i]; b < crow[i + 1]; ++b) {
-    const int32_t j = ccol[b];
-    const double d0 = __dsub_rn(y[3 * j], yi0), d1 = __dsub_rn(y[3 * j + 1], yi1), d2 = __dsub_rn(y[3 * j + 2], yi2);
-    const double dd = sq3(__dsub_rn(yi0, y[3 * j]), __dsub_rn(yi1, y[3 * j + 1]), __dsub_rn(yi2, y[3 * j + 2]));
-    if (!(dd < rc2)) continue;
-    const double d = __dsqrt_rn(dd);
-    const double gap = __dsub_rn(r_contact, d);
-    const double temp = __dadd_rn(__dmul_rn(ki, gap), __dmul_rn(kappa[j], gap));
-    const double Vj = xv[j].w;
-    const double s = __dmul_rn(temp, Vj);
-    f0 = __dsub_rn(f0, __ddiv_rn(__dmul_rn(s, d0), d));
-    f1 = __dsub_rn(f1, __ddiv_rn(__dmul_rn(s, d1), d));
-    f2 = __dsub_rn(f2, __ddiv_rn(__dmul_rn(s, d2), d));
-    if (friction != 0.0) {
-      const double n0 = d0 / d, n1 = d1 / d, n2 = d2 / d;
-      const double vj0 = v[3 * j], vj1 = v[3 * j + 1], vj2 = v[3 * j + 2];
-      const double ci = vi0 * n0 + vi1 * n1 + vi2 * n2;
-      const double cj = vj0 * n0 + vj1 * n1 + vj2 * n2;
-      const double pi0 = vi0 - ci * n0, pi1 = vi1 - ci * n1, pi2 = vi2 - ci * n2;
-      const double pj0 = vj0 - cj * n0, pj1 = vj1 - cj * n1, pj2 = vj2 - cj * n2;
-      const double w0 = pi0 - 0.5 * (pi0 + pj0), w1 = pi1 - 0.5 * (pi1 + pj1), w2 = pi2 - 0.5 * (pi2 + pj2);
-      const double wn = sqrt(w0 * w0 + w1 * w1 + w2 * w2);
-      if (wn != 0.0) {
-        const double fr = friction * s / wn;
-        f0 -= fr * w0;
-        f1 -= fr * w1;
-        f2 -= fr * w2;
+  const int m = *n_active;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+    const int64_t i = active[k];
+    double yi0, yi1, yi2;
+    Y.at(i, yi0, yi1, yi2);
+    const double vi0 = v[3 * i], vi1 = v[3 * i + 1], vi2 = v[3 * i + 2];
+    const double rc2 = __dmul_rn(r_contact, r_contact);
+    const double ki = kappa[i];
+    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+    for (int64_t b = crow[i]; b < crow[i + 1]; ++b) {
+      const int32_t j = ccol[b];
+      double yj0, yj1, yj2;
+      Y.at(j, yj0, yj1, yj2);
+      const double d0 = __dsub_rn(yj0, yi0), d1 = __dsub_rn(yj1, yi1), d2 = __dsub_rn(yj2, yi2);
+      const double dd = sq3(__dsub_rn(yi0, yj0), __dsub_rn(yi1, yj1), __dsub_rn(yi2, yj2));
+      if (!(dd < rc2)) continue;
+      const double d = __dsqrt_rn(dd);
+      const double gap = __dsub_rn(r_contact, d);
+      const double temp = __dadd_rn(__dmul_rn(ki, gap), __dmul_rn(kappa[j], gap));
+      const double Vj = xv[j].w;
+      const double s = __dmul_rn(temp, Vj);
+      f0 = __dsub_rn(f0, __ddiv_rn(__dmul_rn(s, d0), d));
+      f1 = __dsub_rn(f1, __ddiv_rn(__dmul_rn(s, d1), d));
+      f2 = __dsub_rn(f2, __ddiv_rn(__dmul_rn(s, d2), d));
+      if (friction != 0.0) {
+        const double n0 = d0 / d, n1 = d1 / d, n2 = d2 / d;
+        const double vj0 = v[3 * j], vj1 = v[3 * j + 1], vj2 = v[3 * j + 2];
+        const double ci = vi0 * n0 + vi1 * n1 + vi2 * n2;
+        const double cj = vj0 * n0 + vj1 * n1 + vj2 * n2;
+        const double pi0 = vi0 - ci * n0, pi1 = vi1 - ci * n1, pi2 = vi2 - ci * n2;
+        const double pj0 = vj0 - cj * n0, pj1 = vj1 - cj * n1, pj2 = vj2 - cj * n2;
+        const double w0 = pi0 - 0.5 * (pi0 + pj0), w1 = pi1 - 0.5 * (pi1 + pj1), w2 = pi2 - 0.5 * (pi2 + pj2);
+        const double wn = sqrt(w0 * w0 + w1 * w1 + w2 * w2);
+        if (wn != 0.0) {
+          const double fr = friction * s / wn;
+          f0 -= fr * w0;
+          f1 -= fr * w1;
+          f2 -= fr * w2;
+        }
       }
     }
+    if (!isfinite(f0) || !isfinite(f1) || !isfinite(f2)) atomicOr(status, ST_NONFINITE_CONTACT);
+    fc[3 * i] = f0;
+    fc[3 * i + 1] = f1;
+    fc[3 * i + 2] = f2;
   }
-  if (!isfinite(f0) || !isfinite(f1) || !isfinite(f2)) atomicOr(status, ST_NONFINITE_CONTACT);
-  fc[3 * i] = f0;
-  fc[3 * i + 1] = f1;
-  fc[3 * i + 2] = f2;
 }
 
 __global__ void k_bbox(int64_t n, const double4* __restrict__ pos, double* __restrict__ partial) {
@@ -250,9 +302,11 @@ static int contact_search(pd_ctx* c, const double4* pos) {
   int rc = bin_points(c, pos, n, g, idx_s, cell_start, &cs->bins);
   if (rc != PD_OK) return rc;
   PD_CUDA_TRY(c, counts.reserve(n + 1));
-  const unsigned gw = (unsigned)((n * 32 + 255) / 256);
-  k_contact_search<false><<<gw, 256, 0, c->stream>>>(n, pos, g, cell_start.p, idx_s.p, cs->r_search, c->row.p,
-                                                     c->col.p, counts.p, nullptr, nullptr);
+  PD_CUDA_TRY(c, cs->pos_s.reserve(n));
+  const unsigned g1 = (unsigned)((n + 255) / 256), gw = (unsigned)((n * 8 + 255) / 256);
+  k_sorted_positions<<<g1, 256, 0, c->stream>>>(n, idx_s.p, pos, cs->pos_s.p);
+  k_contact_search<false><<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search,
+                                                     c->row.p, c->col.p, counts.p, nullptr, nullptr);
   PD_CUDA_TRY(c, cudaGetLastError());
   if (cs->crow.count < (size_t)(n + 1)) PD_CUDA_TRY(c, cs->crow.alloc(n + 1));
   PD_CUDA_TRY(c, cudaMemsetAsync(counts.p + n, 0, sizeof(int64_t), c->stream));
@@ -266,9 +320,14 @@ static int contact_search(pd_ctx* c, const double4* pos) {
   PD_CUDA_TRY(c, cudaMemcpyAsync(&np, cs->crow.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
   PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if (cs->ccol.count < (size_t)std::max<int64_t>(np, 1)) PD_CUDA_TRY(c, cs->ccol.alloc((size_t)std::max<int64_t>(np, 1) * 5 / 4 + 16));
-  k_contact_search<true><<<gw, 256, 0, c->stream>>>(n, pos, g, cell_start.p, idx_s.p, cs->r_search, c->row.p,
-                                                    c->col.p, nullptr, cs->crow.p, cs->ccol.p);
+  k_contact_search<true><<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search,
+                                                    c->row.p, c->col.p, nullptr, cs->crow.p, cs->ccol.p);
+  PD_CUDA_TRY(c, cs->active.reserve(n));
+  PD_CUDA_TRY(c, cs->n_active.reserve(1));
+  PD_CUDA_TRY(c, dzero(c, cs->n_active.p, sizeof(int)));
+  k_contact_active<<<g1, 256, 0, c->stream>>>(n, cs->crow.p, cs->active.p, cs->n_active.p);
   PD_CUDA_TRY(c, cudaGetLastError());
+  cs->fc_follows = false;
   cs->npairs = np;
   cs->have_list = true;
   return PD_OK;
@@ -322,16 +381,23 @@ int contact_prepare(pd_ctx* c, int64_t step) {
   return contact_search(c, cs->pos.p);
 }
 
+static void launch_contact_force(pd_ctx* c, const ContactCoords& Y, const double* v, double* fc) {
+  const ContactState* cs = c->contact;
+  const unsigned g = (unsigned)std::min<int64_t>((c->n + 127) / 128, 4 * 148);
+  k_contact_force<<<g, 128, 0, c->stream>>>(cs->n_active.p, cs->active.p, cs->crow.p, cs->ccol.p, Y, v, c->xv.p,
+                                            cs->kappa.p, cs->r_contact, cs->friction, fc, c->status.p);
+}
+
 // Contact force density of the current configuration into c->fc.
 int contact_eval(pd_ctx* c) {
   ContactState* cs = c->contact;
   if (!cs) return PD_OK;
-  const int64_t n = c->n;
-  const unsigned g1 = (unsigned)((n + 255) / 256);
-  const double4* st = c->precision != PD_SPLIT_FP32 ? c->st[c->cur].p : nullptr;
-  k_contact_positions<<<g1, 256, 0, c->stream>>>(n, c->xv.p, c->u.p, st, cs->pos.p, cs->y.p);
-  k_contact_force<<<g1, 256, 0, c->stream>>>(n, cs->crow.p, cs->ccol.p, cs->y.p, c->v.p, c->xv.p, cs->kappa.p,
-                                             cs->r_contact, cs->friction, c->fc.p, c->status.p);
+  const bool split = c->precision == PD_SPLIT_FP32;
+  if (!cs->fc_follows) {  // the first evaluation with this list
+    PD_CUDA_TRY(c, dzero(c, c->fc.p, 3 * (size_t)c->n * sizeof(double)));
+    cs->fc_follows = true;
+  }
+  launch_contact_force(c, ContactCoords{nullptr, split ? nullptr : c->st[c->cur].p, c->xv.p, c->u.p}, c->v.p, c->fc.p);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;
 }
@@ -362,13 +428,13 @@ int contact_force_from(pd_ctx* c, const double* y_dev, const double* v_dev, doub
   ContactState* cs = c->contact;
   const int64_t n = c->n;
   const unsigned g1 = (unsigned)((n + 255) / 256);
+  PD_CUDA_TRY(c, dzero(c, fc_dev, 3 * (size_t)n * sizeof(double)));
   PD_CUDA_TRY(c, cudaMemcpyAsync(cs->y.p, y_dev, 3 * n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
   k_pos_from_y<<<g1, 256, 0, c->stream>>>(n, cs->y.p, cs->pos.p);
   PD_CUDA_TRY(c, cudaGetLastError());
   int rc = contact_search(c, cs->pos.p);
   if (rc != PD_OK) return rc;
-  k_contact_force<<<g1, 256, 0, c->stream>>>(n, cs->crow.p, cs->ccol.p, cs->y.p, v_dev, c->xv.p, cs->kappa.p,
-                                             cs->r_contact, cs->friction, fc_dev, c->status.p);
+  launch_contact_force(c, ContactCoords{cs->y.p, nullptr, c->xv.p, nullptr}, v_dev, fc_dev);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;
 }

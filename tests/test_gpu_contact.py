@@ -84,3 +84,32 @@ def test_plate_sphere_explicit_matches_oracle():
     assert np.array_equal(bd, ref["bond_damage"])
     assert np.abs(u - ref["u"]).max() <= 1e-9 * np.abs(ref["u"]).max()
     assert np.abs(v - ref["v"]).max() <= 1e-9 * np.abs(ref["v"]).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "split"])
+def test_contact_force_of_points_that_left_the_list_is_zero(precision):
+    """Only the points with a pair are visited: a call with other coordinates
+    (two bodies far apart, an empty list) between steps leaves no force behind."""
+    h = 1.0e-3
+    xa, va = workloads.lattice(4, 4, 3, h)
+    xb, vb = workloads.lattice(4, 4, 3, h, origin=(0.0, 0.0, 6.6 * h))
+    x, vol = np.concatenate([xa, xb]), np.concatenate([va, vb])
+    block = np.repeat([0, 1], len(va)).astype(np.int32)
+    u = np.zeros_like(x)
+    u[xa.size + 2::3] = -3.8 * h  # faces at 2.5 h and 7.1 h: 0.8 h apart
+    with Context(precision=precision) as ctx:
+        ctx.set_points(x, vol, block)
+        ctx.set_horizons([3.015 * h] * 2)
+        ctx.build_bonds()
+        for b in (0, 1):
+            ctx.material(130.0e9, 78.0e9, 7800.0, block=b)
+        ctx.contact(1.5 * h, 1000, 0.9 * h, 130.0e9)
+        ctx.set_state(u, np.zeros_like(x))
+        ctx.verlet_begin(1.0e-9)
+        ctx.verlet_step(2)
+        fc = ctx.field("Contact_Force_Density").reshape(-1, 3)
+        face = np.abs(fc[:, 2]) > 0
+        assert face.sum() == 32 and np.allclose(fc[face][:, 2].sum(), 0.0, atol=1e-6 * np.abs(fc).max())
+        assert not ctx.contact_force(x, np.zeros_like(x)).any()  # apart: no pair
+        ctx.verlet_step(1)
+        assert not ctx.field("Contact_Force_Density").any()
