@@ -382,6 +382,7 @@ int finalize_bonds(pd_ctx* c, bool sort_rows) {
   c->dmg_gen++;
   c->dmg_asym = c->phantoms;  // the two halves differ along every phantom bond
   c->chunk_hi_nb = -1;  // the upload chunks' neighbor bounds follow the bond set
+  c->small_threads = -1;
   PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->trial_valid = false;
   c->wv_done = false;

@@ -30,6 +30,7 @@
 #include <cub/cub.cuh>
 
 #include "fp64_math.cuh"
+#include "grid_sync.cuh"
 #include "pd_internal.cuh"
 
 namespace pdb {
@@ -1781,6 +1782,426 @@ __global__ void k_min_reduce(int64_t m, const double* __restrict__ partial, doub
 }
 
 // ---------------------------------------------------------------------------
+// Time steps of a small body in one cooperative launch
+//
+// At some thousand points a pass is a few dependent round trips to L2, and the
+// launches cost as much again. Where all lanes of a body are resident at once
+// and its bond stream fits the SMs' shared memory, a step is two phases
+// (dilatation, force and update) between grid barriers: the stream stays in
+// shared memory and each component's u and v in a register over the launch; a
+// phase gathers the neighbors' records and nothing else. Lanes per point and
+// the order of the sums are those of the general passes, so the results have
+// the same bits. 100x10x10 points, split: 26 -> 12 us a step; 27x7x6 points, FP64:
+// 19 -> 8 us.
+// ---------------------------------------------------------------------------
+struct SmallArgs {
+  int64_t n;
+  const int64_t* row;
+  const int64_t* soff;
+  const int32_t* col;  // split: the sliced stream's ids and damage; FP64: the CSR's
+  uint8_t* dmg;
+  uint8_t* dmg_csr;
+  const float* bx3;
+  Rec8* ur[2];
+  double4* st[2];
+  double4* ab64;
+  const double4* xv;
+  const double4* pt;
+  const float4* own;
+  const float* scf;
+  const double* sc;
+  float s_min;
+  double s_gate;
+  int damage_on, pair, cur;
+  int slots;  // bonds per lane in shared memory
+  double* theta;
+  double* node_damage;
+  EpiArgs E;  // f_out: of the last step
+  int64_t step0;
+  int nsteps, last;  // steps step0 .. step0 + nsteps - 1; last: the run ends with them
+  unsigned int* bar;
+};
+
+// One component of a point over the steps of a launch: verlet_epilogue's
+// arithmetic with u and v in registers (no contact, no prescribed functions).
+struct SmallDof {
+  double u = 0.0, v = 0.0, acc = 0.0, a = 0.0, b = 0.0;
+  bool held = false;
+  __device__ __forceinline__ void load(const EpiArgs& E, int64_t i, int c) {
+    const int64_t k = 3 * i + c;
+    u = E.u[k], v = E.v[k];
+    held = E.has_bc && ((E.bc_mask[i] >> c) & 1);
+    if (held) a = E.bc_a[k], b = E.bc_b[k];
+  }
+  // Completes step `step` with force density f and advances the state unless
+  // mode is EVAL_LAST; returns dt*v, the increment of u.
+  __device__ __forceinline__ double advance(const EpiArgs& E, int64_t k, int64_t step, int mode, double f, double rho) {
+    if (!isfinite(f)) atomicOr(E.status, ST_NONFINITE_FORCE);
+    const double dt = E.dt, dt2 = E.dt / 2.0;
+    acc = __ddiv_rn(__dadd_rn(f, 0.0), rho);
+    if (step > 0) v = __dadd_rn(v, __dmul_rn(dt2, acc));
+    if (mode == EVAL_LAST) {
+      if (E.f_out) E.f_out[k] = f;
+      return 0.0;
+    }
+    double vh = __dadd_rn(v, __dmul_rn(dt2, acc));
+    if (held) {
+      const double tc = __dadd_rn(E.t0, __dmul_rn((double)(step + 1), dt));
+      const double tp = step == 0 ? E.t0 : __dadd_rn(E.t0, __dmul_rn((double)step, dt));
+      if (tc != tp) {
+        const double cur = __dadd_rn(__dmul_rn(a, tc), b), prev = __dadd_rn(__dmul_rn(a, tp), b);
+        double d = __dsub_rn(cur, prev);
+        if (d == 0.0) d = __dsub_rn(cur, u);
+        vh = __dadd_rn(__dmul_rn(0.0, d), __dmul_rn(__dmul_rn(1.0, d), __ddiv_rn(1.0, __dsub_rn(tc, tp))));
+        if (!isfinite(vh)) atomicOr(E.status, ST_NONFINITE_BC);
+      }
+    }
+    v = vh;
+    const double dx = __dmul_rn(dt, vh);
+    u = __dadd_rn(u, dx);
+    return dx;
+  }
+  __device__ __forceinline__ void store(const EpiArgs& E, int64_t k) const { E.u[k] = u, E.v[k] = v, E.a[k] = acc; }
+};
+
+// Records another block may have written before the last grid barrier.
+__device__ __forceinline__ Rec8 ld_rec_sync(const Rec8* p) {
+  Rec8 r;
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]),
+                 "=f"(r.v[7])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ double4 ld_f64x4_sync(const double4* p) {
+  double4 r;
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
+// Threads per block, one block per SM: 128 registers a thread.
+constexpr int kSmallBlock = 512;
+#ifndef PD_SMALL_BATCH
+#define PD_SMALL_BATCH 6
+#endif
+#ifndef PD_SMALL64_BATCH
+#define PD_SMALL64_BATCH 4
+#endif
+// Bytes of shared memory per thread and bond: (X, id) and damage; FP64: |X|, V, id and damage.
+constexpr int kSmallBond = 17, kSmallBond64 = 21;
+
+template <bool PAIR>
+__global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs A) {
+  constexpr int K = PD_SMALL_BATCH;
+  extern __shared__ __align__(16) unsigned char small_sm[];
+  const int T = blockDim.x, tid = threadIdx.x;
+  float4* sx = reinterpret_cast<float4*>(small_sm) + tid;             // bond t at sx[t T]
+  uint8_t* sd = small_sm + (size_t)16 * A.slots * T + tid;            // its damage at sd[t T]
+  const int64_t i = ((int64_t)blockIdx.x * T + tid) / 4;
+  const int lane = tid & 3;
+  const bool valid = i < A.n;
+  // the lane's groups of its slice (a warp is one slice: G is the warp's)
+  const int64_t sl = min(i, A.n - 1) >> 3, so = A.soff[sl];
+  const int G = (int)(A.soff[sl + 1] - so), full = G & ~3, l32 = (int)(i & 7) * 4 + lane;
+  auto slot_of = [&](int g) { return g < full ? 32 * (so + (g & ~3)) + 4 * l32 + (g & 3) : 32 * (so + g) + l32; };
+  for (int g = 0; g < A.slots; ++g) {
+    float4 v = make_float4(1.0f, 0.0f, 0.0f, __int_as_float((int)min(i, A.n - 1)));
+    uint8_t d = kDummyBond;
+    if (valid && g < G) {
+      const int64_t k = slot_of(g);
+      const float* px = A.bx3 + (g < full ? 96 * (so + (g & ~3)) + 4 * l32 + (g & 3) : 96 * (so + g) + l32);
+      const int plane = g < full ? 128 : 32;
+      v = make_float4(px[0], px[plane], px[2 * plane], __int_as_float(A.col[k]));
+      d = A.dmg[k];
+    }
+    sx[g * T] = v;
+    sd[g * T] = d;
+  }
+  int64_t b0 = 0;
+  int len = 0;
+  float4 ow = make_float4(0.f, 0.f, 0.f, -1.f);
+  double rho = 1.0;
+  SmallDof dof;
+  if (valid) {
+    b0 = A.row[i];
+    len = (int)(A.row[i + 1] - b0);
+    ow = A.own[i];
+    rho = A.pt[i].w;
+    if (lane < 3) dof.load(A.E, i, lane);
+  }
+  const float s_c = A.damage_on ? ow.w : -1.0f;
+  int cur = A.cur;
+  for (int t = 0; t < A.nsteps; ++t) {
+    Rec8* ur = A.ur[cur];
+    const OwnU ui = own_u(ld_rec_sync(ur + min(i, A.n - 1)));
+    float th = 0.0f;
+    int broken = 0;
+    for (int g0 = 0; g0 < G; g0 += K) {
+      float4 X[K];
+      int d[K];
+      Rec8 uj[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int g = g0 + k < G ? g0 + k : g0;
+        X[k] = sx[g * T];
+        d[k] = g0 + k < G ? sd[g * T] : kDummyBond;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) uj[k] = ld_rec_sync(ur + __float_as_int(X[k].w));
+#pragma unroll
+      for (int k = 0; k < K; ++k) {  // as k_dilatation_split
+        const SplitBond sb = split_bond<false>(X[k].x, X[k].y, X[k].z, ui, uj[k]);
+        const bool own_ok = (d[k] & 5) == 0;
+        bool brk = false, brkp = false;
+        if (PAIR) {
+          if (A.damage_on && sb.e > A.s_min * sb.zeta) {
+            brk = own_ok && s_c >= 0.0f && sb.e > s_c * sb.zeta;
+            if ((d[k] & 6) == 0) {
+              const float scj = __ldg(A.scf + __float_as_int(X[k].w));
+              brkp = scj >= 0.0f && sb.e > scj * sb.zeta;
+            }
+          }
+        } else {
+          brk = brkp = own_ok && s_c >= 0.0f && sb.e > s_c * sb.zeta;
+        }
+        if (brk || brkp) {
+          const uint8_t nd = (uint8_t)(d[k] | (brk ? 1 : 0) | (brkp ? 2 : 0));
+          sd[(g0 + k) * T] = nd;
+          A.dmg[slot_of(g0 + k)] = nd;
+          A.dmg_csr[b0 + lane + 4 * (g0 + k)] = nd;
+        }
+        broken += ((d[k] & 1) || brk) ? 1 : 0;
+        // (a bond past the lane's last adds nothing: its product is not taken)
+        if (g0 + k < G) th = fmaf((own_ok && !brk) ? uj[k].v[5] * sb.zeta : 0.0f, sb.e, th);
+      }
+    }
+    th = group_sum<4>(th);
+    broken = group_sum<4>(broken);
+    if (valid && lane == 0) {
+      const float theta = th * ow.x;
+      *reinterpret_cast<float2*>(&ur[i].v[6]) = make_float2(theta * ow.y, ow.z);
+      A.theta[i] = (double)theta;
+      A.node_damage[i] = len > 0 ? (double)broken / (double)len : 0.0;
+    }
+    if (!grid_sync(A.bar, A.E.status)) return;
+    const Rec8 ri = ld_rec_sync(ur + min(i, A.n - 1));
+    const float Ai = ri.v[6], Bi = ri.v[7];
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    for (int g0 = 0; g0 < G; g0 += K) {
+      float4 X[K];
+      int d[K];
+      Rec8 uj[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int g = g0 + k < G ? g0 + k : g0;
+        X[k] = sx[g * T];
+        d[k] = g0 + k < G ? sd[g * T] : kDummyBond;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) uj[k] = ld_rec_sync(ur + __float_as_int(X[k].w));
+#pragma unroll
+      for (int k = 0; k < K; ++k) {  // as k_force_split
+        const SplitBond sb = split_bond<true>(X[k].x, X[k].y, X[k].z, ui, uj[k]);
+        float wv = uj[k].v[5];
+        float a = Ai + uj[k].v[6], b = Bi + uj[k].v[7];
+        if (PAIR) {
+          if (d[k] != 0) {
+            const bool own_live = (d[k] & 5) == 0, part_live = (d[k] & 6) == 0;
+            a = (own_live ? Ai : 0.0f) + (part_live ? uj[k].v[6] : 0.0f);
+            b = (own_live ? Bi : 0.0f) + (part_live ? uj[k].v[7] : 0.0f);
+          }
+        } else {
+          wv = d[k] == 0 ? wv : 0.0f;
+        }
+        const float w = fmaf(sb.zeta, a, sb.e * b) * wv * sb.ry;
+        if (g0 + k < G) {
+          fx = fmaf(w, sb.Yx, fx);
+          fy = fmaf(w, sb.Yy, fy);
+          fz = fmaf(w, sb.Yz, fz);
+        }
+      }
+    }
+    fx = group_sum<4>(fx);
+    fy = group_sum<4>(fy);
+    fz = group_sum<4>(fz);
+    const int mode = A.last && t == A.nsteps - 1 ? EVAL_LAST : EVAL_ADVANCE;
+    if (valid && lane < 3)
+      dof.advance(A.E, 3 * i + lane, A.step0 + t, mode, (double)(lane == 0 ? fx : (lane == 1 ? fy : fz)), rho);
+    if (mode == EVAL_ADVANCE) store_u_record_group<4>(A.ur[cur ^ 1] + i, lane, dof.u, valid);
+    if (t + 1 < A.nsteps && !grid_sync(A.bar, A.E.status)) return;
+    cur ^= 1;
+  }
+  if (valid && lane < 3) dof.store(A.E, 3 * i + lane);
+}
+
+// The same in FP64, the reference's operation order, 16 lanes per point;
+// |X| of a bond is constant and stays in shared memory with V.
+__global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_fp64(SmallArgs A) {
+  constexpr int L = 16, K = PD_SMALL64_BATCH;
+  extern __shared__ __align__(16) unsigned char small_sm[];
+  const int T = blockDim.x, tid = threadIdx.x, S = A.slots;
+  double* sz = reinterpret_cast<double*>(small_sm) + tid;
+  double* sv = reinterpret_cast<double*>(small_sm) + (size_t)S * T + tid;
+  int32_t* sj = reinterpret_cast<int32_t*>(small_sm + (size_t)16 * S * T) + tid;
+  uint8_t* sd = small_sm + (size_t)20 * S * T + tid;
+  const int64_t i = ((int64_t)blockIdx.x * T + tid) / L;
+  const int lane = tid & (L - 1);
+  const bool valid = i < A.n;
+  const int64_t ic = min(i, A.n - 1);
+  const int64_t b0 = A.row[ic], b1 = A.row[ic + 1];
+  const int len = (int)(b1 - b0);
+  const double4 p = A.pt[ic], xi = A.xv[ic];
+  for (int t = 0; t < S; ++t) {
+    double zeta = 1.0, V = 0.0;
+    int32_t j = (int32_t)ic;
+    uint8_t d = kDummyBond | 3;
+    const int64_t b = b0 + lane + t * L;
+    if (valid && b < b1) {
+      j = A.col[b];
+      const double4 xj = A.xv[j];
+      zeta = __dsqrt_rn(sq3_rn(__dsub_rn(xj.x, xi.x), __dsub_rn(xj.y, xi.y), __dsub_rn(xj.z, xi.z)));
+      V = xj.w;
+      d = A.dmg[b];
+    }
+    sz[t * T] = zeta, sv[t * T] = V, sj[t * T] = j, sd[t * T] = d;
+  }
+  const bool m_in = root_in_range(p.x);
+  const double rm = __drcp_rn(p.x);
+  const double s_c = A.damage_on ? A.sc[ic] : -1.0;
+  const double gate = A.damage_on ? A.s_gate : INFINITY;
+  SmallDof dof;
+  if (valid && lane < 3) dof.load(A.E, i, lane);
+  const double xc = comp3(xi, lane);
+  int cur = A.cur;
+  for (int t = 0; t < A.nsteps; ++t) {
+    const double4* st = A.st[cur];
+    const double4 yi = ld_f64x4_sync(st + ic);
+    double th = 0.0;
+    int broken = 0;
+    for (int t0 = 0; t0 < S; t0 += K) {  // as k_dilatation_fp64
+      double zeta[K], e[K], yy[K], q[K], V[K];
+      int d[K], j[K];
+      double4 yj[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int s = (t0 + k < S ? t0 + k : t0) * T;
+        j[k] = sj[s], zeta[k] = sz[s], V[k] = sv[s];
+        d[k] = t0 + k < S ? sd[s] : kDummyBond | 3;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) yj[k] = ld_f64x4_sync(st + j[k]);
+      bool odd = !m_in, hot = false;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double y2 = sq3_rn(__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z));
+        yy[k] = (d[k] & 3) != 3 ? y2 : 1.0;
+        e[k] = __dsub_rn(root_d(yy[k]).root, zeta[k]);
+        q[k] = quotient_d(__dmul_rn(__dmul_rn(__dmul_rn(3.0, zeta[k]), e[k]), V[k]), p.x, rm);
+        odd |= !root_in_range(yy[k]);
+      }
+      if (odd)
+        for (int k = 0; k < K; ++k) {
+          e[k] = __dsub_rn(__dsqrt_rn(yy[k]), zeta[k]);
+          q[k] = __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(3.0, zeta[k]), e[k]), V[k]), p.x);
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) hot |= e[k] > gate * zeta[k];
+      if (hot)
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if ((d[k] & 3) == 3) continue;
+          const double scj = A.pair ? A.sc[j[k]] : s_c;
+          const double rel = __ddiv_rn(e[k], zeta[k]);
+          const bool brk = !(d[k] & 1) && s_c >= 0.0 && rel > s_c;
+          const bool brkp = !(d[k] & 2) && scj >= 0.0 && rel > scj;
+          if (brk || brkp) {
+            d[k] |= (brk ? 1 : 0) | (brkp ? 2 : 0);
+            sd[(t0 + k) * T] = (uint8_t)d[k];
+            A.dmg[b0 + lane + (t0 + k) * L] = (uint8_t)d[k];
+          }
+        }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        broken += (d[k] & (kDummyBond | 1)) == 1 ? 1 : 0;
+        if (!(d[k] & 1)) th = __dadd_rn(th, q[k]);
+      }
+    }
+    th = group_sum<L>(th);
+    broken = group_sum<L>(broken);
+    if (valid && lane == 0) {
+      const double alpha = __ddiv_rn(__dmul_rn(15.0, p.z), p.x);
+      const double q = __dsub_rn(__ddiv_rn(__dmul_rn(3.0, p.y), p.x), __ddiv_rn(alpha, 3.0));
+      A.ab64[i] = make_double4(th, q, alpha, __dmul_rn(th, q));
+      A.theta[i] = th;
+      A.node_damage[i] = len > 0 ? (double)broken / (double)len : 0.0;
+    }
+    if (!grid_sync(A.bar, A.E.status)) return;
+    const double4 ai = ld_f64x4_sync(A.ab64 + ic);
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int t0 = 0; t0 < S; t0 += K / 2) {  // as k_force_fp64
+      constexpr int H = K / 2;
+      double zeta[H], V[H], yy[H], Y[H][3], fi[H][3], fj[H][3];
+      int d[H], j[H];
+      double4 yj[H], aj[H];
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+        const int s = (t0 + k < S ? t0 + k : t0) * T;
+        j[k] = sj[s], zeta[k] = sz[s], V[k] = sv[s];
+        d[k] = t0 + k < S ? sd[s] & 3 : 3;
+      }
+#pragma unroll
+      for (int k = 0; k < H; ++k) yj[k] = ld_f64x4_sync(st + j[k]), aj[k] = ld_f64x4_sync(A.ab64 + j[k]);
+      bool odd = false;
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+        Y[k][0] = __dsub_rn(yj[k].x, yi.x), Y[k][1] = __dsub_rn(yj[k].y, yi.y), Y[k][2] = __dsub_rn(yj[k].z, yi.z);
+        const double y2 = sq3_rn(Y[k][0], Y[k][1], Y[k][2]);
+        yy[k] = d[k] != 3 ? y2 : 1.0;
+        odd |= !root_in_range(yy[k]);
+        const RootD r = root_d(yy[k]);
+        const double e = __dsub_rn(r.root, zeta[k]), rd = recip_d(r.root, r.inv);
+        const double ti = __dadd_rn(__dmul_rn(ai.w, zeta[k]), __dmul_rn(ai.z, e));
+        const double tj = __dadd_rn(__dmul_rn(aj[k].w, zeta[k]), __dmul_rn(aj[k].z, e));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          fi[k][c] = quotient_d(__dmul_rn(ti, Y[k][c]), r.root, rd);
+          fj[k][c] = quotient_d(__dmul_rn(tj, Y[k][c]), r.root, rd);
+        }
+      }
+      if (odd)
+        for (int k = 0; k < H; ++k) {
+          const double dY = __dsqrt_rn(yy[k]), e = __dsub_rn(dY, zeta[k]);
+          const double ti = __dadd_rn(__dmul_rn(ai.w, zeta[k]), __dmul_rn(ai.z, e));
+          const double tj = __dadd_rn(__dmul_rn(aj[k].w, zeta[k]), __dmul_rn(aj[k].z, e));
+          for (int c = 0; c < 3; ++c) {
+            fi[k][c] = __ddiv_rn(__dmul_rn(ti, Y[k][c]), dY);
+            fj[k][c] = __ddiv_rn(__dmul_rn(tj, Y[k][c]), dY);
+          }
+        }
+#pragma unroll
+      for (int k = 0; k < H; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (!(d[k] & 1)) f[c] = __dadd_rn(f[c], __dmul_rn(fi[k][c], V[k]));
+          if (!(d[k] & 2)) f[c] = __dadd_rn(f[c], __dmul_rn(fj[k][c], V[k]));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = group_sum<L>(f[c]);
+    const int mode = A.last && t == A.nsteps - 1 ? EVAL_LAST : EVAL_ADVANCE;
+    if (valid && lane < 3) {
+      const double u0 = dof.u;
+      const double dx = dof.advance(A.E, 3 * i + lane, A.step0 + t, mode, lane == 0 ? f[0] : (lane == 1 ? f[1] : f[2]), p.w);
+      if (mode == EVAL_ADVANCE) *comp_ptr(&A.st[cur ^ 1][i], lane) = __dadd_rn(__dadd_rn(xc, u0), dx);  // y = x+u+dt*v
+    }
+    if (t + 1 < A.nsteps && !grid_sync(A.bar, A.E.status)) return;
+    cur ^= 1;
+  }
+  if (valid && lane < 3) dof.store(A.E, 3 * i + lane);
+}
+
+// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 static inline unsigned grid_for(int64_t n, int tpo) { return (unsigned)((n * tpo + kBlock - 1) / kBlock); }
@@ -2243,6 +2664,112 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
   }
   if (ev) cudaEventRecord(ev[2], c->stream);
   return cudaGetLastError();
+}
+
+static const void* small_kernel(const pd_ctx* c, bool pair) {
+  if (c->precision == PD_FP64) return (const void*)&k_verlet_small_fp64;
+  return pair ? (const void*)&k_verlet_small_split<true> : (const void*)&k_verlet_small_split<false>;
+}
+
+// Whether steps of this context run as one cooperative launch: LPS with
+// omega = 1 on the default lane counts, nothing between the passes (contact,
+// prescribed functions, kernel timing, phantom halves), and one block per SM
+// with its bonds in shared memory (split: to about 13,000 points of 123 bonds,
+// FP64: to about 4,700).
+bool small_steps(pd_ctx* c) {
+  if (c->n == 0 || c->material_model != PD_MATERIAL_LPS || c->influence != PD_INFLUENCE_ONE || c->contact ||
+      c->n_bc_expr || c->ktime || c->phantoms)
+    return false;
+  if (c->small_threads >= 0 && c->small_row == c->row.p && c->small_nb == c->nb) return c->small_threads > 0;
+  // once per bond set
+  c->small_threads = 0;
+  c->small_row = c->row.p;
+  c->small_nb = c->nb;
+  const bool f64 = c->precision == PD_FP64;
+  if (!(f64 && c->tpo == 16) && !(c->precision == PD_SPLIT_FP32 && c->sell && c->tpo_split == 4)) return false;
+  const int lanes = f64 ? 16 : 4, bond = f64 ? kSmallBond64 : kSmallBond;
+  int sms = 0, coop = 0, smem = 0, per = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess || !coop)
+    return false;
+  // whole warps per SM, the lanes spread evenly
+  const int64_t threads = ((c->n * lanes + sms - 1) / sms + 31) / 32 * 32;
+  const int64_t slots = (c->max_row + lanes - 1) / lanes;
+  const int64_t bytes = (threads * slots * bond + 15) / 16 * 16;
+  if (threads > kSmallBlock || slots == 0 || bytes > smem - 1024) return false;
+  for (int pair = 0; pair < 2; ++pair) {
+    const void* k = small_kernel(c, pair != 0);
+    // (one value for every context, whatever it needs: the attribute is the kernel's)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, (int)threads, (size_t)bytes) != cudaSuccess || per < 1) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  c->small_threads = (int)threads;
+  c->small_slots = (int)slots;
+  c->small_bytes = (int)bytes;
+  return true;
+}
+
+// Steps step0 .. step0 + nsteps - 1 (the last one of the run: last) from the
+// state of parity c->cur, on the committed damage; c->cur follows.
+cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int nsteps, bool last) {
+  const bool split = c->precision == PD_SPLIT_FP32, pair = c->sc_pair || c->dmg_asym;
+  if (split && (c->sell_src != c->dmg.p || c->sell_gen != c->dmg_gen)) {
+    k_sell_dmg<<<grid_for(c->n, 4), kBlock, 0, c->stream>>>(c->n, c->row.p, c->sell_off.p, c->dmg.p, c->sell_dmg.p);
+    c->sell_src = c->dmg.p;
+    c->sell_gen = c->dmg_gen;
+  }
+  if (c->small_bar.count < 2) TRY_CUDA(c->small_bar.alloc(2));
+  TRY_CUDA(dzero(c, c->small_bar.p, 2 * sizeof(unsigned int)));
+  SmallArgs A{};
+  A.n = c->n;
+  A.row = c->row.p;
+  A.soff = c->sell_off.p;
+  A.col = split ? c->sell_col.p : c->col.p;
+  A.dmg = split ? c->sell_dmg.p : c->dmg.p;
+  A.dmg_csr = c->dmg.p;
+  A.bx3 = c->bx3.p;
+  for (int k = 0; k < 2; ++k) A.ur[k] = c->ur[k].p, A.st[k] = c->st[k].p;
+  A.ab64 = c->ab64.p;
+  A.xv = c->xv.p;
+  A.pt = c->pt.p;
+  A.own = c->own.p;
+  A.scf = c->scf.p;
+  A.sc = c->sc.p;
+  A.s_min = c->sc_min;
+  A.s_gate = c->sc_gate64;
+  A.damage_on = sp.damage_on;
+  A.pair = pair;
+  A.cur = c->cur;
+  A.slots = c->small_slots;
+  A.theta = c->theta.p;
+  A.node_damage = c->node_damage.p;
+  A.E.dt = sp.dt;
+  A.E.t0 = sp.t0;
+  A.E.has_bc = sp.has_bc;
+  A.E.split = split;
+  A.E.f_out = last ? c->f.p : nullptr;
+  A.E.u = c->u.p;
+  A.E.v = c->v.p;
+  A.E.a = c->a.p;
+  A.E.bc_mask = c->bc_mask.p;
+  A.E.bc_a = c->bc_a.p;
+  A.E.bc_b = c->bc_b.p;
+  A.E.status = c->status.p;
+  A.step0 = step0;
+  A.nsteps = nsteps;
+  A.last = last;
+  A.bar = c->small_bar.p;
+  const int lanes = split ? 4 : 16, T = c->small_threads;
+  const void* k = small_kernel(c, pair);
+  void* args[] = {&A};
+  TRY_CUDA(cudaLaunchCooperativeKernel(k, dim3((unsigned)((c->n * lanes + T - 1) / T)), dim3(T), args,
+                                       (size_t)c->small_bytes, c->stream));
+  c->cur ^= (nsteps - (last ? 1 : 0)) & 1;
+  return cudaSuccess;
 }
 
 // Node damage over the points' own families (phantom halves are neither

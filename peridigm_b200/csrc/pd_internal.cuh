@@ -221,6 +221,14 @@ struct pd_ctx {
   int64_t vstep = 0;
   cudaEvent_t vbeg = nullptr;
 
+  // steps in one cooperative launch: threads per block (0: the general passes,
+  // -1: not determined), bonds per lane and bytes of shared memory per block,
+  // for the bond set of (small_row, small_nb)
+  int small_threads = -1, small_slots = 0, small_bytes = 0;
+  const int64_t* small_row = nullptr;
+  int64_t small_nb = -1;
+  pdb::DBuf<unsigned int> small_bar;  // its grid barrier
+
   // boundary conditions
   std::vector<uint8_t> h_bc_mask;
   std::vector<double> h_bc_a, h_bc_b;
@@ -288,6 +296,10 @@ int64_t critical_dt_partials(const pd_ctx* c);
 cudaError_t launch_critical_dt_into(pd_ctx* c, double* partial, double* dt_out_dev);
 cudaError_t collect_kernel_times(pd_ctx* c);
 cudaError_t launch_fp64_eval_at(pd_ctx* c, const double4* y4, double4* ab, double* theta, double* nd, double* f_out);
+// Verlet steps of a small body in one cooperative launch (k_lps.cu).
+bool small_steps(pd_ctx* c);
+cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int nsteps, bool last);
+constexpr int kSmallSteps = 1024;  // steps per launch
 int ensure_ready_internal(pd_ctx* c);
 
 // quasi-static (k_qs.cu) and the learned preconditioner (k_mpnn.cu)
