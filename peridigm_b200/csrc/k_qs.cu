@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "cg.cuh"
+#include "grid_sync.cuh"
 #include "pd_internal.cuh"
 
 namespace pdb {
@@ -72,6 +73,7 @@ struct QsState {
   DBuf<CgCtl> ctl;           // scalars and state of the running solve
   CgReport* report = nullptr;      // its progress, in mapped pinned memory
   CgReport* report_dev = nullptr;
+  int small_lanes = -1;  // of the one-launch solve (-1: not determined, 0: the general loop)
   ~QsState() {
     if (report) cudaFreeHost(report);
   }
@@ -300,6 +302,13 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
   }
   double sum[1] = {pq};
   if (cg_grid_sum<1, kQsBlock>(sum, partial, &ctl->ticket[0]) && threadIdx.x == 0) ctl->pq = sum[0];
+}
+
+// 256-bit load of a record that no thread writes during the kernel.
+__device__ __forceinline__ double4 ld_point_nc(const double4* p) {
+  double4 r;
+  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
 }
 
 // Inverse 3x3 diagonal blocks of K (prescribed rows/columns set to identity).
@@ -567,6 +576,188 @@ __global__ void k_cg_direction(int64_t n, const double* __restrict__ z, double4*
   }
 }
 
+// ---------------------------------------------------------------------------
+// A whole CG solve of a small body in one cooperative launch (no
+// preconditioner or block Jacobi). Where every lane of the tangent passes is
+// resident at once, an iteration is four phases between grid barriers: p
+// published, q dtheta, K p with p.q, the update with the dot products. At some
+// thousand points a phase is one or two round trips to L2, and the launches of
+// the general loop cost several times that. Lanes 0-2 of a point keep x, r and
+// p of their component in registers; every block adds the blocks' partial sums
+// in the same order, so all of them see the same scalars and stop together.
+// ---------------------------------------------------------------------------
+// A point's (p, q dtheta) that another block may have written before the last barrier.
+__device__ __forceinline__ double4 ld_w_sync(const double4* p) {
+  double4 r;
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
+// Sums over the grid: this block's to partial[NV blk ..], a barrier, then all
+// partials in block order. False when the barrier's wait ran out.
+template <int NV>
+__device__ __forceinline__ bool cg_sum_sync(double (&v)[NV], double* partial, unsigned int* bar, int* status) {
+  __shared__ double sh[NV][kQsBlock / 32];
+  cg_block_sum<NV, kQsBlock>(v, sh);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) partial[(size_t)NV * blockIdx.x + k] = v[k];
+  if (!grid_sync(bar, status)) return false;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+#pragma unroll 4
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += kQsBlock)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += __ldcg(partial + (size_t)NV * b + k);
+  cg_block_sum<NV, kQsBlock>(v, sh);
+  return true;
+}
+
+struct CgSmallArgs {
+  int64_t n;
+  const int64_t* row;
+  const int32_t* col;
+  const double4* g;
+  const double2* gc;
+  const double4* ab;
+  const double4* pt;
+  const double4* xv;
+  const uint8_t* fixed;
+  const double* dinv;  // null: no preconditioner
+  const double* r;     // right-hand side
+  double* x;           // solution
+  double4* w;
+  double* partial;
+  double jk, jm, tol;
+  long long max_it;
+  CgCtl* ctl;
+  unsigned int* bar;
+  int* status;
+};
+
+template <int TPO>
+__global__ void __launch_bounds__(kQsBlock, 3) k_cg_small(CgSmallArgs A) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / TPO;
+  const int lane = threadIdx.x & (TPO - 1);
+  const bool valid = i < A.n, dof = valid && lane < 3;
+  int64_t b0 = 0, b1 = 0;
+  double s = 0.0, V = 0.0, rho = 0.0, D[3] = {0.0, 0.0, 0.0};
+  bool held = false;
+  double r = 0.0, x = 0.0, p = 0.0;
+  if (valid) {
+    b0 = A.row[i];
+    b1 = A.row[i + 1];
+    const double4 m = A.pt[i];
+    s = 3.0 * (A.ab[i].y / m.x);
+    V = A.xv[i].w;
+    rho = m.w;
+  }
+  if (dof) {
+    held = (A.fixed[i] >> lane) & 1;
+    r = A.r[3 * i + lane];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) D[c] = A.dinv ? A.dinv[9 * i + 3 * lane + c] : (c == lane ? 1.0 : 0.0);
+  }
+  double* part_pq = A.partial + 2 * (size_t)gridDim.x;
+  auto precond = [&](double rv) {  // lanes 0-2: their component of P r
+    const double r0 = __shfl_sync(0xffffffffu, rv, 0, TPO), r1 = __shfl_sync(0xffffffffu, rv, 1, TPO),
+                 r2 = __shfl_sync(0xffffffffu, rv, 2, TPO);
+    return A.dinv ? D[0] * r0 + D[1] * r1 + D[2] * r2 : rv;
+  };
+  double z = precond(r);
+  double dots[2] = {dof ? r * z : 0.0, dof ? r * r : 0.0};
+  if (!cg_sum_sync<2>(dots, A.partial, A.bar, A.status)) return;
+  const double rr0 = dots[1];
+  double rz = dots[0], rel = 1.0;
+  int state = rr0 == 0.0 ? CG_ZERO_RHS : CG_RUNNING;
+  if (rr0 == 0.0) rel = 0.0;
+  long long it = 0;
+  p = z;
+  while (state == CG_RUNNING && it < A.max_it) {
+    if (dof) (lane == 0 ? A.w[i].x : (lane == 1 ? A.w[i].y : A.w[i].z)) = p;
+    if (!grid_sync(A.bar, A.status)) return;
+    // tangent pass 1 (k_qs_dtheta_g)
+    const double p0 = __shfl_sync(0xffffffffu, p, 0, TPO), p1 = __shfl_sync(0xffffffffu, p, 1, TPO),
+                 p2 = __shfl_sync(0xffffffffu, p, 2, TPO);
+    double acc = 0.0;
+    if (valid)
+      for (int64_t b = b0 + lane; b < b1; b += 4 * TPO) {
+        double4 gb[4], wj[4];
+        int32_t j[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool in = b + k * TPO < b1;
+          j[k] = in ? __ldg(A.col + b + k * TPO) : (int32_t)i;
+          gb[k] = in ? ld_point_nc(A.g + b + k * TPO) : make_double4(0.0, 0.0, 0.0, 0.0);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) wj[k] = ld_w_sync(A.w + j[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          acc += gb[k].w * (gb[k].x * (wj[k].x - p0) + gb[k].y * (wj[k].y - p1) + gb[k].z * (wj[k].z - p2));
+      }
+    acc = s * qs_group_sum<TPO>(acc);
+    if (valid && lane == 0) A.w[i].w = acc;
+    if (!grid_sync(A.bar, A.status)) return;
+    // tangent pass 2 (k_qs_df_g)
+    double d[3] = {0.0, 0.0, 0.0};
+    if (valid)
+      for (int64_t b = b0 + lane; b < b1; b += 2 * TPO) {
+        double4 gb[2], wj[2];
+        double2 cb[2];
+        int32_t j[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const bool in = b + k * TPO < b1;
+          j[k] = in ? __ldg(A.col + b + k * TPO) : (int32_t)i;
+          gb[k] = in ? ld_point_nc(A.g + b + k * TPO) : make_double4(0.0, 0.0, 0.0, 0.0);
+          cb[k] = in ? __ldg(A.gc + b + k * TPO) : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) wj[k] = ld_w_sync(A.w + j[k]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const double w0 = wj[k].x - p0, w1 = wj[k].y - p1, w2 = wj[k].z - p2;
+          const double de = gb[k].x * w0 + gb[k].y * w1 + gb[k].z * w2;
+          const double sy = gb[k].w * (acc + wj[k].w) + (cb[k].y - cb[k].x) * de;
+          d[0] += sy * gb[k].x + cb[k].x * w0;
+          d[1] += sy * gb[k].y + cb[k].x * w1;
+          d[2] += sy * gb[k].z + cb[k].x * w2;
+        }
+      }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d[c] = qs_group_sum<TPO>(d[c]);
+    double q = 0.0;
+    if (dof) {
+      q = -V * (lane == 0 ? d[0] : (lane == 1 ? d[1] : d[2]));
+      if (A.jm != 0.0) q = A.jm * rho * p + A.jk * q;  // implicit dynamics: (rho I + beta dt^2 K) p
+      if (held) q = p;
+    }
+    double pq[1] = {p * q};
+    if (!cg_sum_sync<1>(pq, part_pq, A.bar, A.status)) return;
+    const double alpha = rz / pq[0];
+    x += alpha * p;
+    r -= alpha * q;
+    z = precond(r);
+    dots[0] = dof ? r * z : 0.0;
+    dots[1] = dof ? r * r : 0.0;
+    if (!cg_sum_sync<2>(dots, A.partial, A.bar, A.status)) return;
+    rel = sqrt(dots[1]) / sqrt(rr0);
+    ++it;
+    if (!isfinite(rel)) state = CG_NONFINITE;
+    else if (rel <= A.tol) state = CG_CONVERGED;
+    p = z + (dots[0] / rz) * p;
+    rz = dots[0];
+  }
+  if (state == CG_RUNNING) state = CG_MAX_ITERATIONS;
+  if (dof) A.x[3 * i + lane] = x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.ctl->it = it;
+    A.ctl->rel = rel;
+    A.ctl->state = state;
+  }
+}
+
 // The start of a solve (state, tolerance, where the report goes).
 __global__ void k_cg_begin(CgCtl* ctl, double tol, long long max_it, CgReport* report) {
   ctl->state = CG_RUNNING;
@@ -610,6 +801,7 @@ static int qs_alloc(pd_ctx* c) {
   PD_CUDA_TRY(c, s->scal.alloc(16));
   PD_CUDA_TRY(c, s->fixed.alloc(n));
   PD_CUDA_TRY(c, dzero(c, s->pred.p, s->pred.bytes()));
+  s->small_lanes = -1;
   s->n = n;
   return PD_OK;
 }
@@ -864,6 +1056,74 @@ static int cg_wait(pd_ctx* c, long long it, CgReport* out) {
   }
 }
 
+// Lanes per point of the one-launch solve; 0 when the body's lanes are not all
+// resident (or the device takes no cooperative launches).
+static int cg_small_lanes(pd_ctx* c) {
+  QsState* s = c->qs;
+  if (s->small_lanes < 0) {
+    int sms = 0, coop = 0, per = 0;
+    s->small_lanes = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop) {
+      auto fits = [&](const void* k, int L) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kQsBlock, 0) == cudaSuccess &&
+               c->n * L <= (int64_t)per * sms * kQsBlock;
+      };
+      if (fits((const void*)&k_cg_small<32>, 32)) s->small_lanes = 32;
+      else if (fits((const void*)&k_cg_small<16>, 16)) s->small_lanes = 16;
+      else if (fits((const void*)&k_cg_small<8>, 8)) s->small_lanes = 8;
+    }
+  }
+  return s->small_lanes;
+}
+
+static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out, int lanes) {
+  QsState* s = c->qs;
+  TRY_RC(qs_geometry(c));
+  if (c->small_bar.count < 2) PD_CUDA_TRY(c, c->small_bar.alloc(2));
+  PD_CUDA_TRY(c, dzero(c, c->small_bar.p, 2 * sizeof(unsigned int)));
+  PD_CUDA_TRY(c, dzero(c, s->ctl.p, s->ctl.bytes()));
+  CgSmallArgs A{};
+  A.n = c->n;
+  A.row = c->row.p;
+  A.col = c->col.p;
+  A.g = s->geo.p;
+  A.gc = s->gco.p;
+  A.ab = s->abq.p;
+  A.pt = c->pt.p;
+  A.xv = c->xv.p;
+  A.fixed = s->fixed.p;
+  A.dinv = precond == PD_PRECOND_NONE ? nullptr : s->dinv.p;
+  A.r = s->r.p;
+  A.x = s->x.p;
+  A.w = s->w.p;
+  A.partial = s->partial.p;
+  A.jk = s->jk;
+  A.jm = s->jm;
+  A.tol = rel_tol;
+  A.max_it = max_it;
+  A.ctl = s->ctl.p;
+  A.bar = c->small_bar.p;
+  A.status = c->status.p;
+  const void* k = lanes == 32 ? (const void*)&k_cg_small<32> : (lanes == 16 ? (const void*)&k_cg_small<16> : (const void*)&k_cg_small<8>);
+  void* args[] = {&A};
+  PD_CUDA_TRY(c, cudaLaunchCooperativeKernel(k, dim3(gt(c->n, lanes)), dim3(kQsBlock), args, 0, c->stream));
+  CgCtl h{};
+  PD_CUDA_TRY(c, d2h(c, &h, s->ctl.p, sizeof(h)));
+  *iters = (int)h.it;
+  *rel_out = h.rel;
+  switch (h.state) {
+    case CG_CONVERGED:
+    case CG_ZERO_RHS: return PD_OK;
+    case CG_MAX_ITERATIONS: return PD_ERR_NOT_CONVERGED;
+    case CG_NONFINITE: c->err = "CG diverged (non-finite residual)"; return PD_ERR_NONFINITE;
+    default:
+      PD_CUDA_TRY(c, dzero(c, c->status.p, sizeof(int)));
+      c->err = "a bounded device wait ran out";
+      return PD_ERR_TIMEOUT;
+  }
+}
+
 // CG with a fixed preconditioner (none, block Jacobi, two-level): the scalars
 // and the stopping test stay on the device, and the host runs kCgAhead
 // iterations ahead of the last one reported. Launches after the end of the
@@ -875,6 +1135,10 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
   const int ahead = every > 0 ? 0 : kCgAhead;  // training pairs are taken at the reported iterate
   const bool coarse = s->coarse_on && precond == PD_PRECOND_TWO_LEVEL;
   const int use_bj = precond != PD_PRECOND_NONE;
+  if (!coarse && every == 0) {
+    const int lanes = cg_small_lanes(c);
+    if (lanes) return cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, lanes);
+  }
   auto update = [&](bool first) -> int {
     if (coarse)
       return coarse_cg_update(c, s->w.p, s->q.p, s->x.p, s->r.p, s->z.p, s->dinv.p, s->fixed.p, s->partial.p, s->ctl.p,
