@@ -105,7 +105,7 @@ __global__ void k_sorted_positions(int64_t n, const int32_t* __restrict__ sorted
 // counts, FILL = true writes the row (most points have no pair and leave at
 // once). A cell is little wider than the search radius and holds a few points:
 // a warp to a point, cell by cell, had 3 of 32 lanes at work (two bodies of
-// 814,000 points: count 3.33 -> 0.29 ms, fill 3.83 -> 0.02 ms).
+// 814,000 points: count 3.33 -> 0.75 ms, fill 3.83 -> 0.04 ms).
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4* __restrict__ pos,
                                                        const double4* __restrict__ pos_s, Grid g,
@@ -181,7 +181,7 @@ struct ContactCoords {
 // Contact force density on each point that has a pair (gather over its
 // contact list); the force of the others stays zero from the search on. Only
 // the coordinates of the pairs are formed: a pass over all points for them and
-// one for the forces were 26 us a step at 814,000 points, this one is 4.
+// one for the forces were 26 us a step at 814,000 points, this one is 8.
 __global__ void __launch_bounds__(128) k_contact_force(const int* __restrict__ n_active,
                                                       const int32_t* __restrict__ active,
                                                       const int64_t* __restrict__ crow,
