@@ -1791,8 +1791,8 @@ __global__ void k_min_reduce(int64_t m, const double* __restrict__ partial, doub
 // shared memory and each component's u and v in a register over the launch; a
 // phase gathers the neighbors' records and nothing else. Lanes per point and
 // the order of the sums are those of the general passes, so the results have
-// the same bits. 100x10x10 points, split: 26 -> 12 us a step; 27x7x6 points, FP64:
-// 19 -> 8 us.
+// the same bits. 100x10x10 points, split: 26 -> 17 us a step; 27x7x6 points, FP64:
+// 19 -> 6 us.
 // ---------------------------------------------------------------------------
 struct SmallArgs {
   int64_t n;
@@ -1880,13 +1880,12 @@ __device__ __forceinline__ double4 ld_f64x4_sync(const double4* p) {
   return r;
 }
 
-// Threads per block, one block per SM: 128 registers a thread.
-constexpr int kSmallBlock = 512;
+// Threads per block at most, one block per SM: few enough that a lane keeps two
+// batches of records in registers (the stream in shared memory ends a little
+// below it), FP64 with 8 bonds in flight up to 256 threads, else 4.
+constexpr int kSmallBlock = 352, kSmallBlock64 = 512, kSmallWide64 = 256;
 #ifndef PD_SMALL_BATCH
 #define PD_SMALL_BATCH 6
-#endif
-#ifndef PD_SMALL64_BATCH
-#define PD_SMALL64_BATCH 4
 #endif
 // Bytes of shared memory per thread and bond: (X, id) and damage; FP64: |X|, V, id and damage.
 constexpr int kSmallBond = 17, kSmallBond64 = 21;
@@ -1931,12 +1930,19 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
     if (lane < 3) dof.load(A.E, i, lane);
   }
   const float s_c = A.damage_on ? ow.w : -1.0f;
+  unsigned int target = 0;
   int cur = A.cur;
   for (int t = 0; t < A.nsteps; ++t) {
     Rec8* ur = A.ur[cur];
+    Rec8 un[K];  // the next batch's records, gathered while this one is computed
+    auto next = [&](int g0) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) un[k] = ld_rec_sync(ur + __float_as_int(sx[(g0 + k < G ? g0 + k : g0) * T].w));
+    };
     const OwnU ui = own_u(ld_rec_sync(ur + min(i, A.n - 1)));
     float th = 0.0f;
     int broken = 0;
+    next(0);
     for (int g0 = 0; g0 < G; g0 += K) {
       float4 X[K];
       int d[K];
@@ -1946,9 +1952,9 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
         const int g = g0 + k < G ? g0 + k : g0;
         X[k] = sx[g * T];
         d[k] = g0 + k < G ? sd[g * T] : kDummyBond;
+        uj[k] = un[k];
       }
-#pragma unroll
-      for (int k = 0; k < K; ++k) uj[k] = ld_rec_sync(ur + __float_as_int(X[k].w));
+      if (g0 + K < G) next(g0 + K);
 #pragma unroll
       for (int k = 0; k < K; ++k) {  // as k_dilatation_split
         const SplitBond sb = split_bond<false>(X[k].x, X[k].y, X[k].z, ui, uj[k]);
@@ -1984,10 +1990,11 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
       A.theta[i] = (double)theta;
       A.node_damage[i] = len > 0 ? (double)broken / (double)len : 0.0;
     }
-    if (!grid_sync(A.bar, A.E.status)) return;
+    if (!grid_sync(A.bar, target, A.E.status)) return;
     const Rec8 ri = ld_rec_sync(ur + min(i, A.n - 1));
     const float Ai = ri.v[6], Bi = ri.v[7];
     float fx = 0.f, fy = 0.f, fz = 0.f;
+    next(0);
     for (int g0 = 0; g0 < G; g0 += K) {
       float4 X[K];
       int d[K];
@@ -1997,9 +2004,9 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
         const int g = g0 + k < G ? g0 + k : g0;
         X[k] = sx[g * T];
         d[k] = g0 + k < G ? sd[g * T] : kDummyBond;
+        uj[k] = un[k];
       }
-#pragma unroll
-      for (int k = 0; k < K; ++k) uj[k] = ld_rec_sync(ur + __float_as_int(X[k].w));
+      if (g0 + K < G) next(g0 + K);
 #pragma unroll
       for (int k = 0; k < K; ++k) {  // as k_force_split
         const SplitBond sb = split_bond<true>(X[k].x, X[k].y, X[k].z, ui, uj[k]);
@@ -2029,7 +2036,7 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
     if (valid && lane < 3)
       dof.advance(A.E, 3 * i + lane, A.step0 + t, mode, (double)(lane == 0 ? fx : (lane == 1 ? fy : fz)), rho);
     if (mode == EVAL_ADVANCE) store_u_record_group<4>(A.ur[cur ^ 1] + i, lane, dof.u, valid);
-    if (t + 1 < A.nsteps && !grid_sync(A.bar, A.E.status)) return;
+    if (t + 1 < A.nsteps && !grid_sync(A.bar, target, A.E.status)) return;
     cur ^= 1;
   }
   if (valid && lane < 3) dof.store(A.E, 3 * i + lane);
@@ -2037,8 +2044,9 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_split(SmallArgs
 
 // The same in FP64, the reference's operation order, 16 lanes per point;
 // |X| of a bond is constant and stays in shared memory with V.
-__global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_fp64(SmallArgs A) {
-  constexpr int L = 16, K = PD_SMALL64_BATCH;
+template <int K, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) k_verlet_small_fp64(SmallArgs A) {
+  constexpr int L = 16;
   extern __shared__ __align__(16) unsigned char small_sm[];
   const int T = blockDim.x, tid = threadIdx.x, S = A.slots;
   double* sz = reinterpret_cast<double*>(small_sm) + tid;
@@ -2073,6 +2081,7 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_fp64(SmallArgs 
   SmallDof dof;
   if (valid && lane < 3) dof.load(A.E, i, lane);
   const double xc = comp3(xi, lane);
+  unsigned int target = 0;
   int cur = A.cur;
   for (int t = 0; t < A.nsteps; ++t) {
     const double4* st = A.st[cur];
@@ -2136,7 +2145,7 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_fp64(SmallArgs 
       A.theta[i] = th;
       A.node_damage[i] = len > 0 ? (double)broken / (double)len : 0.0;
     }
-    if (!grid_sync(A.bar, A.E.status)) return;
+    if (!grid_sync(A.bar, target, A.E.status)) return;
     const double4 ai = ld_f64x4_sync(A.ab64 + ic);
     double f[3] = {0.0, 0.0, 0.0};
     for (int t0 = 0; t0 < S; t0 += K / 2) {  // as k_force_fp64
@@ -2195,7 +2204,7 @@ __global__ void __launch_bounds__(kSmallBlock, 1) k_verlet_small_fp64(SmallArgs 
       const double dx = dof.advance(A.E, 3 * i + lane, A.step0 + t, mode, lane == 0 ? f[0] : (lane == 1 ? f[1] : f[2]), p.w);
       if (mode == EVAL_ADVANCE) *comp_ptr(&A.st[cur ^ 1][i], lane) = __dadd_rn(__dadd_rn(xc, u0), dx);  // y = x+u+dt*v
     }
-    if (t + 1 < A.nsteps && !grid_sync(A.bar, A.E.status)) return;
+    if (t + 1 < A.nsteps && !grid_sync(A.bar, target, A.E.status)) return;
     cur ^= 1;
   }
   if (valid && lane < 3) dof.store(A.E, 3 * i + lane);
@@ -2666,15 +2675,17 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
   return cudaGetLastError();
 }
 
-static const void* small_kernel(const pd_ctx* c, bool pair) {
-  if (c->precision == PD_FP64) return (const void*)&k_verlet_small_fp64;
+static const void* small_kernel(const pd_ctx* c, bool pair, int threads) {
+  if (c->precision == PD_FP64)
+    return threads <= kSmallWide64 ? (const void*)&k_verlet_small_fp64<8, kSmallWide64>
+                                   : (const void*)&k_verlet_small_fp64<4, kSmallBlock64>;
   return pair ? (const void*)&k_verlet_small_split<true> : (const void*)&k_verlet_small_split<false>;
 }
 
 // Whether steps of this context run as one cooperative launch: LPS with
 // omega = 1 on the default lane counts, nothing between the passes (contact,
 // prescribed functions, kernel timing, phantom halves), and one block per SM
-// with its bonds in shared memory (split: to about 13,000 points of 123 bonds,
+// with its bonds in shared memory (split: to about 13,000 points of 110 bonds,
 // FP64: to about 4,700).
 bool small_steps(pd_ctx* c) {
   if (c->n == 0 || c->material_model != PD_MATERIAL_LPS || c->influence != PD_INFLUENCE_ONE || c->contact ||
@@ -2697,9 +2708,9 @@ bool small_steps(pd_ctx* c) {
   const int64_t threads = ((c->n * lanes + sms - 1) / sms + 31) / 32 * 32;
   const int64_t slots = (c->max_row + lanes - 1) / lanes;
   const int64_t bytes = (threads * slots * bond + 15) / 16 * 16;
-  if (threads > kSmallBlock || slots == 0 || bytes > smem - 1024) return false;
+  if (threads > (f64 ? kSmallBlock64 : kSmallBlock) || slots == 0 || bytes > smem - 1024) return false;
   for (int pair = 0; pair < 2; ++pair) {
-    const void* k = small_kernel(c, pair != 0);
+    const void* k = small_kernel(c, pair != 0, (int)threads);
     // (one value for every context, whatever it needs: the attribute is the kernel's)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, (int)threads, (size_t)bytes) != cudaSuccess || per < 1) {
@@ -2722,8 +2733,8 @@ cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, i
     c->sell_src = c->dmg.p;
     c->sell_gen = c->dmg_gen;
   }
-  if (c->small_bar.count < 2) TRY_CUDA(c->small_bar.alloc(2));
-  TRY_CUDA(dzero(c, c->small_bar.p, 2 * sizeof(unsigned int)));
+  if (c->small_bar.count < 1) TRY_CUDA(c->small_bar.alloc(1));
+  TRY_CUDA(dzero(c, c->small_bar.p, sizeof(unsigned int)));
   SmallArgs A{};
   A.n = c->n;
   A.row = c->row.p;
@@ -2764,7 +2775,7 @@ cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, i
   A.last = last;
   A.bar = c->small_bar.p;
   const int lanes = split ? 4 : 16, T = c->small_threads;
-  const void* k = small_kernel(c, pair);
+  const void* k = small_kernel(c, pair, T);
   void* args[] = {&A};
   TRY_CUDA(cudaLaunchCooperativeKernel(k, dim3((unsigned)((c->n * lanes + T - 1) / T)), dim3(T), args,
                                        (size_t)c->small_bytes, c->stream));

@@ -35,10 +35,23 @@ namespace pdb {
 
 constexpr int kQsBlock = 256;
 constexpr int kQsTpo = 8;
+// Bonds per lane in flight in the tangent passes and their resident blocks per
+// SM, at 60x60x60 points (24.9 M bonds): first pass 126 us at 4 bonds and 5
+// blocks (48 registers; 6 blocks 128, unbounded 132 to 167), second 200 us at
+// 4 bonds and 4 blocks (64 registers; 2 bonds 203, 3 blocks 229, 5 blocks 247).
 #ifndef PD_QS_BATCH
 #define PD_QS_BATCH 4
 #endif
-constexpr int kQsBatch = PD_QS_BATCH;  // bonds per lane in flight in the tangent passes
+#ifndef PD_QS_BATCH2
+#define PD_QS_BATCH2 4
+#endif
+#ifndef PD_QS_MINB
+#define PD_QS_MINB 5
+#endif
+#ifndef PD_QS_MINB2
+#define PD_QS_MINB2 4
+#endif
+constexpr int kQsBatch = PD_QS_BATCH, kQsBatch2 = PD_QS_BATCH2;
 #ifndef PD_QS_WIDE
 #define PD_QS_WIDE 16384
 #endif
@@ -54,8 +67,8 @@ struct QsState {
   int64_t n = 0;
   bool coarse_on = false;  // the preconditioner adds the aggregate coarse correction (k_coarse.cu)
   // Per-bond tangent geometry at the current (y, theta, q, alpha), rebuilt
-  // after every change of the state (geo_dirty): g = (yh, V_j om zeta),
-  // gc = (V_j T / |Y|, V_j om (alpha_i + alpha_j)); zero for broken bonds.
+  // after every change of the state (geo_dirty), see k_qs_bond_geom; zero for
+  // broken bonds.
   DBuf<double4> geo;
   DBuf<double2> gco;
   bool geo_dirty = true;
@@ -73,7 +86,9 @@ struct QsState {
   DBuf<CgCtl> ctl;           // scalars and state of the running solve
   CgReport* report = nullptr;      // its progress, in mapped pinned memory
   CgReport* report_dev = nullptr;
-  int small_lanes = -1;  // of the one-launch solve (-1: not determined, 0: the general loop)
+  // one-launch solve: threads per block (-1: not determined, 0: the general
+  // loop) and bonds per lane, for rows of up to small_max_row bonds
+  int small_threads = -1, small_slots = 0, small_max_row = -1;
   ~QsState() {
     if (report) cudaFreeHost(report);
   }
@@ -167,7 +182,18 @@ __global__ void k_qs_reduce(const double* __restrict__ partial, int nblk, int wi
   }
 }
 
-// Per-bond tangent geometry (one lane group per owner, bonds strided over lanes).
+// Per-bond tangent geometry (one lane group per owner, bonds strided over
+// lanes). With c1 = V_j om zeta and yh = Y/|Y| the terms of the two passes are
+//   c1 yh.dw                           = G.dw                       G = c1 yh
+//   V_j [dT yh + (T/|Y|) (dw - yh de)] = (q dth_i + q dth_j + k2 (G.dw)) G + cx dw
+//   cx = V_j T/|Y|, k2 = (V_j om (alpha_i + alpha_j) - cx) / c1^2
+// The neighbor's id rides in the fourth number of G's record: the first pass of
+// a CG iteration streams 32 B per bond and the second 48, a record in one
+// 256-bit load. (yh, c1, the two coefficients and the id apart were 36 and 52 B
+// in twice as many loads; G in three planes, 28 and 44 B, took more L1
+// wavefronts than the bytes it saved; gathering the coordinates instead of
+// streaming G, 12 and 28 B, left both passes bound by the L1's gathers.) A bond of c1 = 0 (coincident points) takes c1 = 1e-100: no
+// term in the first pass, its own in the second.
 __global__ void __launch_bounds__(kQsBlock) k_qs_bond_geom(int64_t n, const int64_t* __restrict__ row,
                                                            const int32_t* __restrict__ col,
                                                            const uint8_t* __restrict__ dmg,
@@ -175,7 +201,8 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_bond_geom(int64_t n, const int6
                                                            const double4* __restrict__ y,
                                                            const double4* __restrict__ ab,
                                                            const double* __restrict__ hp, int influence,
-                                                           double4* __restrict__ g, double2* __restrict__ gc) {
+                                                           double4* __restrict__ g,
+                                                           double2* __restrict__ gc) {
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kQsTpo;
   const int lane = threadIdx.x & (kQsTpo - 1);
   if (i >= n) return;
@@ -183,7 +210,7 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_bond_geom(int64_t n, const int6
   const double h = hp[i];
   for (int64_t b = row[i] + lane; b < row[i + 1]; b += kQsTpo) {
     if (dmg[b]) {
-      g[b] = make_double4(0.0, 0.0, 0.0, 0.0);
+      g[b] = make_double4(0.0, 0.0, 0.0, __longlong_as_double(col[b]));
       gc[b] = make_double2(0.0, 0.0);
       continue;
     }
@@ -197,19 +224,35 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_bond_geom(int64_t n, const int6
     const double om = qs_omega(influence, zeta, h);
     const double T = om * (zeta * (ai.x * ai.y + aj.x * aj.y) + (ai.z + aj.z) * e);
     const double V = xj.w;
-    g[b] = make_double4(Y0 / dY, Y1 / dY, Y2 / dY, V * om * zeta);
-    gc[b] = make_double2(V * T / dY, V * om * (ai.z + aj.z));
+    const double cx = V * T / dY, cd = V * om * (ai.z + aj.z) - cx;
+    double c1 = V * om * zeta;
+    if (c1 == 0.0 && cd != 0.0) c1 = 1e-100;
+    const double s = c1 / dY;
+    g[b] = make_double4(s * Y0, s * Y1, s * Y2, __longlong_as_double(j));
+    gc[b] = make_double2(c1 != 0.0 ? cd / c1 / c1 : 0.0, cx);
   }
 }
 
-// Tangent pass 1 on the geometry: w[i].w = q_i dtheta_i = 3 (q_i/m_i) sum_j V_j om zeta yh.(w_j - w_i)
+// 256-bit loads: of a bond's record (read once per pass), of a point's (p, q dtheta).
+__device__ __forceinline__ double4 ld_bond(const double4* p) {
+  double4 r;
+  asm("ld.global.cs.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ double4 ld_w(const double4* p) {
+  double4 r;
+  asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ int64_t bond_id(const double4& g) { return __double_as_longlong(g.w); }
+
+// Tangent pass 1 on the geometry: w[i].w = q_i dtheta_i = 3 (q_i/m_i) sum_j G_ij.(w_j - w_i)
 // (a solve that has ended makes the kernel return)
 template <int TPO>
-__global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_g(int64_t n, const int64_t* __restrict__ row,
-                                                          const int32_t* __restrict__ col,
+__global__ void __launch_bounds__(kQsBlock, PD_QS_MINB) k_qs_dtheta_g(int64_t n, const int64_t* __restrict__ row,
                                                           const double4* __restrict__ g,
                                                           const double4* __restrict__ ab,
-                                                          const double4* __restrict__ pt, double4* __restrict__ w,
+                                                          const double4* __restrict__ pt, double4* w,
                                                           const CgCtl* __restrict__ ctl) {
   if (ctl->state) return;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / TPO;
@@ -220,23 +263,23 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_g(int64_t n, const int64
     const double4 wi = w[i];
     const int64_t b1 = row[i + 1];
     int64_t b = row[i] + lane;
+    auto bond = [&](const double4& gb, const double4& wj) {
+      acc += gb.x * (wj.x - wi.x) + gb.y * (wj.y - wi.y) + gb.z * (wj.z - wi.z);
+    };
     // batches of kQsBatch bonds per lane: stream loads, then gathers, then the
     // sums in bond order (the same order as one bond at a time)
     for (; b + (kQsBatch - 1) * TPO < b1; b += kQsBatch * TPO) {
       double4 gb[kQsBatch], wj[kQsBatch];
-      int32_t j[kQsBatch];
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * TPO], j[k] = col[b + k * TPO];
+      for (int k = 0; k < kQsBatch; ++k) gb[k] = ld_bond(g + b + k * TPO);
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) wj[k] = w[j[k]];
+      for (int k = 0; k < kQsBatch; ++k) wj[k] = ld_w(w + bond_id(gb[k]));
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k)
-        acc += gb[k].w * (gb[k].x * (wj[k].x - wi.x) + gb[k].y * (wj[k].y - wi.y) + gb[k].z * (wj[k].z - wi.z));
+      for (int k = 0; k < kQsBatch; ++k) bond(gb[k], wj[k]);
     }
     for (; b < b1; b += TPO) {
-      const double4 gb = g[b];
-      const double4 wj = w[col[b]];
-      acc += gb.w * (gb.x * (wj.x - wi.x) + gb.y * (wj.y - wi.y) + gb.z * (wj.z - wi.z));
+      const double4 gb = ld_bond(g + b);
+      bond(gb, ld_w(w + bond_id(gb)));
     }
   }
   acc = qs_group_sum<TPO>(acc);
@@ -245,10 +288,8 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_g(int64_t n, const int64
 
 // Tangent pass 2 on the geometry: q = K p = -V d f (prescribed rows: q = p), or
 // (jm rho I + jk K) p for implicit dynamics; p.q goes to ctl->pq
-//   V_j [dT yh + (T/|Y|)(dw - yh de)] = c2 (q dth_i + q dth_j) yh + V_j om (a_i + a_j) de yh + V_j T/|Y| (dw - yh de)
 template <int TPO>
-__global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* __restrict__ row,
-                                                      const int32_t* __restrict__ col,
+__global__ void __launch_bounds__(kQsBlock, PD_QS_MINB2) k_qs_df_g(int64_t n, const int64_t* __restrict__ row,
                                                       const double4* __restrict__ g,
                                                       const double2* __restrict__ gc,
                                                       const double4* __restrict__ xv,
@@ -268,24 +309,25 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
     int64_t b = row[i] + lane;
     auto bond = [&](const double4& gb, const double2& cb, const double4& wj) {
       const double w0 = wj.x - wi.x, w1 = wj.y - wi.y, w2 = wj.z - wi.z;
-      const double de = gb.x * w0 + gb.y * w1 + gb.z * w2;
-      const double sy = gb.w * (wi.w + wj.w) + (cb.y - cb.x) * de;
-      d0 += sy * gb.x + cb.x * w0;
-      d1 += sy * gb.y + cb.x * w1;
-      d2 += sy * gb.z + cb.x * w2;
+      const double sy = (wi.w + wj.w) + cb.x * (gb.x * w0 + gb.y * w1 + gb.z * w2);
+      d0 += sy * gb.x + cb.y * w0;
+      d1 += sy * gb.y + cb.y * w1;
+      d2 += sy * gb.z + cb.y * w2;
     };
-    for (; b + (kQsBatch - 1) * TPO < b1; b += kQsBatch * TPO) {  // batched as in k_qs_dtheta_g
-      double4 gb[kQsBatch], wj[kQsBatch];
-      double2 cb[kQsBatch];
-      int32_t j[kQsBatch];
+    for (; b + (kQsBatch2 - 1) * TPO < b1; b += kQsBatch2 * TPO) {  // batched as in k_qs_dtheta_g
+      double4 gb[kQsBatch2], wj[kQsBatch2];
+      double2 cb[kQsBatch2];
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) gb[k] = g[b + k * TPO], cb[k] = gc[b + k * TPO], j[k] = col[b + k * TPO];
+      for (int k = 0; k < kQsBatch2; ++k) gb[k] = ld_bond(g + b + k * TPO), cb[k] = __ldcs(gc + b + k * TPO);
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) wj[k] = w[j[k]];
+      for (int k = 0; k < kQsBatch2; ++k) wj[k] = ld_w(w + bond_id(gb[k]));
 #pragma unroll
-      for (int k = 0; k < kQsBatch; ++k) bond(gb[k], cb[k], wj[k]);
+      for (int k = 0; k < kQsBatch2; ++k) bond(gb[k], cb[k], wj[k]);
     }
-    for (; b < b1; b += TPO) bond(g[b], gc[b], w[col[b]]);
+    for (; b < b1; b += TPO) {
+      const double4 gb = ld_bond(g + b);
+      bond(gb, __ldcs(gc + b), ld_w(w + bond_id(gb)));
+    }
   }
   d0 = qs_group_sum<TPO>(d0);
   d1 = qs_group_sum<TPO>(d1);
@@ -302,13 +344,6 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_g(int64_t n, const int64_t* 
   }
   double sum[1] = {pq};
   if (cg_grid_sum<1, kQsBlock>(sum, partial, &ctl->ticket[0]) && threadIdx.x == 0) ctl->pq = sum[0];
-}
-
-// 256-bit load of a record that no thread writes during the kernel.
-__device__ __forceinline__ double4 ld_point_nc(const double4* p) {
-  double4 r;
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
-  return r;
 }
 
 // Inverse 3x3 diagonal blocks of K (prescribed rows/columns set to identity).
@@ -582,7 +617,8 @@ __global__ void k_cg_direction(int64_t n, const double* __restrict__ z, double4*
 // resident at once, an iteration is four phases between grid barriers: p
 // published, q dtheta, K p with p.q, the update with the dot products. At some
 // thousand points a phase is one or two round trips to L2, and the launches of
-// the general loop cost several times that. Lanes 0-2 of a point keep x, r and
+// the general loop cost as much again: 37x11x11 points, 63 us an iteration in
+// eleven launches, 35 us in four, 21 us here. Lanes 0-2 of a point keep x, r and
 // p of their component in registers; every block adds the blocks' partial sums
 // in the same order, so all of them see the same scalars and stop together.
 // ---------------------------------------------------------------------------
@@ -595,28 +631,42 @@ __device__ __forceinline__ double4 ld_w_sync(const double4* p) {
 
 // Sums over the grid: this block's to partial[NV blk ..], a barrier, then all
 // partials in block order. False when the barrier's wait ran out.
+// Every warp adds the blocks' partials for itself (lane l those of blocks l,
+// l + 32, ..), which saves a block barrier.
 template <int NV>
-__device__ __forceinline__ bool cg_sum_sync(double (&v)[NV], double* partial, unsigned int* bar, int* status) {
-  __shared__ double sh[NV][kQsBlock / 32];
-  cg_block_sum<NV, kQsBlock>(v, sh);
-  if (threadIdx.x == 0)
+__device__ __forceinline__ bool cg_sum_sync(double (&v)[NV], double* partial, unsigned int* bar, unsigned int& target,
+                                            int* status) {
+  __shared__ double sh[NV][32];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) partial[(size_t)NV * blockIdx.x + k] = v[k];
-  if (!grid_sync(bar, status)) return false;
+  for (int k = 0; k < NV; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double s = sh[threadIdx.x][0];
+    for (unsigned w = 1; w < blockDim.x / 32; ++w) s += sh[threadIdx.x][w];
+    partial[(size_t)NV * blockIdx.x + threadIdx.x] = s;
+  }
+  if (!grid_sync(bar, target, status)) return false;
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = 0.0;
-#pragma unroll 4
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += kQsBlock)
+#pragma unroll 5
+  for (unsigned b = threadIdx.x & 31; b < gridDim.x; b += 32)
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] += __ldcg(partial + (size_t)NV * b + k);
-  cg_block_sum<NV, kQsBlock>(v, sh);
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
   return true;
 }
 
 struct CgSmallArgs {
   int64_t n;
   const int64_t* row;
-  const int32_t* col;
+  int slots;  // bonds per lane
   const double4* g;
   const double2* gc;
   const double4* ab;
@@ -635,114 +685,115 @@ struct CgSmallArgs {
   int* status;
 };
 
-template <int TPO>
-__global__ void __launch_bounds__(kQsBlock, 3) k_cg_small(CgSmallArgs A) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / TPO;
-  const int lane = threadIdx.x & (TPO - 1);
+// 16 lanes per point, one block per SM, the geometry of the lanes' bonds (G,
+// k2, cx and the neighbor id) in shared memory.
+constexpr int kCgLanes = 16, kCgSmallBlock = 512, kCgBond = 44;
+__global__ void __launch_bounds__(kCgSmallBlock, 1) k_cg_small(CgSmallArgs A) {
+  constexpr int L = kCgLanes, K = 4;
+  extern __shared__ __align__(16) unsigned char cg_sm[];
+  const int T = blockDim.x, tid = threadIdx.x, S = A.slots;
+  double* sg = reinterpret_cast<double*>(cg_sm) + tid;  // bond t: G at sg[(3 t + c) T], k2 and cx at sk[2 t T], ..
+  double* sk = sg + (size_t)3 * S * T;
+  int32_t* sj = reinterpret_cast<int32_t*>(cg_sm + (size_t)40 * S * T) + tid;
+  const int64_t i = ((int64_t)blockIdx.x * T + tid) / L;
+  const int lane = tid & (L - 1);
   const bool valid = i < A.n, dof = valid && lane < 3;
-  int64_t b0 = 0, b1 = 0;
-  double s = 0.0, V = 0.0, rho = 0.0, D[3] = {0.0, 0.0, 0.0};
+  const int64_t ic = min(i, A.n - 1);
+  double D[3] = {0.0, 0.0, 0.0};
   bool held = false;
   double r = 0.0, x = 0.0, p = 0.0;
-  if (valid) {
-    b0 = A.row[i];
-    b1 = A.row[i + 1];
-    const double4 m = A.pt[i];
-    s = 3.0 * (A.ab[i].y / m.x);
-    V = A.xv[i].w;
-    rho = m.w;
+  const double4 m = A.pt[ic];
+  const double s = 3.0 * (A.ab[ic].y / m.x), V = A.xv[ic].w, rho = m.w;
+  {
+    const int64_t b0 = A.row[ic], b1 = A.row[ic + 1];
+    for (int t = 0; t < S; ++t) {
+      const int64_t b = b0 + lane + t * L;
+      const bool in = valid && b < b1;
+      const double4 gb = in ? ld_bond(A.g + b) : make_double4(0.0, 0.0, 0.0, __longlong_as_double(ic));
+      const double2 kc = in ? A.gc[b] : make_double2(0.0, 0.0);
+      sg[3 * t * T] = gb.x, sg[(3 * t + 1) * T] = gb.y, sg[(3 * t + 2) * T] = gb.z;
+      sk[2 * t * T] = kc.x, sk[(2 * t + 1) * T] = kc.y;
+      sj[t * T] = (int32_t)bond_id(gb);
+    }
   }
   if (dof) {
     held = (A.fixed[i] >> lane) & 1;
     r = A.r[3 * i + lane];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) D[c] = A.dinv ? A.dinv[9 * i + 3 * lane + c] : (c == lane ? 1.0 : 0.0);
+    for (int c = 0; c < 3; ++c) D[c] = A.dinv ? A.dinv[9 * i + 3 * lane + c] : 0.0;
   }
+  unsigned int target = 0;
   double* part_pq = A.partial + 2 * (size_t)gridDim.x;
   auto precond = [&](double rv) {  // lanes 0-2: their component of P r
-    const double r0 = __shfl_sync(0xffffffffu, rv, 0, TPO), r1 = __shfl_sync(0xffffffffu, rv, 1, TPO),
-                 r2 = __shfl_sync(0xffffffffu, rv, 2, TPO);
+    const double r0 = __shfl_sync(0xffffffffu, rv, 0, L), r1 = __shfl_sync(0xffffffffu, rv, 1, L),
+                 r2 = __shfl_sync(0xffffffffu, rv, 2, L);
     return A.dinv ? D[0] * r0 + D[1] * r1 + D[2] * r2 : rv;
   };
   double z = precond(r);
   double dots[2] = {dof ? r * z : 0.0, dof ? r * r : 0.0};
-  if (!cg_sum_sync<2>(dots, A.partial, A.bar, A.status)) return;
-  const double rr0 = dots[1];
-  double rz = dots[0], rel = 1.0;
+  if (!cg_sum_sync<2>(dots, A.partial, A.bar, target, A.status)) return;
+  const double rr0 = dots[1], r0 = sqrt(rr0);
+  double rz = dots[0], rel = rr0 == 0.0 ? 0.0 : 1.0;
   int state = rr0 == 0.0 ? CG_ZERO_RHS : CG_RUNNING;
-  if (rr0 == 0.0) rel = 0.0;
   long long it = 0;
   p = z;
   while (state == CG_RUNNING && it < A.max_it) {
     if (dof) (lane == 0 ? A.w[i].x : (lane == 1 ? A.w[i].y : A.w[i].z)) = p;
-    if (!grid_sync(A.bar, A.status)) return;
+    const double p0 = __shfl_sync(0xffffffffu, p, 0, L), p1 = __shfl_sync(0xffffffffu, p, 1, L),
+                 p2 = __shfl_sync(0xffffffffu, p, 2, L);
+    if (!grid_sync(A.bar, target, A.status)) return;
     // tangent pass 1 (k_qs_dtheta_g)
-    const double p0 = __shfl_sync(0xffffffffu, p, 0, TPO), p1 = __shfl_sync(0xffffffffu, p, 1, TPO),
-                 p2 = __shfl_sync(0xffffffffu, p, 2, TPO);
     double acc = 0.0;
-    if (valid)
-      for (int64_t b = b0 + lane; b < b1; b += 4 * TPO) {
-        double4 gb[4], wj[4];
-        int32_t j[4];
+    for (int t0 = 0; t0 < S; t0 += K) {
+      double4 wj[K];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool in = b + k * TPO < b1;
-          j[k] = in ? __ldg(A.col + b + k * TPO) : (int32_t)i;
-          gb[k] = in ? ld_point_nc(A.g + b + k * TPO) : make_double4(0.0, 0.0, 0.0, 0.0);
+      for (int k = 0; k < K; ++k) wj[k] = ld_w_sync(A.w + sj[(t0 + k < S ? t0 + k : t0) * T]);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (t0 + k < S) {
+          const double* G = sg + 3 * (t0 + k) * T;
+          acc += G[0] * (wj[k].x - p0) + G[T] * (wj[k].y - p1) + G[2 * T] * (wj[k].z - p2);
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) wj[k] = ld_w_sync(A.w + j[k]);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          acc += gb[k].w * (gb[k].x * (wj[k].x - p0) + gb[k].y * (wj[k].y - p1) + gb[k].z * (wj[k].z - p2));
-      }
-    acc = s * qs_group_sum<TPO>(acc);
+    }
+    acc = s * qs_group_sum<L>(acc);
     if (valid && lane == 0) A.w[i].w = acc;
-    if (!grid_sync(A.bar, A.status)) return;
+    if (!grid_sync(A.bar, target, A.status)) return;
     // tangent pass 2 (k_qs_df_g)
     double d[3] = {0.0, 0.0, 0.0};
-    if (valid)
-      for (int64_t b = b0 + lane; b < b1; b += 2 * TPO) {
-        double4 gb[2], wj[2];
-        double2 cb[2];
-        int32_t j[2];
+    for (int t0 = 0; t0 < S; t0 += K) {
+      double4 wj[K];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const bool in = b + k * TPO < b1;
-          j[k] = in ? __ldg(A.col + b + k * TPO) : (int32_t)i;
-          gb[k] = in ? ld_point_nc(A.g + b + k * TPO) : make_double4(0.0, 0.0, 0.0, 0.0);
-          cb[k] = in ? __ldg(A.gc + b + k * TPO) : make_double2(0.0, 0.0);
+      for (int k = 0; k < K; ++k) wj[k] = ld_w_sync(A.w + sj[(t0 + k < S ? t0 + k : t0) * T]);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (t0 + k < S) {
+          const int t = t0 + k;
+          const double* G = sg + 3 * t * T;
+          const double w0 = wj[k].x - p0, w1 = wj[k].y - p1, w2 = wj[k].z - p2, cx = sk[(2 * t + 1) * T];
+          const double sy = (acc + wj[k].w) + sk[2 * t * T] * (G[0] * w0 + G[T] * w1 + G[2 * T] * w2);
+          d[0] += sy * G[0] + cx * w0;
+          d[1] += sy * G[T] + cx * w1;
+          d[2] += sy * G[2 * T] + cx * w2;
         }
+    }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) wj[k] = ld_w_sync(A.w + j[k]);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const double w0 = wj[k].x - p0, w1 = wj[k].y - p1, w2 = wj[k].z - p2;
-          const double de = gb[k].x * w0 + gb[k].y * w1 + gb[k].z * w2;
-          const double sy = gb[k].w * (acc + wj[k].w) + (cb[k].y - cb[k].x) * de;
-          d[0] += sy * gb[k].x + cb[k].x * w0;
-          d[1] += sy * gb[k].y + cb[k].x * w1;
-          d[2] += sy * gb[k].z + cb[k].x * w2;
-        }
-      }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) d[c] = qs_group_sum<TPO>(d[c]);
+    for (int c = 0; c < 3; ++c) d[c] = qs_group_sum<L>(d[c]);
     double q = 0.0;
     if (dof) {
       q = -V * (lane == 0 ? d[0] : (lane == 1 ? d[1] : d[2]));
       if (A.jm != 0.0) q = A.jm * rho * p + A.jk * q;  // implicit dynamics: (rho I + beta dt^2 K) p
       if (held) q = p;
     }
-    double pq[1] = {p * q};
-    if (!cg_sum_sync<1>(pq, part_pq, A.bar, A.status)) return;
+    double pq[1] = {dof ? p * q : 0.0};
+    if (!cg_sum_sync<1>(pq, part_pq, A.bar, target, A.status)) return;
     const double alpha = rz / pq[0];
     x += alpha * p;
     r -= alpha * q;
     z = precond(r);
     dots[0] = dof ? r * z : 0.0;
     dots[1] = dof ? r * r : 0.0;
-    if (!cg_sum_sync<2>(dots, A.partial, A.bar, A.status)) return;
-    rel = sqrt(dots[1]) / sqrt(rr0);
+    if (!cg_sum_sync<2>(dots, A.partial, A.bar, target, A.status)) return;
+    rel = sqrt(dots[1]) / r0;
     ++it;
     if (!isfinite(rel)) state = CG_NONFINITE;
     else if (rel <= A.tol) state = CG_CONVERGED;
@@ -801,7 +852,7 @@ static int qs_alloc(pd_ctx* c) {
   PD_CUDA_TRY(c, s->scal.alloc(16));
   PD_CUDA_TRY(c, s->fixed.alloc(n));
   PD_CUDA_TRY(c, dzero(c, s->pred.p, s->pred.bytes()));
-  s->small_lanes = -1;
+  s->small_threads = -1;
   s->n = n;
   return PD_OK;
 }
@@ -851,8 +902,8 @@ static int qs_apply_learned(pd_ctx* c, const double* r, double* z) {
 static int qs_geometry(pd_ctx* c) {
   QsState* s = c->qs;
   const int64_t n = c->n;
-  if (s->geo_dirty || s->geo.count < (size_t)c->nb) {
-    if (s->geo.count < (size_t)c->nb) {
+  if (s->geo_dirty || s->gco.count < (size_t)c->nb) {
+    if (s->gco.count < (size_t)c->nb) {
       PD_CUDA_TRY(c, s->geo.alloc((size_t)c->nb));
       PD_CUDA_TRY(c, s->gco.alloc((size_t)c->nb));
     }
@@ -868,9 +919,9 @@ template <int TPO>
 static void launch_tangent(pd_ctx* c) {
   QsState* s = c->qs;
   const int64_t n = c->n;
-  k_qs_dtheta_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->abq.p, c->pt.p,
+  k_qs_dtheta_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, s->geo.p, s->abq.p, c->pt.p,
                                                              s->w.p, s->ctl.p);
-  k_qs_df_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->gco.p, c->xv.p, s->w.p,
+  k_qs_df_g<TPO><<<gt(n, TPO), kQsBlock, 0, c->stream>>>(n, c->row.p, s->geo.p, s->gco.p, c->xv.p, s->w.p,
                                                          s->fixed.p, s->q.p, s->partial.p, c->pt.p, s->jk, s->jm,
                                                          s->ctl.p);
 }
@@ -1056,37 +1107,45 @@ static int cg_wait(pd_ctx* c, long long it, CgReport* out) {
   }
 }
 
-// Lanes per point of the one-launch solve; 0 when the body's lanes are not all
-// resident (or the device takes no cooperative launches).
-static int cg_small_lanes(pd_ctx* c) {
+// Threads per block of the one-launch solve; 0 when the body's lanes are not
+// all resident with their geometry in shared memory (about 4,500 points of 110
+// bonds), or the device takes no cooperative launches.
+static int cg_small_threads(pd_ctx* c) {
   QsState* s = c->qs;
-  if (s->small_lanes < 0) {
-    int sms = 0, coop = 0, per = 0;
-    s->small_lanes = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) == cudaSuccess &&
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop) {
-      auto fits = [&](const void* k, int L) {
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kQsBlock, 0) == cudaSuccess &&
-               c->n * L <= (int64_t)per * sms * kQsBlock;
-      };
-      if (fits((const void*)&k_cg_small<32>, 32)) s->small_lanes = 32;
-      else if (fits((const void*)&k_cg_small<16>, 16)) s->small_lanes = 16;
-      else if (fits((const void*)&k_cg_small<8>, 8)) s->small_lanes = 8;
+  if (s->small_threads < 0 || s->small_max_row != c->max_row) {
+    s->small_threads = 0;
+    s->small_max_row = c->max_row;
+    int sms = 0, coop = 0, smem = 0, per = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess || !coop)
+      return 0;
+    const int64_t threads = ((c->n * kCgLanes + sms - 1) / sms + 31) / 32 * 32;
+    const int64_t slots = std::max(1, (c->max_row + kCgLanes - 1) / kCgLanes), bytes = threads * slots * kCgBond;
+    if (threads > kCgSmallBlock || bytes > smem - 2048) return 0;
+    // (one value for every context, whatever it needs: the attribute is the kernel's)
+    if (cudaFuncSetAttribute(k_cg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 2048) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cg_small, (int)threads, (size_t)bytes) != cudaSuccess ||
+        per < 1) {
+      cudaGetLastError();
+      return 0;
     }
+    s->small_threads = (int)threads;
+    s->small_slots = (int)slots;
   }
-  return s->small_lanes;
+  return s->small_threads;
 }
 
-static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out, int lanes) {
+static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out, int threads) {
   QsState* s = c->qs;
   TRY_RC(qs_geometry(c));
-  if (c->small_bar.count < 2) PD_CUDA_TRY(c, c->small_bar.alloc(2));
-  PD_CUDA_TRY(c, dzero(c, c->small_bar.p, 2 * sizeof(unsigned int)));
+  if (c->small_bar.count < 1) PD_CUDA_TRY(c, c->small_bar.alloc(1));
+  PD_CUDA_TRY(c, dzero(c, c->small_bar.p, sizeof(unsigned int)));
   PD_CUDA_TRY(c, dzero(c, s->ctl.p, s->ctl.bytes()));
   CgSmallArgs A{};
   A.n = c->n;
   A.row = c->row.p;
-  A.col = c->col.p;
+  A.slots = s->small_slots;
   A.g = s->geo.p;
   A.gc = s->gco.p;
   A.ab = s->abq.p;
@@ -1105,9 +1164,10 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   A.ctl = s->ctl.p;
   A.bar = c->small_bar.p;
   A.status = c->status.p;
-  const void* k = lanes == 32 ? (const void*)&k_cg_small<32> : (lanes == 16 ? (const void*)&k_cg_small<16> : (const void*)&k_cg_small<8>);
   void* args[] = {&A};
-  PD_CUDA_TRY(c, cudaLaunchCooperativeKernel(k, dim3(gt(c->n, lanes)), dim3(kQsBlock), args, 0, c->stream));
+  PD_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void*)&k_cg_small,
+                                             dim3((unsigned)((c->n * kCgLanes + threads - 1) / threads)), dim3(threads),
+                                             args, (size_t)threads * s->small_slots * kCgBond, c->stream));
   CgCtl h{};
   PD_CUDA_TRY(c, d2h(c, &h, s->ctl.p, sizeof(h)));
   *iters = (int)h.it;
@@ -1136,8 +1196,8 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
   const bool coarse = s->coarse_on && precond == PD_PRECOND_TWO_LEVEL;
   const int use_bj = precond != PD_PRECOND_NONE;
   if (!coarse && every == 0) {
-    const int lanes = cg_small_lanes(c);
-    if (lanes) return cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, lanes);
+    const int threads = cg_small_threads(c);
+    if (threads) return cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, threads);
   }
   auto update = [&](bool first) -> int {
     if (coarse)
@@ -1312,7 +1372,6 @@ int qs_apply_K(pd_ctx* c, const double* w_dev, double* kw_dev) {
 // vectors point-major, p[(i * kQsMulti + v) * 3 + c]; prescribed components of
 // p are dropped; prescribed rows of q = p. dth [kQsMulti n] scratch.
 __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_multi(int64_t n, const int64_t* __restrict__ row,
-                                                              const int32_t* __restrict__ col,
                                                               const double4* __restrict__ g,
                                                               const double4* __restrict__ ab,
                                                               const double4* __restrict__ pt,
@@ -1330,15 +1389,15 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_multi(int64_t n, const i
     for (int v = 0; v < NV; ++v)
       for (int c = 0; c < 3; ++c) pi[v][c] = ((fi >> c) & 1) ? 0.0 : p[(i * NV + v) * 3 + c];
     for (int64_t b = row[i] + lane; b < row[i + 1]; b += kQsTpo) {
-      const double4 gb = g[b];
-      const int32_t j = col[b];
+      const double4 gb = ld_bond(g + b);
+      const int64_t j = bond_id(gb);
       const uint8_t fj = fixed[j];
-      const double* pj = p + (int64_t)j * NV * 3;
+      const double* pj = p + j * NV * 3;
       for (int v = 0; v < NV; ++v) {
         const double w0 = ((fj & 1) ? 0.0 : pj[3 * v]) - pi[v][0];
         const double w1 = ((fj & 2) ? 0.0 : pj[3 * v + 1]) - pi[v][1];
         const double w2 = ((fj & 4) ? 0.0 : pj[3 * v + 2]) - pi[v][2];
-        acc[v] += gb.w * (gb.x * w0 + gb.y * w1 + gb.z * w2);
+        acc[v] += gb.x * w0 + gb.y * w1 + gb.z * w2;
       }
     }
   }
@@ -1350,7 +1409,6 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_dtheta_multi(int64_t n, const i
 }
 
 __global__ void __launch_bounds__(kQsBlock) k_qs_df_multi(int64_t n, const int64_t* __restrict__ row,
-                                                          const int32_t* __restrict__ col,
                                                           const double4* __restrict__ g,
                                                           const double2* __restrict__ gc,
                                                           const double4* __restrict__ xv,
@@ -1372,21 +1430,20 @@ __global__ void __launch_bounds__(kQsBlock) k_qs_df_multi(int64_t n, const int64
       for (int c = 0; c < 3; ++c) pi[v][c] = ((fi >> c) & 1) ? 0.0 : p[(i * NV + v) * 3 + c];
     }
     for (int64_t b = row[i] + lane; b < row[i + 1]; b += kQsTpo) {
-      const double4 gb = g[b];
+      const double4 gb = ld_bond(g + b);
       const double2 cb = gc[b];
-      const int32_t j = col[b];
+      const int64_t j = bond_id(gb);
       const uint8_t fj = fixed[j];
-      const double* pj = p + (int64_t)j * NV * 3;
-      const double* tj = dth + (int64_t)j * NV;
+      const double* pj = p + j * NV * 3;
+      const double* tj = dth + j * NV;
       for (int v = 0; v < NV; ++v) {
         const double w0 = ((fj & 1) ? 0.0 : pj[3 * v]) - pi[v][0];
         const double w1 = ((fj & 2) ? 0.0 : pj[3 * v + 1]) - pi[v][1];
         const double w2 = ((fj & 4) ? 0.0 : pj[3 * v + 2]) - pi[v][2];
-        const double de = gb.x * w0 + gb.y * w1 + gb.z * w2;
-        const double sy = gb.w * (ti[v] + tj[v]) + (cb.y - cb.x) * de;
-        d[v][0] += sy * gb.x + cb.x * w0;
-        d[v][1] += sy * gb.y + cb.x * w1;
-        d[v][2] += sy * gb.z + cb.x * w2;
+        const double sy = (ti[v] + tj[v]) + cb.x * (gb.x * w0 + gb.y * w1 + gb.z * w2);
+        d[v][0] += sy * gb.x + cb.y * w0;
+        d[v][1] += sy * gb.y + cb.y * w1;
+        d[v][2] += sy * gb.z + cb.y * w2;
       }
     }
   }
@@ -1409,9 +1466,9 @@ int qs_apply_K_multi(pd_ctx* c, const double* p_dev, double* q_dev, double* dth_
   QsState* s = c->qs;
   const int64_t n = c->n;
   TRY_RC(qs_geometry(c));
-  k_qs_dtheta_multi<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->abq.p, c->pt.p,
+  k_qs_dtheta_multi<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, s->geo.p, s->abq.p, c->pt.p,
                                                        s->fixed.p, p_dev, dth_dev);
-  k_qs_df_multi<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, c->col.p, s->geo.p, s->gco.p, c->xv.p, s->fixed.p,
+  k_qs_df_multi<<<gt(n), kQsBlock, 0, c->stream>>>(n, c->row.p, s->geo.p, s->gco.p, c->xv.p, s->fixed.p,
                                                    p_dev, dth_dev, q_dev);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;

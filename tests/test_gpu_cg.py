@@ -45,9 +45,11 @@ def _step(ctx, precond, max_cg, max_newton, tol):
     return st, ctx.field("Displacement")
 
 
-@pytest.mark.parametrize("precond,modes", [("none", 3), ("block_jacobi", 3), ("two_level", 3), ("two_level", 6)])
-def test_iteration_limit_and_convergence(precond, modes):
-    w = workloads.qs_cube(n=13, jitter=0.05, load_steps=4)
+@pytest.mark.parametrize("precond,modes,n", [("none", 3, 13), ("block_jacobi", 3, 8), ("block_jacobi", 3, 13),
+                                             ("block_jacobi", 3, 18), ("two_level", 3, 13), ("two_level", 6, 13)])
+def test_iteration_limit_and_convergence(precond, modes, n):
+    """13^3 points and fewer: one launch for the solve (without a coarse level); 18^3: the launch-by-launch loop."""
+    w = workloads.qs_cube(n=n, jitter=0.05, load_steps=4)
     with Context(precision="fp64") as ctx:
         workloads.setup_context(ctx, w)
         ctx.coarse_modes(modes)
