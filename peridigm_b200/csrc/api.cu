@@ -198,11 +198,14 @@ int ensure_ready(pd_ctx* c) {
   return PD_OK;
 }
 
-int check_status(pd_ctx* c) {
-  int st = 0;
-  PD_CUDA_TRY(c, cudaMemcpyAsync(&st, c->status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+// broke (may be null): whether a sliced pass broke a bond since the last check.
+int check_status(pd_ctx* c, bool* broke = nullptr) {
+  int word[2] = {0, 0};
+  PD_CUDA_TRY(c, cudaMemcpyAsync(word, c->status.p, sizeof(word), cudaMemcpyDeviceToHost, c->stream));
   PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  if (st) PD_CUDA_TRY(c, cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream));
+  const int st = word[0];
+  if (broke) *broke = word[1] != 0;
+  if (st || word[1]) PD_CUDA_TRY(c, cudaMemsetAsync(c->status.p, 0, sizeof(word), c->stream));
   // a non-finite prescribed value first: it makes the next forces non-finite too
   if (st & ST_NONFINITE_BC) return fail(c, PD_ERR_NONFINITE, "NaN returned by dirichlet increment BC evaluation");
   if (st & ST_NONFINITE_FORCE) return fail(c, PD_ERR_NONFINITE, "NaN returned by force evaluation");
@@ -217,8 +220,13 @@ int check_status(pd_ctx* c) {
 // tells whether the evaluation copied it there.
 int eval_trial(pd_ctx* c, double* f_dev, double* f_host = nullptr, bool* host_done = nullptr,
                const double* y_host = nullptr) {
-  PD_CUDA_TRY(c, cudaMemcpyAsync(c->dmg_trial.p, c->dmg.p, (size_t)c->nb, cudaMemcpyDeviceToDevice, c->stream));
-  note_damage_copy(c, c->dmg_trial.p, c->dmg.p);
+  if (!c->trial_same) {
+    PD_CUDA_TRY(c, cudaMemcpyAsync(c->dmg_trial.p, c->dmg.p, (size_t)c->nb, cudaMemcpyDeviceToDevice, c->stream));
+    note_damage_copy(c, c->dmg_trial.p, c->dmg.p);
+  } else if (c->sell_src == c->dmg.p) {
+    c->sell_src = c->dmg_trial.p;  // equal contents: the mirror serves the trial buffer
+  }
+  c->trial_same = false;
   StepParams sp{};
   sp.mode = EVAL_ONLY;
   sp.damage_on = c->any_damage ? 1 : 0;
@@ -227,7 +235,13 @@ int eval_trial(pd_ctx* c, double* f_dev, double* f_host = nullptr, bool* host_do
   sp.y_host = y_host;
   PD_CUDA_TRY(c, launch_eval(c, sp, c->dmg_trial.p, host_done));
   c->trial_valid = true;
-  return check_status(c);
+  bool broke = true;
+  const int rc = check_status(c, &broke);
+  // passes that report breaks: LPS and linear LPS on the sliced stream, and any without damage
+  const bool reports = !sp.damage_on || c->precision == PD_FP64_SLICED ||
+                       (c->precision == PD_SPLIT_FP32 && c->sell && c->material_model != PD_MATERIAL_BOND_BASED);
+  c->trial_same = rc == PD_OK && reports && !(sp.damage_on && broke);
+  return rc;
 }
 
 }  // namespace
@@ -266,7 +280,7 @@ int pd_create(const pd_config* cfg, pd_ctx** out) {
     return PD_ERR_CUDA;
   }
   if (cudaSetDevice(c->device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      c->status.alloc(1) != cudaSuccess || dzero(c, c->status.p, sizeof(int)) != cudaSuccess) {
+      c->status.alloc(2) != cudaSuccess || dzero(c, c->status.p, 2 * sizeof(int)) != cudaSuccess) {
     delete c;
     return PD_ERR_CUDA;
   }
@@ -595,6 +609,7 @@ int pd_set_bond_damage(pd_ctx* c, const double* bd) {
     else return fail(c, PD_ERR_UNSUPPORTED, "bond damage must be 0 or 1 (critical-stretch values)");
   }
   TRY(ensure_device(c));
+  c->trial_same = false;
   // the rows' own halves, then each bond's partner half (bit 1) from the partner's row
   PD_CUDA_TRY(c, h2d(c, c->dmg_trial.p, h.data(), (size_t)c->nb));
   TRY(mirror_damage(c, c->dmg_trial.p, c->dmg.p));
@@ -699,6 +714,7 @@ int pd_verlet_run(pd_ctx* c, double dt, double t0, int64_t nsteps, pd_stats* sta
   sp.has_bc = c->has_bc ? 1 : 0;
   sp.has_contact = contact ? 1 : 0;
   // initial evaluation (Peridigm.cpp:1393-1423): its damage is not committed
+  c->trial_same = false;
   PD_CUDA_TRY(c, cudaMemcpyAsync(c->dmg_trial.p, c->dmg.p, (size_t)c->nb, cudaMemcpyDeviceToDevice, c->stream));
   note_damage_copy(c, c->dmg_trial.p, c->dmg.p);
   if (contact) {
@@ -769,6 +785,7 @@ int pd_verlet_begin(pd_ctx* c, double dt, double t0) {
   if (!c->vbeg) PD_CUDA_TRY(c, cudaEventCreate(&c->vbeg));
   PD_CUDA_TRY(c, cudaEventRecord(c->vbeg, c->stream));
   // initial evaluation (Peridigm.cpp:1393-1423): its damage is not committed
+  c->trial_same = false;
   PD_CUDA_TRY(c, cudaMemcpyAsync(c->dmg_trial.p, c->dmg.p, (size_t)c->nb, cudaMemcpyDeviceToDevice, c->stream));
   note_damage_copy(c, c->dmg_trial.p, c->dmg.p);
   if (sp.has_contact) {
@@ -790,6 +807,7 @@ int pd_verlet_begin(pd_ctx* c, double dt, double t0) {
 int pd_verlet_step(pd_ctx* c, int64_t nsteps) {
   CHECK_CTX(c);
   if (!c->vrun) return fail(c, PD_ERR_STATE, "pd_verlet_step: call pd_verlet_begin first");
+  c->trial_same = false;
   if (nsteps < 0) return fail(c, PD_ERR_ARG, "pd_verlet_step: nsteps must be >= 0");
   StepParams sp = verlet_params(c, c->vdt, c->vt0);
   int64_t done = 0;
@@ -816,6 +834,7 @@ int pd_verlet_step(pd_ctx* c, int64_t nsteps) {
 int pd_verlet_finish(pd_ctx* c, pd_stats* stats) {
   CHECK_CTX(c);
   if (!c->vrun) return fail(c, PD_ERR_STATE, "pd_verlet_finish: call pd_verlet_begin first");
+  c->trial_same = false;
   StepParams sp = verlet_params(c, c->vdt, c->vt0);
   sp.step = ++c->vstep;
   sp.mode = EVAL_LAST;

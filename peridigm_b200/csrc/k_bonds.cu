@@ -385,6 +385,7 @@ int finalize_bonds(pd_ctx* c, bool sort_rows) {
   c->small_threads = -1;
   PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->trial_valid = false;
+  c->trial_same = false;
   c->wv_done = false;
   return PD_OK;
 }

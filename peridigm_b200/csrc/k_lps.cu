@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
     const float* __restrict__ bx3, Rec8* __restrict__ ur, const float4* __restrict__ own, int damage_on,
     double* __restrict__ theta_out, double* __restrict__ node_damage, const int64_t* __restrict__ soff,
     uint8_t* __restrict__ dmg_csr, const double* __restrict__ hp, int influence, const float* __restrict__ scf,
-    float s_min, int64_t i0 = 0) {
+    float s_min, int* __restrict__ broke, int64_t i0 = 0) {
   // owners i0 .. n-1 (a chunk starts at a multiple of 64 owners)
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = i0 + g / TPO;
@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
         const uint8_t nd = (uint8_t)(d | (brk ? 1 : 0) | (brkp ? 2 : 0));
         *pdm = nd;
         if (SELL) cdm[r] = nd;  // the CSR copy stays canonical
+        *broke = 1;
       }
       broken += ((d & 1) || brk) ? 1 : 0;
       float wv = uj.v[5];  // V_j
@@ -1199,7 +1200,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
     const double* __restrict__ bx, const double4* __restrict__ st, const double4* __restrict__ pt,
     const double* __restrict__ sc, int damage_on, double s_gate, double4* __restrict__ ab64,
     double* __restrict__ theta_out, double* __restrict__ node_damage, const int64_t* __restrict__ soff,
-    uint8_t* __restrict__ dmg_csr) {
+    uint8_t* __restrict__ dmg_csr, int* __restrict__ broke) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = g / 4;
   const int lane = threadIdx.x & 3;
@@ -1254,6 +1255,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
             d[k] |= (brk ? 1 : 0) | (brkp ? 2 : 0);
             pdm[k * step] = (uint8_t)d[k];
             cdm[r + 4 * k] = (uint8_t)d[k];  // the CSR copy stays canonical
+            *broke = 1;
           }
         }
       }
@@ -2549,7 +2551,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
     kd<<<grid_split(c->n, 4), kSplitBlock, 0, c->stream>>>(c->n, c->row.p, c->sell_col.p, c->sell_dmg.p, c->bx64.p,
                                                            c->st[c->cur].p, c->pt.p, c->sc.p, sp.damage_on,
                                                            c->sc_gate64, c->ab64.p, c->theta.p, c->node_damage.p,
-                                                           c->sell_off.p, dmg);
+                                                           c->sell_off.p, dmg, c->status.p + 1);
     TRY_CUDA(cudaGetLastError());
     TRY_CUDA(own_node_damage(c, dmg));
     if (ev) cudaEventRecord(ev[1], c->stream);
@@ -2611,13 +2613,13 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
         TRY_CUDA(form_through(std::max<int>(k, (int)(c->chunk_hi[k] / per))));
         kd<<<grid_split(i1 - i0, tpo), kSplitBlock, 0, c->stream>>>(
             i1, c->row.p, scol, sdmg, c->bx3.p, c->ur[c->cur].p, c->own.p, sp.damage_on, c->theta.p,
-            c->node_damage.p, soff, dmg, c->hp.p, c->influence, c->scf.p, c->sc_min, i0);
+            c->node_damage.p, soff, dmg, c->hp.p, c->influence, c->scf.p, c->sc_min, c->status.p + 1, i0);
       }
       TRY_CUDA(form_through(nk - 1));
     } else {
       kd<<<sgrid, kSplitBlock, 0, c->stream>>>(c->n, c->row.p, scol, sdmg, c->bx3.p, c->ur[c->cur].p, c->own.p,
                                                sp.damage_on, c->theta.p, c->node_damage.p, soff, sell ? dmg : nullptr,
-                                               c->hp.p, c->influence, c->scf.p, c->sc_min, 0);
+                                               c->hp.p, c->influence, c->scf.p, c->sc_min, c->status.p + 1, 0);
     }
   } else if (c->material_model == PD_MATERIAL_LINEAR_LPS) {
     PD_DISPATCH_TPO(tpo, k_dilatation_lin_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p,

@@ -180,6 +180,10 @@ struct pd_ctx {
   pdb::DBuf<uint8_t> dmg;        // committed (N) bond damage
   pdb::DBuf<uint8_t> dmg_trial;  // NP1 scratch for non-committing evaluations
   bool trial_valid = false;
+  // dmg_trial holds what dmg holds: the last trial evaluation broke no bond
+  // (its kernels report that in status[1]) and nothing wrote either since. The
+  // next one then needs no copy, and the sliced mirror serves both.
+  bool trial_same = false;
 
   // material
   bool wv_done = false;
@@ -247,7 +251,7 @@ struct pd_ctx {
   pdb::DBuf<double2> bc_cp;           // per dof (u(t_c), u(t_p)) of the evaluation in flight
 
   // misc
-  pdb::DBuf<int> status;      // device status word (non-finite etc.)
+  pdb::DBuf<int> status;      // device status word (non-finite etc.); [1]: a sliced pass broke a bond
   pdb::DBuf<double> scratch;  // reduction partials
   bool ktime = false;                 // bracket bond-pass launches with events
   std::vector<cudaEvent_t> kev;        // 3 per evaluation while ktime
