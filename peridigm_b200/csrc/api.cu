@@ -284,6 +284,7 @@ int pd_create(const pd_config* cfg, pd_ctx** out) {
     delete c;
     return PD_ERR_CUDA;
   }
+  host_pipe_retain();
   c->block_h.assign(1, 0.0);
   c->block_K.assign(1, 0.0);
   c->block_mu.assign(1, 0.0);
@@ -312,6 +313,7 @@ int pd_destroy(pd_ctx* c) {
   cudaStream_t s = c->stream;
   delete c;
   if (s) cudaStreamDestroy(s);
+  host_pipe_release();
   return PD_OK;
 }
 
@@ -571,8 +573,7 @@ int pd_compute_force(pd_ctx* c, const double* y, double* f_out) {
   bool copied = false;
   TRY(eval_trial(c, c->f.p, f_out, &copied, y));
   if (f_out && !copied) {
-    PD_CUDA_TRY(c, cudaMemcpyAsync(f_out, c->f.p, bytes, cudaMemcpyDeviceToHost, c->stream));
-    PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    PD_CUDA_TRY(c, d2h_user(c, f_out, c->f.p, bytes));
   }
   return PD_OK;
 }
@@ -635,9 +636,9 @@ int pd_set_state(pd_ctx* c, const double* u, const double* v) {
   CHECK_CTX(c);
   TRY(ensure_ready(c));
   const size_t bytes = 3 * (size_t)c->n * sizeof(double);
-  if (u) PD_CUDA_TRY(c, h2d(c, c->u.p, u, bytes));
+  if (u) PD_CUDA_TRY(c, h2d_user(c, c->u.p, u, bytes));
   else if (!c->state_init) PD_CUDA_TRY(c, dzero(c, c->u.p, bytes));
-  if (v) PD_CUDA_TRY(c, h2d(c, c->v.p, v, bytes));
+  if (v) PD_CUDA_TRY(c, h2d_user(c, c->v.p, v, bytes));
   else if (!c->state_init) PD_CUDA_TRY(c, dzero(c, c->v.p, bytes));
   if (u || !c->state_init) {
     c->cur = 0;
@@ -1094,20 +1095,20 @@ int pd_get_field(pd_ctx* c, int32_t field, double* out) {
   switch (field) {
     case PD_FIELD_DISPLACEMENT:
     case PD_FIELD_COORDINATES: {
-      PD_CUDA_TRY(c, d2h(c, out, c->u.p, b3));
+      PD_CUDA_TRY(c, d2h_user(c, out, c->u.p, b3));
       if (field == PD_FIELD_COORDINATES)
         for (int64_t k = 0; k < 3 * n; ++k) out[k] = c->hx[k] + out[k];
       return PD_OK;
     }
-    case PD_FIELD_VELOCITY: PD_CUDA_TRY(c, d2h(c, out, c->v.p, b3)); return PD_OK;
-    case PD_FIELD_ACCELERATION: PD_CUDA_TRY(c, d2h(c, out, c->a.p, b3)); return PD_OK;
-    case PD_FIELD_FORCE_DENSITY: PD_CUDA_TRY(c, d2h(c, out, c->f.p, b3)); return PD_OK;
-    case PD_FIELD_CONTACT_FORCE: PD_CUDA_TRY(c, d2h(c, out, c->fc.p, b3)); return PD_OK;
+    case PD_FIELD_VELOCITY: PD_CUDA_TRY(c, d2h_user(c, out, c->v.p, b3)); return PD_OK;
+    case PD_FIELD_ACCELERATION: PD_CUDA_TRY(c, d2h_user(c, out, c->a.p, b3)); return PD_OK;
+    case PD_FIELD_FORCE_DENSITY: PD_CUDA_TRY(c, d2h_user(c, out, c->f.p, b3)); return PD_OK;
+    case PD_FIELD_CONTACT_FORCE: PD_CUDA_TRY(c, d2h_user(c, out, c->fc.p, b3)); return PD_OK;
     case PD_FIELD_DILATATION:
-      PD_CUDA_TRY(c, d2h(c, out, c->theta.p, n * sizeof(double)));
+      PD_CUDA_TRY(c, d2h_user(c, out, c->theta.p, n * sizeof(double)));
       return PD_OK;
     case PD_FIELD_DAMAGE:
-      PD_CUDA_TRY(c, d2h(c, out, c->node_damage.p, n * sizeof(double)));
+      PD_CUDA_TRY(c, d2h_user(c, out, c->node_damage.p, n * sizeof(double)));
       return PD_OK;
     case PD_FIELD_WEIGHTED_VOLUME: return pd_weighted_volume(c, out);
     case PD_FIELD_BOND_DAMAGE: {
@@ -1119,7 +1120,7 @@ int pd_get_field(pd_ctx* c, int32_t field, double* out) {
       return PD_OK;
     }
     case PD_FIELD_FORCE: {
-      PD_CUDA_TRY(c, d2h(c, out, c->f.p, b3));
+      PD_CUDA_TRY(c, d2h_user(c, out, c->f.p, b3));
       for (int64_t k = 0; k < 3 * n; ++k) out[k] *= c->hvol[k / 3];
       return PD_OK;
     }

@@ -1,0 +1,271 @@
+// The pinned ring and its workers (host_pipe.cuh).
+#include "host_pipe.cuh"
+
+#include <algorithm>
+#include <condition_variable>
+#include <cstring>
+#include <deque>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace pdb {
+
+namespace {
+constexpr size_t kSlotBytes = size_t(512) << 10;
+constexpr int kSlots = 16;
+// Transfers below this go to the driver: the hand-over to the workers costs
+// some tens of microseconds.
+constexpr size_t kPipeMin = size_t(1) << 20;
+}  // namespace
+
+struct HostRing {
+  struct Job {
+    void* dst;
+    const void* src;
+    size_t bytes;
+    cudaEvent_t after;  // the slot's DMA, where there is one to wait for
+    int slot;
+  };
+  char* pinned = nullptr;
+  cudaEvent_t ev[kSlots] = {};
+  bool recorded[kSlots] = {};  // ev[k] stands for a DMA of this lease
+  bool busy[kSlots] = {};      // a job on the slot is not done
+  int device = -1;             // of the events
+  bool stop = false;
+  cudaError_t error = cudaSuccess;
+  std::mutex m;
+  std::condition_variable work, done;
+  std::deque<Job> jobs;
+  std::vector<std::thread> workers;
+
+  bool start() {
+    if (cudaHostAlloc((void**)&pinned, kSlotBytes * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      pinned = nullptr;
+      return false;
+    }
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int count = (int)std::min(6u, std::max(1u, hw / 2));
+    try {
+      for (int k = 0; k < count; ++k) workers.emplace_back([this] { run(); });
+    } catch (...) {  // as many as there could be
+    }
+    return !workers.empty();
+  }
+  void run() {
+    for (;;) {
+      Job j;
+      int dev;
+      {
+        std::unique_lock<std::mutex> l(m);
+        work.wait(l, [this] { return stop || !jobs.empty(); });
+        if (jobs.empty()) return;
+        j = jobs.front();
+        jobs.pop_front();
+        dev = device;
+      }
+      cudaError_t e = cudaSuccess;
+      if (j.after) {
+        cudaSetDevice(dev);
+        e = cudaEventSynchronize(j.after);
+      }
+      if (e == cudaSuccess) std::memcpy(j.dst, j.src, j.bytes);
+      {
+        std::lock_guard<std::mutex> l(m);
+        if (e != cudaSuccess) error = e;
+        busy[j.slot] = false;
+      }
+      done.notify_all();
+    }
+  }
+  void push(const Job& j) {
+    {
+      std::lock_guard<std::mutex> l(m);
+      busy[j.slot] = true;
+      jobs.push_back(j);
+    }
+    work.notify_one();
+  }
+  cudaError_t wait(int slot) {
+    std::unique_lock<std::mutex> l(m);
+    done.wait(l, [&] { return !busy[slot]; });
+    return error;
+  }
+  // Nothing of a lease left in flight, in the workers or the DMA.
+  void drain() {
+    std::unique_lock<std::mutex> l(m);
+    done.wait(l, [&] { return jobs.empty() && std::none_of(busy, busy + kSlots, [](bool b) { return b; }); });
+    l.unlock();
+    for (int k = 0; k < kSlots; ++k) {
+      if (recorded[k]) cudaEventSynchronize(ev[k]);
+      recorded[k] = false;
+    }
+    error = cudaSuccess;
+  }
+  bool on(int dev) {  // events of this device
+    if (device == dev) return true;
+    drop_events();
+    for (auto& e : ev)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        drop_events();
+        return false;
+      }
+    device = dev;
+    return true;
+  }
+  void drop_events() {
+    for (auto& e : ev) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+    device = -1;
+  }
+  ~HostRing() {
+    {
+      std::lock_guard<std::mutex> l(m);
+      stop = true;
+    }
+    work.notify_all();
+    for (auto& t : workers) t.join();
+    drop_events();
+    if (pinned) cudaFreeHost(pinned);
+  }
+};
+
+namespace {
+// (plain objects that no exit handler destroys: contexts may outlive statics)
+struct Shared {
+  std::mutex count_m;  // users and the ring's life
+  std::mutex lease_m;  // held by the lease
+  int users = 0;
+  HostRing* ring = nullptr;
+  bool failed = false;
+};
+Shared& shared() {
+  static Shared* s = new Shared();
+  return *s;
+}
+}  // namespace
+
+void host_pipe_retain() {
+  Shared& s = shared();
+  std::lock_guard<std::mutex> l(s.count_m);
+  ++s.users;
+}
+
+void host_pipe_release() {
+  Shared& s = shared();
+  HostRing* r = nullptr;
+  {
+    std::lock_guard<std::mutex> l(s.count_m);
+    if (--s.users > 0) return;
+    r = s.ring;  // (no context is left that could hold a lease)
+    s.ring = nullptr;
+    s.failed = false;
+  }
+  delete r;
+}
+
+HostLease::HostLease(int device, const void* host, size_t bytes) {
+  if (!host || bytes < kPipeMin) return;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (a.type != cudaMemoryTypeUnregistered) return;
+  Shared& s = shared();
+  if (!s.lease_m.try_lock()) return;
+  HostRing* r = nullptr;
+  {
+    std::lock_guard<std::mutex> l(s.count_m);
+    if (!s.ring && !s.failed) {
+      try {
+        s.ring = new HostRing();
+        if (!s.ring->start()) {
+          delete s.ring;
+          s.ring = nullptr;
+        }
+      } catch (...) {
+        s.ring = nullptr;
+      }
+      s.failed = s.ring == nullptr;
+    }
+    r = s.ring;
+  }
+  if (!r || !r->on(device)) {
+    s.lease_m.unlock();
+    return;
+  }
+  ring_ = r;
+}
+
+HostLease::~HostLease() {
+  if (!ring_) return;
+  ring_->drain();
+  shared().lease_m.unlock();
+}
+
+void HostLease::upload(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  up_dst_ = static_cast<char*>(dst);
+  up_src_ = static_cast<const char*>(src);
+  up_bytes_ = bytes;
+  up_issued_ = up_queued_ = 0;
+  up_stream_ = stream;
+}
+
+cudaError_t HostLease::through(size_t end) {
+  const size_t pieces = (up_bytes_ + kSlotBytes - 1) / kSlotBytes;
+  const size_t need = std::min(pieces, (end + kSlotBytes - 1) / kSlotBytes);
+  while (up_issued_ < need) {
+    // the workers run ahead by the ring; a slot's last DMA ends before it is filled again
+    for (; up_queued_ < pieces && up_queued_ < up_issued_ + kSlots; ++up_queued_) {
+      const int k = (int)(up_queued_ % kSlots);
+      const size_t off = up_queued_ * kSlotBytes;
+      ring_->push({ring_->pinned + k * kSlotBytes, up_src_ + off, std::min(kSlotBytes, up_bytes_ - off),
+                   ring_->recorded[k] ? ring_->ev[k] : nullptr, k});
+    }
+    const int k = (int)(up_issued_ % kSlots);
+    const size_t off = up_issued_ * kSlotBytes;
+    cudaError_t e = ring_->wait(k);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(up_dst_ + off, ring_->pinned + k * kSlotBytes, std::min(kSlotBytes, up_bytes_ - off),
+                          cudaMemcpyHostToDevice, up_stream_);
+    if (e == cudaSuccess) e = cudaEventRecord(ring_->ev[k], up_stream_);
+    if (e != cudaSuccess) return e;
+    ring_->recorded[k] = true;
+    ++up_issued_;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t HostLease::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  for (size_t off = 0; off < bytes; off += kSlotBytes, ++down_) {
+    const int k = (int)(down_ % kSlots);
+    const size_t len = std::min(kSlotBytes, bytes - off);
+    cudaError_t e = ring_->wait(k);  // the slot's last piece has been taken out (or its upload read)
+    // (a DMA that still reads the slot for an upload comes first on its stream or is waited for here)
+    if (e == cudaSuccess && ring_->recorded[k]) e = cudaStreamWaitEvent(stream, ring_->ev[k], 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(ring_->pinned + k * kSlotBytes, static_cast<const char*>(src) + off, len,
+                          cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaEventRecord(ring_->ev[k], stream);
+    if (e != cudaSuccess) return e;
+    ring_->recorded[k] = true;
+    ring_->push({static_cast<char*>(dst) + off, ring_->pinned + k * kSlotBytes, len, ring_->ev[k], k});
+  }
+  return cudaSuccess;
+}
+
+cudaError_t HostLease::finish() {
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < kSlots; ++k) {
+    const cudaError_t w = ring_->wait(k);
+    if (w != cudaSuccess) e = w;
+  }
+  return e;
+}
+
+}  // namespace pdb

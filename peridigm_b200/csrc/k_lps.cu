@@ -2538,8 +2538,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
   // (LPS and linear LPS), else one upload before the passes
   const bool chunk_in = sp.y_host && sp.f_out && sell && c->material_model != PD_MATERIAL_BOND_BASED;
   if (sp.y_host && !chunk_in) {
-    TRY_CUDA(cudaMemcpyAsync(sp.f_out, sp.y_host, 3 * (size_t)c->n * sizeof(double), cudaMemcpyHostToDevice,
-                             c->stream));
+    TRY_CUDA(h2d_user(c, sp.f_out, sp.y_host, 3 * (size_t)c->n * sizeof(double)));
     TRY_CUDA(launch_state_from_y(c, sp.f_out));
   }
   // half-bond damage: the two halves of a bond can differ (critical stretch
@@ -2592,17 +2591,27 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
       // (every earlier use of the staging buffer ended with its call: the
       // entry points synchronise both streams before they return)
       const int64_t n = c->n, per = host_chunk(n);
-      int nk = 0;
-      for (int64_t i0 = 0; i0 < n; i0 += per, ++nk) {
-        const int64_t i1 = std::min(n, i0 + per);
-        TRY_CUDA(cudaMemcpyAsync(sp.f_out + 3 * i0, sp.y_host + 3 * i0, 3 * (i1 - i0) * sizeof(double),
-                                 cudaMemcpyHostToDevice, c->copy_stream));
-        TRY_CUDA(cudaEventRecord(c->up_ev[nk], c->copy_stream));
-      }
+      const int nk = (int)((n + per - 1) / per);
+      // (pageable memory through the ring, a chunk when its turn comes: the
+      // kernels of the chunks before run meanwhile; else all chunks at once)
+      HostLease lease(c->device, sp.y_host, 3 * (size_t)n * sizeof(double));
+      auto up = [&](int k) -> cudaError_t {
+        const int64_t i0 = k * per, i1 = std::min(n, i0 + per);
+        if (lease)
+          TRY_CUDA(lease.through(3 * (size_t)i1 * sizeof(double)));
+        else
+          TRY_CUDA(cudaMemcpyAsync(sp.f_out + 3 * i0, sp.y_host + 3 * i0, 3 * (i1 - i0) * sizeof(double),
+                                   cudaMemcpyHostToDevice, c->copy_stream));
+        return cudaEventRecord(c->up_ev[k], c->copy_stream);
+      };
+      if (lease) lease.upload(sp.f_out, sp.y_host, 3 * (size_t)n * sizeof(double), c->copy_stream);
+      else
+        for (int k = 0; k < nk; ++k) TRY_CUDA(up(k));
       int formed = 0;  // chunks whose records are formed
       auto form_through = [&](int k) -> cudaError_t {
         for (; formed <= k && formed < nk; ++formed) {
           const int64_t j0 = formed * per, j1 = std::min(n, j0 + per);
+          if (lease) TRY_CUDA(up(formed));
           TRY_CUDA(cudaStreamWaitEvent(c->stream, c->up_ev[formed], 0));
           TRY_CUDA(launch_state_from_y(c, sp.f_out, j0, j1));
         }
@@ -2648,12 +2657,18 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
                                                                   c->pt.p, E, soff, c->hp.p, c->influence, i0);
         TRY_CUDA(cudaEventRecord(c->chunk_ev[k], c->stream));
       }
+      HostLease lease(c->device, sp.f_host, 3 * (size_t)n * sizeof(double));
       for (int64_t i0 = 0, k = 0; i0 < n; i0 += per, ++k) {
         const int64_t i1 = std::min(n, i0 + per);
         TRY_CUDA(cudaStreamWaitEvent(c->copy_stream, c->chunk_ev[k], 0));
-        TRY_CUDA(cudaMemcpyAsync(sp.f_host + 3 * i0, sp.f_out + 3 * i0, 3 * (i1 - i0) * sizeof(double),
-                                 cudaMemcpyDeviceToHost, c->copy_stream));
+        if (lease)
+          TRY_CUDA(lease.download(sp.f_host + 3 * i0, sp.f_out + 3 * i0, 3 * (size_t)(i1 - i0) * sizeof(double),
+                                  c->copy_stream));
+        else
+          TRY_CUDA(cudaMemcpyAsync(sp.f_host + 3 * i0, sp.f_out + 3 * i0, 3 * (i1 - i0) * sizeof(double),
+                                   cudaMemcpyDeviceToHost, c->copy_stream));
       }
+      if (lease) TRY_CUDA(lease.finish());
       TRY_CUDA(cudaEventRecord(c->chunk_ev[kHostChunks], c->copy_stream));
       TRY_CUDA(cudaStreamWaitEvent(c->stream, c->chunk_ev[kHostChunks], 0));
       *host_done = true;

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/pd_b200.h"
+#include "host_pipe.cuh"
 
 namespace pdb {
 
@@ -406,6 +407,20 @@ inline cudaError_t h2d(const pd_ctx* c, void* dst, const void* src, size_t bytes
 inline cudaError_t d2h(const pd_ctx* c, void* dst, const void* src, size_t bytes) {
   cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream);
   return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+}
+// The same for arrays of the caller, which may be large and pageable.
+inline cudaError_t h2d_user(const pd_ctx* c, void* dst, const void* src, size_t bytes) {
+  HostLease lease(c->device, src, bytes);
+  if (!lease) return h2d(c, dst, src, bytes);
+  lease.upload(dst, src, bytes, c->stream);
+  const cudaError_t e = lease.through(bytes);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
+}
+inline cudaError_t d2h_user(const pd_ctx* c, void* dst, const void* src, size_t bytes) {
+  HostLease lease(c->device, dst, bytes);
+  if (!lease) return d2h(c, dst, src, bytes);
+  const cudaError_t e = lease.download(dst, src, bytes, c->stream), w = lease.finish();
+  return e != cudaSuccess ? e : w;
 }
 inline cudaError_t dzero(const pd_ctx* c, void* dst, size_t bytes) { return cudaMemsetAsync(dst, 0, bytes, c->stream); }
 }  // namespace pdb
