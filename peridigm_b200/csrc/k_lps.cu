@@ -225,9 +225,23 @@ __device__ __forceinline__ SplitBond split_bond(float X0, float X1, float X2, co
 // Position of the X of stream slot k in bx3 (component c at +32c).
 __device__ __forceinline__ int64_t xs_index(int64_t k) { return 96 * (k >> 5) + (k & 31); }
 
-// Streaming loads of bond-ordered data (read once per pass; kept out of L1 so
-// the neighbor records stay resident there).
-//
+// Streaming loads of bond-ordered data that no thread writes (read once per
+// pass; kept out of L1 so that the neighbor records stay resident there).
+// L1::no_allocate against the evict-first hint (.cs): the bond-based pass
+// 141.6 -> 133.9 us at 257x129x9 points, the full-bond dilatation 105.7 -> 104.5
+// us at the notched plate, the others within 0.4 %; with 256-byte L2 prefetches
+// but no hint for L1 every pass was slower (force 104.8 -> 119.4 us).
+__device__ __forceinline__ int4 ld_stream(const int4* p) {
+  int4 r;
+  asm("ld.global.nc.L1::no_allocate.v4.s32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 r;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+  return r;
+}
+
 // The split passes walk a row kUnroll bonds per lane at a time: first the
 // bond-ordered loads of the batch (damage, neighbor id, X), all independent,
 // then the batch's neighbor-record gathers, then the arithmetic. Loads do not
@@ -347,13 +361,13 @@ __device__ __forceinline__ void sell_walk(int64_t i, int lane, const int64_t* __
   const int4* pc = reinterpret_cast<const int4*>(col + 32 * so + 4 * l32);
   uint32_t* pd = reinterpret_cast<uint32_t*>(dmg + 32 * so + 4 * l32);
   const float4* px = reinterpret_cast<const float4*>(bx3 + 96 * so + 4 * l32);
-  int4 jn = F > 0 ? __ldcs(pc) : make_int4(0, 0, 0, 0);
+  int4 jn = F > 0 ? ld_stream(pc) : make_int4(0, 0, 0, 0);
 #pragma unroll 1
   for (int b = 0; b < F; ++b, pc += 32, pd += 32, px += 96) {
     const int4 jj = jn;
-    if (b + 1 < F) jn = __ldcs(pc + 32);
+    if (b + 1 < F) jn = ld_stream(pc + 32);
     const uint32_t dw = __ldcs(pd);
-    const float4 xa = __ldcs(px), xb = __ldcs(px + 32), xc = __ldcs(px + 64);
+    const float4 xa = ld_stream(px), xb = ld_stream(px + 32), xc = ld_stream(px + 64);
     const Rec8 u0 = ld_rec_t<NC>(ur + jj.x), u1 = ld_rec_t<NC>(ur + jj.y), u2 = ld_rec_t<NC>(ur + jj.z),
                u3 = ld_rec_t<NC>(ur + jj.w);
     uint8_t* pb = reinterpret_cast<uint8_t*>(pd);
