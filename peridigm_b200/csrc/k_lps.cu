@@ -242,6 +242,16 @@ __device__ __forceinline__ float4 ld_stream(const float4* p) {
   return r;
 }
 
+// Asks for a line of the stream a block ahead. Where a lane's X of the block
+// after next would otherwise be asked for only when its turn comes, it is in L2
+// by then: full-bond dilatation 104.8 -> 100.2 us at the notched plate, FP64
+// sliced dilatation 678 -> 659 us and force 822 -> 816 us at 160x160x40 points. The
+// passes with more registers in flight or of half-bond damage lose by it (full-
+// bond force 105.4 -> 112.3 us, bond-based 133.9 -> 143.4 us, half-bond dilatation
+// 1855 -> 1860 us at 250x200x80 points), and two to four blocks ahead gain
+// nothing.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // The split passes walk a row kUnroll bonds per lane at a time: first the
 // bond-ordered loads of the batch (damage, neighbor id, X), all independent,
 // then the batch's neighbor-record gathers, then the arithmetic. Loads do not
@@ -350,8 +360,9 @@ __device__ __forceinline__ Rec8 ld_rec_t(const Rec8* p) {
 // and three float4 of X per block, then the tail groups. For each bond, in
 // the lane's row order, body(X0, X1, X2, damage byte, neighbor record,
 // neighbor id, the bond's damage byte in the stream, row offset r - lane).
-// NC: how neighbor records are loaded (ld_rec_t).
-template <int NC, typename Body>
+// NC: how neighbor records are loaded (ld_rec_t). AHEAD: the next block's X is
+// asked for (prefetch_l2).
+template <int NC, bool AHEAD, typename Body>
 __device__ __forceinline__ void sell_walk(int64_t i, int lane, const int64_t* __restrict__ soff,
                                           const int32_t* __restrict__ col, uint8_t* __restrict__ dmg,
                                           const float* __restrict__ bx3, const Rec8* __restrict__ ur, Body&& body) {
@@ -367,6 +378,7 @@ __device__ __forceinline__ void sell_walk(int64_t i, int lane, const int64_t* __
     const int4 jj = jn;
     if (b + 1 < F) jn = ld_stream(pc + 32);
     const uint32_t dw = __ldcs(pd);
+    if (AHEAD && b + 1 < F) prefetch_l2(px + 96), prefetch_l2(px + 128), prefetch_l2(px + 160);
     const float4 xa = ld_stream(px), xb = ld_stream(px + 32), xc = ld_stream(px + 64);
     const Rec8 u0 = ld_rec_t<NC>(ur + jj.x), u1 = ld_rec_t<NC>(ur + jj.y), u2 = ld_rec_t<NC>(ur + jj.z),
                u3 = ld_rec_t<NC>(ur + jj.w);
@@ -653,7 +665,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
     // material)
     constexpr int kRec = 0;
     if constexpr (SELL)
-      sell_walk<kRec>(i, lane, soff, col, dmg, bx3, ur, body);
+      sell_walk<kRec, !PAIR>(i, lane, soff, col, dmg, bx3, ur, body);
     else
       csr_walk<TPO, kRec>(i, lane, b0, b0 + len, col, dmg, bx3, ur, body);
   }
@@ -976,7 +988,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_BOND_MINB) k_forc
     };
     uint8_t* dm = const_cast<uint8_t*>(dmg);  // not written by this pass
     if constexpr (SELL)
-      sell_walk<PD_FORCE_NC>(i, lane, soff, col, dm, bx3, ur, body);
+      sell_walk<PD_FORCE_NC, false>(i, lane, soff, col, dm, bx3, ur, body);
     else
       csr_walk<TPO, PD_FORCE_NC>(i, lane, row[i], row[i + 1], col, dm, bx3, ur, body);
   }
@@ -1146,6 +1158,7 @@ __device__ __forceinline__ void sell_walk64(int64_t i, int lane, const int64_t* 
     const int jv[4] = {jn.x, jn.y, jn.z, jn.w};
     if (b + 1 < F) jn = __ldcs(pc + 32);
     const uint32_t dw = __ldcs(pd);
+    if (b + 1 < F) prefetch_l2(px + 384), prefetch_l2(px + 512), prefetch_l2(px + 640);
     double X0[4], X1[4], X2[4];
     ldcs_f64x4(px, X0);
     ldcs_f64x4(px + 128, X1);
@@ -1255,6 +1268,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
         const double s_c = sc[i];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
+          if (!(e[k] > gate * zeta[k])) continue;
           const double rel = __ddiv_rn(e[k], zeta[k]);
           const bool brk = (d[k] & 5) == 0 && s_c >= 0.0 && rel > s_c;
           bool brkp = brk;
@@ -1689,7 +1703,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_BOND_MINB) k_bb_split(int64_t 
       fz = fmaf(w, sb.Yz, fz);
     };
     if constexpr (SELL)
-      sell_walk<1>(i, lane, soff, col, dmg, bx3, ur, body);
+      sell_walk<1, false>(i, lane, soff, col, dmg, bx3, ur, body);
     else
       csr_walk<TPO, 1>(i, lane, b0, b0 + len, col, dmg, bx3, ur, body);
   }
@@ -2135,7 +2149,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_verlet_small_fp64(SmallArgs A) {
       if (hot)
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-          if ((d[k] & 3) == 3) continue;
+          if ((d[k] & 3) == 3 || !(e[k] > gate * zeta[k])) continue;
           const double scj = A.pair ? A.sc[j[k]] : s_c;
           const double rel = __ddiv_rn(e[k], zeta[k]);
           const bool brk = !(d[k] & 1) && s_c >= 0.0 && rel > s_c;
