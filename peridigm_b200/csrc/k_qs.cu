@@ -629,6 +629,12 @@ __device__ __forceinline__ double4 ld_w_sync(const double4* p) {
   return r;
 }
 
+__device__ __forceinline__ double ld_t_sync(const double* p) {
+  double r;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p) : "memory");
+  return r;
+}
+
 // Sums over the grid: this block's to partial[NV blk ..], a barrier, then all
 // partials in block order. False when the barrier's wait ran out.
 // Every warp adds the blocks' partials for itself (lane l those of blocks l,
@@ -677,6 +683,7 @@ struct CgSmallArgs {
   const double* r;     // right-hand side
   double* x;           // solution
   double4* w;
+  double* t;           // q dtheta per point
   double* partial;
   double jk, jm, tol;
   long long max_it;
@@ -742,24 +749,8 @@ __global__ void __launch_bounds__(kCgSmallBlock, 1) k_cg_small(CgSmallArgs A) {
     const double p0 = __shfl_sync(0xffffffffu, p, 0, L), p1 = __shfl_sync(0xffffffffu, p, 1, L),
                  p2 = __shfl_sync(0xffffffffu, p, 2, L);
     if (!grid_sync(A.bar, target, A.status)) return;
-    // tangent pass 1 (k_qs_dtheta_g)
-    double acc = 0.0;
-    for (int t0 = 0; t0 < S; t0 += K) {
-      double4 wj[K];
-#pragma unroll
-      for (int k = 0; k < K; ++k) wj[k] = ld_w_sync(A.w + sj[(t0 + k < S ? t0 + k : t0) * T]);
-#pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (t0 + k < S) {
-          const double* G = sg + 3 * (t0 + k) * T;
-          acc += G[0] * (wj[k].x - p0) + G[T] * (wj[k].y - p1) + G[2 * T] * (wj[k].z - p2);
-        }
-    }
-    acc = s * qs_group_sum<L>(acc);
-    if (valid && lane == 0) A.w[i].w = acc;
-    if (!grid_sync(A.bar, target, A.status)) return;
-    // tangent pass 2 (k_qs_df_g)
-    double d[3] = {0.0, 0.0, 0.0};
+    // tangent pass 1 (k_qs_dtheta_g), with the terms of pass 2 that p alone gives
+    double acc = 0.0, d[3] = {0.0, 0.0, 0.0};
     for (int t0 = 0; t0 < S; t0 += K) {
       double4 wj[K];
 #pragma unroll
@@ -768,12 +759,31 @@ __global__ void __launch_bounds__(kCgSmallBlock, 1) k_cg_small(CgSmallArgs A) {
       for (int k = 0; k < K; ++k)
         if (t0 + k < S) {
           const int t = t0 + k;
-          const double* G = sg + 3 * t * T;
+          const double G0 = sg[3 * t * T], G1 = sg[(3 * t + 1) * T], G2 = sg[(3 * t + 2) * T];
           const double w0 = wj[k].x - p0, w1 = wj[k].y - p1, w2 = wj[k].z - p2, cx = sk[(2 * t + 1) * T];
-          const double sy = (acc + wj[k].w) + sk[2 * t * T] * (G[0] * w0 + G[T] * w1 + G[2 * T] * w2);
-          d[0] += sy * G[0] + cx * w0;
-          d[1] += sy * G[T] + cx * w1;
-          d[2] += sy * G[2 * T] + cx * w2;
+          const double gd = G0 * w0 + G1 * w1 + G2 * w2, kg = sk[2 * t * T] * gd;
+          acc += gd;
+          d[0] += kg * G0 + cx * w0;
+          d[1] += kg * G1 + cx * w1;
+          d[2] += kg * G2 + cx * w2;
+        }
+    }
+    acc = s * qs_group_sum<L>(acc);
+    if (valid && lane == 0) A.t[i] = acc;
+    if (!grid_sync(A.bar, target, A.status)) return;
+    // the rest of pass 2 (k_qs_df_g): (q dth_i + q dth_j) G
+    for (int t0 = 0; t0 < S; t0 += 2 * K) {
+      double tj[2 * K];
+#pragma unroll
+      for (int k = 0; k < 2 * K; ++k) tj[k] = ld_t_sync(A.t + sj[(t0 + k < S ? t0 + k : t0) * T]);
+#pragma unroll
+      for (int k = 0; k < 2 * K; ++k)
+        if (t0 + k < S) {
+          const int t = t0 + k;
+          const double ts = acc + tj[k];
+          d[0] += ts * sg[3 * t * T];
+          d[1] += ts * sg[(3 * t + 1) * T];
+          d[2] += ts * sg[(3 * t + 2) * T];
         }
     }
 #pragma unroll
@@ -1156,6 +1166,7 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   A.r = s->r.p;
   A.x = s->x.p;
   A.w = s->w.p;
+  A.t = s->z.p;
   A.partial = s->partial.p;
   A.jk = s->jk;
   A.jm = s->jm;
