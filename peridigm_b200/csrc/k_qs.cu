@@ -53,9 +53,14 @@ constexpr int kQsTpo = 8;
 #endif
 constexpr int kQsBatch = PD_QS_BATCH, kQsBatch2 = PD_QS_BATCH2;
 #ifndef PD_QS_WIDE
-#define PD_QS_WIDE 16384
+#define PD_QS_WIDE 4096
 #endif
-constexpr int64_t kQsWide = PD_QS_WIDE;  // bodies up to this size: 32 lanes per point in the tangent passes
+// Bodies up to this size take 32 lanes per point in the tangent passes, larger
+// ones 8. Both passes of one product, us, cubes of points at 32 and 8 lanes:
+// 14^3 12.8 and 15.1, 16^3 13.7 and 15.2, 17^3 16.3 and 15.6, 20^3 22.4 and
+// 17.1, 25^3 37.2 and 22.7, 40^3 174 and 116: few points leave lanes idle, more
+// of them pay for the wider sums and the rows' idle last lanes.
+constexpr int64_t kQsWide = PD_QS_WIDE;
 constexpr int kRedBlocks = 296;  // 2 x 148 SMs: fixed, so reductions are deterministic
 
 struct QsState {

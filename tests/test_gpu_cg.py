@@ -17,7 +17,7 @@ from peridigm_b200 import Context, PDError, _lib, workloads
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dims", [(7, 6, 5), (32, 32, 16), (33, 31, 17)])
+@pytest.mark.parametrize("dims", [(7, 6, 5), (16, 16, 16), (17, 31, 8), (32, 32, 16), (33, 31, 17)])
 def test_tangent_product_of_both_lane_counts(dims):
     x, vol = workloads.lattice(*dims, 1.0e-3, jitter=0.05, seed=2)
     h, K, mu = 3.015e-3, 130.0e9, 78.0e9
