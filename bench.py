@@ -375,12 +375,12 @@ def qs_leg(local, load_steps, cpu_threads=0, learned_modes=6):
     # Roofline of the CG iterations: bytes one iteration must move at least,
     # over the solve's device time per iteration (Newton set-up included, so
     # the fractions are lower bounds). Tangent apply: pass 1 streams the bond
-    # geometry (32 B) and neighbor id (4 B), pass 2 the geometry, the
-    # coefficient pair (16 B) and the id: 88 B per bond; per point the
+    # geometry with the neighbor id (32 B), pass 2 the same and the
+    # coefficient pair (16 B): 80 B per bond; per point the
     # gathered vector, dilatation increments and output (about 64 B) and about
     # ten FP64 3-vectors of CG and block Jacobi (240 B). The coarse arms also
-    # read the dense FP64 coarse inverse (modes x aggregates squared x 8 B;
-    # aggregates: the non-empty cells of side two horizons).
+    # read half of the symmetric coarse inverse in FP32 (modes x aggregates
+    # squared x 2 B; aggregates: the non-empty cells of side two horizons).
     nb2 = out.pop("_bonds")
     n2 = len(w2["vol"])
     side = 2.0 * w2["horizon"] * (1.0 + 1.0e-6)
@@ -388,10 +388,10 @@ def qs_leg(local, load_steps, cpu_threads=0, learned_modes=6):
     cells = np.floor((P2 - P2.min(0)) / side).astype(np.int64)
     naggr = len(np.unique(cells @ np.array([1, 1 << 20, 1 << 40], np.int64)))
     hbm, peak_src = peak_hbm()
-    it_bytes = 88 * nb2 + 304 * n2
+    it_bytes = 80 * nb2 + 304 * n2
     roof = {"bytes_per_cg_iteration": it_bytes, "aggregates": naggr, "peak_gbs": hbm, "peak_source": peak_src}
     for arm, modes in (("block_jacobi", 0), ("two_level", 3), ("two_level_rigid", 6)):
-        b = it_bytes + 8 * (modes * naggr) ** 2
+        b = it_bytes + 2 * (modes * naggr) ** 2
         ach = b * out[arm]["cg_iterations"] / out[arm]["seconds"] / 1e9
         roof[arm] = {"bytes_per_cg_iteration": b, "achieved_gbs": ach, "frac": ach / hbm}
     out["roofline"] = roof

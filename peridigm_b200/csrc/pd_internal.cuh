@@ -16,7 +16,7 @@
 //   own[n]       float4 (3/m, (3K-5mu)/m, 15mu/m, s_c)  owner terms
 // FP64 paths:
 //   st[2][n]     double4 (y_x, y_y, y_z, V) current coordinates and volume, double buffered
-//   ab64[n]      double4 (theta, 3K/m - alpha/3, alpha, 0); on the FP64 sliced
+//   ab64[n]      double4 (theta, q = 3K/m - alpha/3, alpha, theta*q); on the FP64 sliced
 //                path (A, B, theta, 0) with A = theta*(3K/m - alpha/3), B = alpha
 //   bx64         X per bond in FP64 on the sliced stream (FP64 sliced path)
 // A = theta*(3K-5mu)/m and B = 15mu/m are the owner terms of the LPS force
