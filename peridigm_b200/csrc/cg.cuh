@@ -95,7 +95,7 @@ __device__ __forceinline__ void cg_scalars(CgCtl* c, double rz, double rr, bool 
   c->rz = rz;
   c->state = state;
   c->rel = rel;
-  *(volatile CgReport*)c->report = (unsigned long long)c->it * 8 + state;
+  if (c->report) *(volatile CgReport*)c->report = (unsigned long long)c->it * 8 + state;
 }
 
 }  // namespace pdb
