@@ -20,9 +20,10 @@ constexpr size_t kPipeMin = size_t(1) << 20;
 // Bytes that go to the driver before the ring is made: making it takes some 7
 // ms (the pinned memory, the threads) and it saves about 60 us per MB (two
 // copies of 24.6 MB: 6.7 ms by the driver, 3.8 ms through the ring around the
-// same kernels), so it has paid for itself after about as much again. A program
-// that opens a context per problem and moves a few arrays never makes it: a
-// context's first state, 2 x 7.7 MB, 17 ms, and 24 ms when the ring came with it.
+// same kernels), so it has paid for itself after about as much again. The bytes
+// count from the first of the contexts now open: a program that opens one
+// context per problem and moves a few arrays never makes the ring (a context's
+// first state, 2 x 7.7 MB, 17 ms, and 24 ms when the ring came with it).
 constexpr size_t kPipeEarned = size_t(128) << 20;
 }  // namespace
 
@@ -149,7 +150,7 @@ struct Shared {
   int users = 0;
   HostRing* ring = nullptr;
   bool failed = false;
-  size_t passed = 0;  // bytes offered since there was no ring
+  size_t passed = 0;  // bytes offered without a ring since there was no context
 };
 Shared& shared() {
   static Shared* s = new Shared();
@@ -172,7 +173,7 @@ void host_pipe_release() {
     r = s.ring;  // (no context is left that could hold a lease)
     s.ring = nullptr;
     s.failed = false;
-    if (r) s.passed = 0;
+    s.passed = 0;
   }
   delete r;
 }

@@ -5,9 +5,10 @@
 // GB/s against the link's 50. Here a few worker threads move the bytes between
 // the caller's memory and a ring of pinned slots, beside each other, the DMA
 // and the kernels. One ring and its workers serve every context of the process
-// (8 MB pinned, made once enough bytes have passed to pay for it, given back with
-// the last context); one transfer uses it at a time, and a transfer that finds it
-// taken or not made yet, is small, or has pinned memory goes to the driver.
+// (8 MB pinned, made once the open contexts have moved enough bytes to pay for it,
+// given back with the last of them); one transfer uses it at a time, and a
+// transfer that finds it taken or not made yet, is small, or has pinned memory
+// goes to the driver.
 #pragma once
 
 #include <cuda_runtime.h>

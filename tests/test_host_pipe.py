@@ -1,0 +1,89 @@
+"""The pinned transfer ring's host logic, without a device.
+
+host_pipe.cu is compiled against stand-ins for the CUDA calls it makes
+(fake_cudart.cpp: copies in host memory, events that are complete), each test
+in a process of its own:
+
+* bytes arrive whole, both ways, for sizes around the piece and the ring;
+* the ring is made once the contexts that are open have moved 128 MB, and
+  given back with the last of them: contexts one after another, each with
+  less, never make it.
+"""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "peridigm_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    nvcc = os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")
+    so = str(tmp_path_factory.mktemp("host_pipe") / "host_pipe.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread", "-I", CSRC, "-I",
+                    os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include"), "-x", "c++",
+                    os.path.join(CSRC, "host_pipe.cu"), os.path.join(HERE, "fake_cudart.cpp"), "-o", so], check=True)
+    return so
+
+
+PRELUDE = """
+import ctypes as C, os, sys, time
+import numpy as np
+L = C.CDLL(sys.argv[1])
+MADE, FREED, WAITS, SPINNING = range(4)
+
+def move(fn, dst, src):
+    return fn(C.c_void_p(dst.ctypes.data), C.c_void_p(src.ctypes.data), C.c_size_t(src.nbytes))
+
+def earn():
+    a = np.zeros(32 << 20, np.uint8)
+    b = np.zeros_like(a)
+    for _ in range(4):
+        move(L.up, b, a)
+    assert L.count(MADE) == 1
+"""
+
+
+def run(library, body, seconds=60):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(body), library], capture_output=True, text=True,
+                       timeout=seconds)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_bytes_arrive_whole(library):
+    run(library, """
+        L.open_context()
+        earn()
+        rng = np.random.default_rng(0)
+        for size in (1 << 20, (1 << 20) + 1, (8 << 20) - 3, 8 << 20, (8 << 20) + 5, 20_000_003):
+            a = rng.integers(0, 256, size, dtype=np.uint8)
+            for fn in (L.up, L.down):
+                b = np.zeros_like(a)
+                assert move(fn, b, a) == 1
+                assert np.array_equal(a, b)
+        assert move(L.up, np.zeros(1000, np.uint8), np.zeros(1000, np.uint8)) == 0  # small: the driver's
+        L.close_context()
+        assert L.count(FREED) == 1
+    """)
+
+
+def test_contexts_one_after_another_do_not_make_the_ring(library):
+    run(library, """
+        a = np.zeros(15 << 20, np.uint8)
+        b = np.zeros_like(a)
+        for _ in range(20):  # 300 MB in all, 15 to a context
+            L.open_context()
+            assert move(L.up, b, a) == 0
+            L.close_context()
+        assert L.count(MADE) == 0
+        L.open_context()  # 150 MB in one
+        got = [move(L.down, b, a) for _ in range(10)]
+        assert got == [0] * 8 + [1] * 2 and L.count(MADE) == 1
+        L.close_context()
+        assert L.count(FREED) == 1
+    """)
