@@ -1,6 +1,8 @@
 // The pinned ring and its workers (host_pipe.cuh).
 #include "host_pipe.cuh"
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <condition_variable>
 #include <cstring>
@@ -40,6 +42,7 @@ struct HostRing {
   bool recorded[kSlots] = {};  // ev[k] stands for a DMA of this lease
   bool busy[kSlots] = {};      // a job on the slot is not done
   int device = -1;             // of the events
+  const pid_t owner = getpid();  // a forked child has the ring's memory and none of its workers
   bool stop = false;
   cudaError_t error = cudaSuccess;
   std::mutex m;
@@ -175,7 +178,7 @@ void host_pipe_release() {
     s.failed = false;
     s.passed = 0;
   }
-  delete r;
+  if (r && r->owner == getpid()) delete r;
 }
 
 HostLease::HostLease(int device, const void* host, size_t bytes) {
@@ -205,7 +208,7 @@ HostLease::HostLease(int device, const void* host, size_t bytes) {
     }
     r = s.ring;
   }
-  if (!r || !r->on(device)) {
+  if (!r || r->owner != getpid() || !r->on(device)) {
     s.lease_m.unlock();
     return;
   }

@@ -7,7 +7,9 @@ in a process of its own:
 * bytes arrive whole, both ways, for sizes around the piece and the ring;
 * the ring is made once the contexts that are open have moved 128 MB, and
   given back with the last of them: contexts one after another, each with
-  less, never make it.
+  less, never make it;
+* a forked child, where the workers do not run, lets its contexts go and
+  leaves its transfers to the driver.
 """
 import os
 import shutil
@@ -84,6 +86,32 @@ def test_contexts_one_after_another_do_not_make_the_ring(library):
         L.open_context()  # 150 MB in one
         got = [move(L.down, b, a) for _ in range(10)]
         assert got == [0] * 8 + [1] * 2 and L.count(MADE) == 1
+        L.close_context()
+        assert L.count(FREED) == 1
+    """)
+
+
+def test_a_forked_child_does_without_the_workers(library):
+    run(library, """
+        L.open_context()
+        earn()
+        a, b = np.zeros(4 << 20, np.uint8), np.zeros(4 << 20, np.uint8)
+        child = os.fork()
+        if child == 0:
+            ok = move(L.up, b, a) == 0 and move(L.down, b, a) == 0
+            L.close_context()
+            os._exit(0 if ok else 1)
+        for _ in range(100):  # ten seconds
+            pid, status = os.waitpid(child, os.WNOHANG)
+            if pid:
+                break
+            time.sleep(0.1)
+        else:
+            os.kill(child, 9)
+            os.waitpid(child, 0)
+            sys.exit("the child did not come back")
+        assert status == 0
+        assert move(L.up, b, a) == 1  # the parent's ring is as it was
         L.close_context()
         assert L.count(FREED) == 1
     """)
