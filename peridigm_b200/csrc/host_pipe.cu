@@ -15,7 +15,10 @@ namespace pdb {
 
 namespace {
 constexpr size_t kSlotBytes = size_t(512) << 10;
-constexpr int kSlots = 16;
+constexpr int kSlots = kHostSlots;
+// Pieces between a worker's end of the ring and the DMA's: the other half of
+// the slots is with the workers.
+constexpr size_t kInFlight = kSlots / 2;
 // Transfers below this go to the driver: the hand-over to the workers costs
 // some tens of microseconds.
 constexpr size_t kPipeMin = size_t(1) << 20;
@@ -34,7 +37,6 @@ struct HostRing {
     void* dst;
     const void* src;
     size_t bytes;
-    cudaEvent_t after;  // the slot's DMA, where there is one to wait for
     int slot;
   };
   char* pinned = nullptr;
@@ -44,7 +46,6 @@ struct HostRing {
   int device = -1;             // of the events
   const pid_t owner = getpid();  // a forked child has the ring's memory and none of its workers
   bool stop = false;
-  cudaError_t error = cudaSuccess;
   std::mutex m;
   std::condition_variable work, done;
   std::deque<Job> jobs;
@@ -67,24 +68,16 @@ struct HostRing {
   void run() {
     for (;;) {
       Job j;
-      int dev;
       {
         std::unique_lock<std::mutex> l(m);
         work.wait(l, [this] { return stop || !jobs.empty(); });
         if (jobs.empty()) return;
         j = jobs.front();
         jobs.pop_front();
-        dev = device;
       }
-      cudaError_t e = cudaSuccess;
-      if (j.after) {
-        cudaSetDevice(dev);
-        e = cudaEventSynchronize(j.after);
-      }
-      if (e == cudaSuccess) std::memcpy(j.dst, j.src, j.bytes);
+      std::memcpy(j.dst, j.src, j.bytes);
       {
         std::lock_guard<std::mutex> l(m);
-        if (e != cudaSuccess) error = e;
         busy[j.slot] = false;
       }
       done.notify_all();
@@ -98,10 +91,18 @@ struct HostRing {
     }
     work.notify_one();
   }
-  cudaError_t wait(int slot) {
+  // The slot's last piece has been copied by its worker.
+  void wait(int slot) {
     std::unique_lock<std::mutex> l(m);
     done.wait(l, [&] { return !busy[slot]; });
-    return error;
+  }
+  // The slot's last DMA is done. The calling thread waits for the device, as it
+  // does in the driver's copies; the workers only ever copy or sleep.
+  cudaError_t dma_done(int slot) {
+    if (!recorded[slot]) return cudaSuccess;
+    const cudaError_t e = cudaEventSynchronize(ev[slot]);
+    if (e == cudaSuccess) recorded[slot] = false;
+    return e;
   }
   // Nothing of a lease left in flight, in the workers or the DMA.
   void drain() {
@@ -109,10 +110,9 @@ struct HostRing {
     done.wait(l, [&] { return jobs.empty() && std::none_of(busy, busy + kSlots, [](bool b) { return b; }); });
     l.unlock();
     for (int k = 0; k < kSlots; ++k) {
-      if (recorded[k]) cudaEventSynchronize(ev[k]);
+      dma_done(k);
       recorded[k] = false;
     }
-    error = cudaSuccess;
   }
   bool on(int dev) {  // events of this device
     if (device == dev) return true;
@@ -233,19 +233,19 @@ cudaError_t HostLease::through(size_t end) {
   const size_t pieces = (up_bytes_ + kSlotBytes - 1) / kSlotBytes;
   const size_t need = std::min(pieces, (end + kSlotBytes - 1) / kSlotBytes);
   while (up_issued_ < need) {
-    // the workers run ahead by the ring; a slot's last DMA ends before it is filled again
-    for (; up_queued_ < pieces && up_queued_ < up_issued_ + kSlots; ++up_queued_) {
+    // the workers run ahead; a slot's last DMA ends before it is filled again
+    for (; up_queued_ < pieces && up_queued_ < up_issued_ + kInFlight; ++up_queued_) {
       const int k = (int)(up_queued_ % kSlots);
       const size_t off = up_queued_ * kSlotBytes;
-      ring_->push({ring_->pinned + k * kSlotBytes, up_src_ + off, std::min(kSlotBytes, up_bytes_ - off),
-                   ring_->recorded[k] ? ring_->ev[k] : nullptr, k});
+      const cudaError_t e = ring_->dma_done(k);
+      if (e != cudaSuccess) return e;
+      ring_->push({ring_->pinned + k * kSlotBytes, up_src_ + off, std::min(kSlotBytes, up_bytes_ - off), k});
     }
     const int k = (int)(up_issued_ % kSlots);
     const size_t off = up_issued_ * kSlotBytes;
-    cudaError_t e = ring_->wait(k);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(up_dst_ + off, ring_->pinned + k * kSlotBytes, std::min(kSlotBytes, up_bytes_ - off),
-                          cudaMemcpyHostToDevice, up_stream_);
+    ring_->wait(k);
+    cudaError_t e = cudaMemcpyAsync(up_dst_ + off, ring_->pinned + k * kSlotBytes, std::min(kSlotBytes, up_bytes_ - off),
+                                    cudaMemcpyHostToDevice, up_stream_);
     if (e == cudaSuccess) e = cudaEventRecord(ring_->ev[k], up_stream_);
     if (e != cudaSuccess) return e;
     ring_->recorded[k] = true;
@@ -254,30 +254,37 @@ cudaError_t HostLease::through(size_t end) {
   return cudaSuccess;
 }
 
+cudaError_t HostLease::hand_out(size_t until) {
+  for (; down_out_ < until; ++down_out_) {
+    const int k = (int)(down_out_ % kSlots);
+    const cudaError_t e = ring_->dma_done(k);
+    if (e != cudaSuccess) return e;
+    ring_->push({down_to_[k].dst, ring_->pinned + k * kSlotBytes, down_to_[k].bytes, k});
+  }
+  return cudaSuccess;
+}
+
 cudaError_t HostLease::download(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-  for (size_t off = 0; off < bytes; off += kSlotBytes, ++down_) {
+  for (size_t off = 0; off < bytes; off += kSlotBytes) {
     const int k = (int)(down_ % kSlots);
     const size_t len = std::min(kSlotBytes, bytes - off);
-    cudaError_t e = ring_->wait(k);  // the slot's last piece has been taken out (or its upload read)
-    // (a DMA that still reads the slot for an upload comes first on its stream or is waited for here)
-    if (e == cudaSuccess && ring_->recorded[k]) e = cudaStreamWaitEvent(stream, ring_->ev[k], 0);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(ring_->pinned + k * kSlotBytes, static_cast<const char*>(src) + off, len,
-                          cudaMemcpyDeviceToHost, stream);
+    cudaError_t e = hand_out(down_ < kInFlight ? 0 : down_ - kInFlight);
+    if (e != cudaSuccess) return e;
+    ring_->wait(k);  // the slot's last piece has been taken out
+    e = cudaMemcpyAsync(ring_->pinned + k * kSlotBytes, static_cast<const char*>(src) + off, len, cudaMemcpyDeviceToHost,
+                        stream);
     if (e == cudaSuccess) e = cudaEventRecord(ring_->ev[k], stream);
     if (e != cudaSuccess) return e;
     ring_->recorded[k] = true;
-    ring_->push({static_cast<char*>(dst) + off, ring_->pinned + k * kSlotBytes, len, ring_->ev[k], k});
+    down_to_[k] = {static_cast<char*>(dst) + off, len};
+    ++down_;
   }
   return cudaSuccess;
 }
 
 cudaError_t HostLease::finish() {
-  cudaError_t e = cudaSuccess;
-  for (int k = 0; k < kSlots; ++k) {
-    const cudaError_t w = ring_->wait(k);
-    if (w != cudaSuccess) e = w;
-  }
+  const cudaError_t e = hand_out(down_);
+  for (int k = 0; k < kSlots; ++k) ring_->wait(k);
   return e;
 }
 

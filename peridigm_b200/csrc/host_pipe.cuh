@@ -22,6 +22,7 @@ void host_pipe_retain();
 void host_pipe_release();
 
 struct HostRing;
+constexpr int kHostSlots = 16;
 
 // The ring for the life of the object (of one call); false when the transfer
 // has to go to the driver.
@@ -41,7 +42,7 @@ class HostLease {
   cudaError_t through(size_t end);
 
   // Copies device bytes to host memory after the work on `stream`; the bytes
-  // are there after finish().
+  // are there after finish(). (A lease serves uploads or downloads, not both.)
   cudaError_t download(void* dst, const void* src, size_t bytes, cudaStream_t stream);
   cudaError_t finish();
 
@@ -51,7 +52,13 @@ class HostLease {
   const char* up_src_ = nullptr;
   size_t up_bytes_ = 0, up_issued_ = 0, up_queued_ = 0;  // pieces (of a slot each)
   cudaStream_t up_stream_ = nullptr;
-  size_t down_ = 0;  // pieces issued
+  struct Piece {
+    char* dst;
+    size_t bytes;
+  };
+  cudaError_t hand_out(size_t until);  // pieces before `until` to the workers, each when its DMA is done
+  size_t down_ = 0, down_out_ = 0;     // pieces issued, handed out
+  Piece down_to_[kHostSlots] = {};     // where the issued pieces go
 };
 
 }  // namespace pdb

@@ -8,6 +8,8 @@ in a process of its own:
 * the ring is made once the contexts that are open have moved 128 MB, and
   given back with the last of them: contexts one after another, each with
   less, never make it;
+* only the calling thread waits for the device: a worker that did would spin
+  beside it for as long as the kernels before a copy take;
 * a forked child, where the workers do not run, lets its contexts go and
   leaves its transfers to the driver.
 """
@@ -37,7 +39,7 @@ PRELUDE = """
 import ctypes as C, os, sys, time
 import numpy as np
 L = C.CDLL(sys.argv[1])
-MADE, FREED, WAITS, SPINNING = range(4)
+MADE, FREED, WAITS, WORKER_WAITS = range(4)
 
 def move(fn, dst, src):
     return fn(C.c_void_p(dst.ctypes.data), C.c_void_p(src.ctypes.data), C.c_size_t(src.nbytes))
@@ -88,6 +90,19 @@ def test_contexts_one_after_another_do_not_make_the_ring(library):
         assert got == [0] * 8 + [1] * 2 and L.count(MADE) == 1
         L.close_context()
         assert L.count(FREED) == 1
+    """)
+
+
+def test_the_workers_do_not_wait_for_the_device(library):
+    run(library, """
+        L.open_context()
+        earn()
+        a = np.arange(40_000_001, dtype=np.uint8)
+        for fn in (L.up, L.down):
+            b = np.zeros_like(a)
+            assert move(fn, b, a) == 1 and np.array_equal(a, b)
+        assert L.count(WAITS) > 0 and L.count(WORKER_WAITS) == 0
+        L.close_context()
     """)
 
 
