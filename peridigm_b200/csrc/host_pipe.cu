@@ -19,17 +19,14 @@ constexpr int kSlots = kHostSlots;
 // Pieces between a worker's end of the ring and the DMA's: the other half of
 // the slots is with the workers.
 constexpr size_t kInFlight = kSlots / 2;
-// Transfers below this go to the driver: the hand-over to the workers costs
-// some tens of microseconds.
-constexpr size_t kPipeMin = size_t(1) << 20;
 // Bytes that go to the driver before the ring is made: making it takes some 7
-// ms (the pinned memory, the threads) and it saves about 60 us per MB (two
-// copies of 24.6 MB: 6.7 ms by the driver, 3.8 ms through the ring around the
-// same kernels), so it has paid for itself after about as much again. The bytes
-// count from the first of the contexts now open: a program that opens one
-// context per problem and moves a few arrays never makes the ring (a context's
-// first state, 2 x 7.7 MB, 17 ms, and 24 ms when the ring came with it).
-constexpr size_t kPipeEarned = size_t(128) << 20;
+// ms (the pinned memory, the threads) and it saves some 36 us per MB (a force
+// from host buffers of 24.6 MB each way: 6.0 ms by the driver, 4.2 ms through the
+// ring), so it has paid for itself after about as much again. Only transfers
+// that the ring would take count, from the first of the contexts now open: a
+// program that opens one context per problem and moves a few arrays never makes
+// the ring.
+constexpr size_t kPipeEarned = size_t(192) << 20;
 }  // namespace
 
 struct HostRing {
@@ -38,6 +35,7 @@ struct HostRing {
     const void* src;
     size_t bytes;
     int slot;
+    cudaEvent_t after;  // the DMA into the slot, where the worker waits for it
   };
   char* pinned = nullptr;
   cudaEvent_t ev[kSlots] = {};
@@ -46,6 +44,7 @@ struct HostRing {
   int device = -1;             // of the events
   const pid_t owner = getpid();  // a forked child has the ring's memory and none of its workers
   bool stop = false;
+  cudaError_t error = cudaSuccess;  // of the workers' waits, for the lease
   std::mutex m;
   std::condition_variable work, done;
   std::deque<Job> jobs;
@@ -68,16 +67,24 @@ struct HostRing {
   void run() {
     for (;;) {
       Job j;
+      int dev;
       {
         std::unique_lock<std::mutex> l(m);
         work.wait(l, [this] { return stop || !jobs.empty(); });
         if (jobs.empty()) return;
         j = jobs.front();
         jobs.pop_front();
+        dev = device;
       }
-      std::memcpy(j.dst, j.src, j.bytes);
+      cudaError_t e = cudaSuccess;
+      if (j.after) {
+        cudaSetDevice(dev);
+        e = cudaEventSynchronize(j.after);
+      }
+      if (e == cudaSuccess) std::memcpy(j.dst, j.src, j.bytes);
       {
         std::lock_guard<std::mutex> l(m);
+        if (e != cudaSuccess) error = e;
         busy[j.slot] = false;
       }
       done.notify_all();
@@ -96,8 +103,11 @@ struct HostRing {
     std::unique_lock<std::mutex> l(m);
     done.wait(l, [&] { return !busy[slot]; });
   }
-  // The slot's last DMA is done. The calling thread waits for the device, as it
-  // does in the driver's copies; the workers only ever copy or sleep.
+  cudaError_t failure() {
+    std::lock_guard<std::mutex> l(m);
+    return error;
+  }
+  // The slot's last DMA is done (the calling thread waits).
   cudaError_t dma_done(int slot) {
     if (!recorded[slot]) return cudaSuccess;
     const cudaError_t e = cudaEventSynchronize(ev[slot]);
@@ -113,6 +123,7 @@ struct HostRing {
       dma_done(k);
       recorded[k] = false;
     }
+    error = cudaSuccess;
   }
   bool on(int dev) {  // events of this device
     if (device == dev) return true;
@@ -181,8 +192,8 @@ void host_pipe_release() {
   if (r && r->owner == getpid()) delete r;
 }
 
-HostLease::HostLease(int device, const void* host, size_t bytes) {
-  if (!host || bytes < kPipeMin) return;
+HostLease::HostLease(int device, const void* host, size_t bytes, size_t least) : behind_kernels_(least == kPipeBeside) {
+  if (!host || bytes < least) return;
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
@@ -239,7 +250,7 @@ cudaError_t HostLease::through(size_t end) {
       const size_t off = up_queued_ * kSlotBytes;
       const cudaError_t e = ring_->dma_done(k);
       if (e != cudaSuccess) return e;
-      ring_->push({ring_->pinned + k * kSlotBytes, up_src_ + off, std::min(kSlotBytes, up_bytes_ - off), k});
+      ring_->push({ring_->pinned + k * kSlotBytes, up_src_ + off, std::min(kSlotBytes, up_bytes_ - off), k, nullptr});
     }
     const int k = (int)(up_issued_ % kSlots);
     const size_t off = up_issued_ * kSlotBytes;
@@ -257,9 +268,12 @@ cudaError_t HostLease::through(size_t end) {
 cudaError_t HostLease::hand_out(size_t until) {
   for (; down_out_ < until; ++down_out_) {
     const int k = (int)(down_out_ % kSlots);
-    const cudaError_t e = ring_->dma_done(k);
-    if (e != cudaSuccess) return e;
-    ring_->push({down_to_[k].dst, ring_->pinned + k * kSlotBytes, down_to_[k].bytes, k});
+    if (behind_kernels_) {
+      const cudaError_t e = ring_->dma_done(k);
+      if (e != cudaSuccess) return e;
+    }
+    ring_->push({down_to_[k].dst, ring_->pinned + k * kSlotBytes, down_to_[k].bytes, k,
+                 behind_kernels_ ? nullptr : ring_->ev[k]});
   }
   return cudaSuccess;
 }
@@ -268,7 +282,8 @@ cudaError_t HostLease::download(void* dst, const void* src, size_t bytes, cudaSt
   for (size_t off = 0; off < bytes; off += kSlotBytes) {
     const int k = (int)(down_ % kSlots);
     const size_t len = std::min(kSlotBytes, bytes - off);
-    cudaError_t e = hand_out(down_ < kInFlight ? 0 : down_ - kInFlight);
+    // (alone, every piece is with a worker already)
+    cudaError_t e = hand_out(down_ < kInFlight ? 0 : std::max(down_out_, down_ - kInFlight));
     if (e != cudaSuccess) return e;
     ring_->wait(k);  // the slot's last piece has been taken out
     e = cudaMemcpyAsync(ring_->pinned + k * kSlotBytes, static_cast<const char*>(src) + off, len, cudaMemcpyDeviceToHost,
@@ -278,14 +293,15 @@ cudaError_t HostLease::download(void* dst, const void* src, size_t bytes, cudaSt
     ring_->recorded[k] = true;
     down_to_[k] = {static_cast<char*>(dst) + off, len};
     ++down_;
+    if (!behind_kernels_) hand_out(down_);
   }
   return cudaSuccess;
 }
 
 cudaError_t HostLease::finish() {
-  const cudaError_t e = hand_out(down_);
+  cudaError_t e = hand_out(down_);
   for (int k = 0; k < kSlots; ++k) ring_->wait(k);
-  return e;
+  return e != cudaSuccess ? e : ring_->failure();
 }
 
 }  // namespace pdb

@@ -2622,7 +2622,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
       const int nk = (int)((n + per - 1) / per);
       // (pageable memory through the ring, a chunk when its turn comes: the
       // kernels of the chunks before run meanwhile; else all chunks at once)
-      HostLease lease(c->device, sp.y_host, 3 * (size_t)n * sizeof(double));
+      HostLease lease(c->device, sp.y_host, 3 * (size_t)n * sizeof(double), kPipeBeside);
       auto up = [&](int k) -> cudaError_t {
         const int64_t i0 = k * per, i1 = std::min(n, i0 + per);
         if (lease)
@@ -2685,7 +2685,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
                                                                   c->pt.p, E, soff, c->hp.p, c->influence, i0);
         TRY_CUDA(cudaEventRecord(c->chunk_ev[k], c->stream));
       }
-      HostLease lease(c->device, sp.f_host, 3 * (size_t)n * sizeof(double));
+      HostLease lease(c->device, sp.f_host, 3 * (size_t)n * sizeof(double), kPipeBeside);
       for (int64_t i0 = 0, k = 0; i0 < n; i0 += per, ++k) {
         const int64_t i1 = std::min(n, i0 + per);
         TRY_CUDA(cudaStreamWaitEvent(c->copy_stream, c->chunk_ev[k], 0));

@@ -410,14 +410,14 @@ inline cudaError_t d2h(const pd_ctx* c, void* dst, const void* src, size_t bytes
 }
 // The same for arrays of the caller, which may be large and pageable.
 inline cudaError_t h2d_user(const pd_ctx* c, void* dst, const void* src, size_t bytes) {
-  HostLease lease(c->device, src, bytes);
+  HostLease lease(c->device, src, bytes, kPipeUpload);
   if (!lease) return h2d(c, dst, src, bytes);
   lease.upload(dst, src, bytes, c->stream);
   const cudaError_t e = lease.through(bytes);
   return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
 }
 inline cudaError_t d2h_user(const pd_ctx* c, void* dst, const void* src, size_t bytes) {
-  HostLease lease(c->device, dst, bytes);
+  HostLease lease(c->device, dst, bytes, kPipeDownload);
   if (!lease) return d2h(c, dst, src, bytes);
   const cudaError_t e = lease.download(dst, src, bytes, c->stream), w = lease.finish();
   return e != cudaSuccess ? e : w;

@@ -53,17 +53,17 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
 }
 
 // What the tests call. up and down return 1 when the transfer had the ring, 0
-// when it was left to the driver.
+// when it was left to the driver; beside: as beside kernels, else alone.
 void open_context() { pdb::host_pipe_retain(); }
 void close_context() { pdb::host_pipe_release(); }
-int up(void* dst, const void* src, size_t bytes) {
-  pdb::HostLease lease(0, src, bytes);
+int up(void* dst, const void* src, size_t bytes, int beside) {
+  pdb::HostLease lease(0, src, bytes, beside ? pdb::kPipeBeside : pdb::kPipeUpload);
   if (!lease) return 0;
   lease.upload(dst, src, bytes, nullptr);
   return lease.through(bytes) == cudaSuccess ? 1 : -1;
 }
-int down(void* dst, const void* src, size_t bytes) {
-  pdb::HostLease lease(0, dst, bytes);
+int down(void* dst, const void* src, size_t bytes, int beside) {
+  pdb::HostLease lease(0, dst, bytes, beside ? pdb::kPipeBeside : pdb::kPipeDownload);
   if (!lease) return 0;
   const cudaError_t e = lease.download(dst, src, bytes, nullptr), w = lease.finish();
   return e == cudaSuccess && w == cudaSuccess ? 1 : -1;

@@ -1,12 +1,14 @@
 """Large transfers between the device and pageable memory of the caller.
 
-Arrays of a megabyte and more go through a pinned ring by worker threads, once
-128 MB have passed in the process (a context held open here sees to that): what
-is read back is what was written, bit for bit, at sizes around the threshold,
-the pieces (512 KB) and the ring (8 MB, reused), for a force evaluated from
-host buffers against the same from device pointers, and from several threads
-at once, of which one at a time has the ring.
+Coordinates and forces of a megabyte and more (beside the kernels) and states
+and fields of 40 and 3 MB (alone) go through a pinned ring by worker threads,
+once 192 MB of such have passed in the process (a context held open here sees
+to that): what is read back is what was written, bit for bit, at sizes around
+the thresholds, the pieces (512 KB) and the ring (8 MB, reused), for a force
+evaluated from host buffers against the same from device pointers, and from
+several threads at once, of which one at a time has the ring.
 """
+import os
 import threading
 
 import numpy as np
@@ -32,12 +34,15 @@ def _context(dims, precision="split"):
 def ring():
     ctx, x = _context((101, 103, 71))
     with ctx:
-        for _ in range(4):  # 35 MB each
-            ctx.set_state(x, x)
+        before = len(os.listdir("/proc/self/task"))
+        for _ in range(6):  # 35 MB each
+            ctx.compute_force(x)
+        assert len(os.listdir("/proc/self/task")) > before  # its workers
         yield
 
 
-@pytest.mark.parametrize("dims", [(43, 127, 8), (43691, 1, 1), (65536, 1, 1), (61, 67, 83), (101, 103, 71)])
+@pytest.mark.parametrize("dims", [(43, 127, 8), (43691, 1, 1), (65536, 1, 1), (61, 67, 83), (101, 103, 71), (131_072, 1, 1),
+                                  (1_747_627, 1, 1)])
 def test_state_round_trip(dims):
     ctx, x = _context(dims)
     rng = np.random.default_rng(0)

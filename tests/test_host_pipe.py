@@ -5,11 +5,13 @@ host_pipe.cu is compiled against stand-ins for the CUDA calls it makes
 in a process of its own:
 
 * bytes arrive whole, both ways, for sizes around the piece and the ring;
-* the ring is made once the contexts that are open have moved 128 MB, and
+* the ring is made once the contexts that are open have moved 192 MB, and
   given back with the last of them: contexts one after another, each with
   less, never make it;
-* only the calling thread waits for the device: a worker that did would spin
-  beside it for as long as the kernels before a copy take;
+* a transfer alone takes the ring only at sizes where it gains by it: 40 MB
+  up, 3 MB down;
+* beside kernels only the calling thread waits for the device: a worker that
+  did would spin beside it for as long as the kernels before a copy take;
 * a forked child, where the workers do not run, lets its contexts go and
   leaves its transfers to the driver.
 """
@@ -41,13 +43,13 @@ import numpy as np
 L = C.CDLL(sys.argv[1])
 MADE, FREED, WAITS, WORKER_WAITS = range(4)
 
-def move(fn, dst, src):
-    return fn(C.c_void_p(dst.ctypes.data), C.c_void_p(src.ctypes.data), C.c_size_t(src.nbytes))
+def move(fn, dst, src, beside=1):
+    return fn(C.c_void_p(dst.ctypes.data), C.c_void_p(src.ctypes.data), C.c_size_t(src.nbytes), beside)
 
 def earn():
     a = np.zeros(32 << 20, np.uint8)
     b = np.zeros_like(a)
-    for _ in range(4):
+    for _ in range(6):
         move(L.up, b, a)
     assert L.count(MADE) == 1
 """
@@ -67,9 +69,11 @@ def test_bytes_arrive_whole(library):
         for size in (1 << 20, (1 << 20) + 1, (8 << 20) - 3, 8 << 20, (8 << 20) + 5, 20_000_003):
             a = rng.integers(0, 256, size, dtype=np.uint8)
             for fn in (L.up, L.down):
-                b = np.zeros_like(a)
-                assert move(fn, b, a) == 1
-                assert np.array_equal(a, b)
+                for beside in (1, 0):
+                    b = np.zeros_like(a)
+                    took = move(fn, b, a, beside)
+                    assert took == (beside or (fn == L.down and size >= 3 << 20))
+                    assert not took or np.array_equal(a, b)
         assert move(L.up, np.zeros(1000, np.uint8), np.zeros(1000, np.uint8)) == 0  # small: the driver's
         L.close_context()
         assert L.count(FREED) == 1
@@ -80,16 +84,33 @@ def test_contexts_one_after_another_do_not_make_the_ring(library):
     run(library, """
         a = np.zeros(15 << 20, np.uint8)
         b = np.zeros_like(a)
-        for _ in range(20):  # 300 MB in all, 15 to a context
+        for _ in range(30):  # 450 MB in all, 15 to a context
             L.open_context()
             assert move(L.up, b, a) == 0
             L.close_context()
         assert L.count(MADE) == 0
-        L.open_context()  # 150 MB in one
-        got = [move(L.down, b, a) for _ in range(10)]
-        assert got == [0] * 8 + [1] * 2 and L.count(MADE) == 1
+        L.open_context()  # 225 MB in one
+        got = [move(L.down, b, a) for _ in range(15)]
+        assert got == [0] * 12 + [1] * 3 and L.count(MADE) == 1
         L.close_context()
         assert L.count(FREED) == 1
+    """)
+
+
+def test_transfers_alone_that_the_driver_is_better_at_are_its(library):
+    run(library, """
+        L.open_context()
+        a, b = np.zeros(48 << 20, np.uint8), np.zeros(48 << 20, np.uint8)
+        for _ in range(30):  # nothing that counts towards the ring
+            assert move(L.up, b[:24 << 20], a[:24 << 20], 0) == 0
+            assert move(L.down, b[:2 << 20], a[:2 << 20], 0) == 0
+        assert L.count(MADE) == 0
+        earn()
+        for fn, least in ((L.up, 40 << 20), (L.down, 3 << 20)):
+            for size in (1 << 20, least - 1, least, 41 << 20):
+                assert move(fn, b[:size], a[:size], 0) == (size >= least)
+                assert move(fn, b[:size], a[:size], 1) == 1
+        L.close_context()
     """)
 
 
