@@ -236,7 +236,16 @@ int eval_trial(pd_ctx* c, double* f_dev, double* f_host = nullptr, bool* host_do
   PD_CUDA_TRY(c, launch_eval(c, sp, c->dmg_trial.p, host_done));
   c->trial_valid = true;
   bool broke = true;
-  const int rc = check_status(c, &broke);
+  int rc = check_status(c, &broke);
+  if (rc == PD_ERR_NONFINITE && c->precision != PD_SPLIT_FP32) {
+    // again with the built-in division, which keeps the infinity of a term that overflows
+    sp.y_host = nullptr;  // (its state is formed)
+    sp.builtin = 1;
+    PD_CUDA_TRY(c, launch_eval(c, sp, c->dmg_trial.p, host_done));
+    bool more = true;
+    rc = check_status(c, &more);
+    broke |= more;
+  }
   // passes that report breaks: LPS and linear LPS on the sliced stream, and any without damage
   const bool reports = !sp.damage_on || c->precision == PD_FP64_SLICED ||
                        (c->precision == PD_SPLIT_FP32 && c->sell && c->material_model != PD_MATERIAL_BOND_BASED);

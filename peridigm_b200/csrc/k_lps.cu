@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(kBlock, PD_F64_DIL_MINB) k_dilatation_fp64(
     int64_t n, const int64_t* __restrict__ row, const int32_t* __restrict__ col, uint8_t* __restrict__ dmg,
     const double4* __restrict__ xv, const double4* __restrict__ st, const double4* __restrict__ pt,
     const double* __restrict__ sc, const double* __restrict__ hp, int influence, int damage_on, double s_gate,
-    double4* __restrict__ ab64, double* __restrict__ theta_out, double* __restrict__ node_damage, int pair) {
+    double4* __restrict__ ab64, double* __restrict__ theta_out, double* __restrict__ node_damage, int pair, int builtin) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = g / TPO;
   const int lane = threadIdx.x & (TPO - 1);
@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(kBlock, PD_F64_DIL_MINB) k_dilatation_fp64(
     const double4 xi = xv[i];
     const double4 yi = st[i];
     const double m = pt[i].x;
-    const bool m_in = root_in_range(m);  // m and 1/m far from the ends of the range
+    const bool m_in = !builtin && divisor_in_range(m);
     const double rm = __drcp_rn(m);
     const double s_c = damage_on ? sc[i] : -1.0;
     const double gate = damage_on ? s_gate : INFINITY;
@@ -1014,7 +1014,7 @@ __global__ void __launch_bounds__(kBlock, PD_F64_FORCE_MINB) k_force_fp64(int64_
                                                        const double4* __restrict__ ab64,
                                                        const double4* __restrict__ pt,
                                                        const double* __restrict__ hp, int influence,
-                                                       EpiArgs E) {
+                                                       EpiArgs E, int builtin) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = g / TPO;
   const int lane = threadIdx.x & (TPO - 1);
@@ -1056,7 +1056,7 @@ __global__ void __launch_bounds__(kBlock, PD_F64_FORCE_MINB) k_force_fp64(int64_
       };
       auto om_i = [&](double zeta) { return ONE ? 1.0 : omega_d(influence, zeta, hi); };
       auto om_j = [&](int k, double zeta) { return ONE ? 1.0 : omega_d(influence, zeta, hp[j[k]]); };
-      bool odd = false;
+      bool odd = builtin;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const double Y[3] = {__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z)};
@@ -1068,6 +1068,7 @@ __global__ void __launch_bounds__(kBlock, PD_F64_FORCE_MINB) k_force_fp64(int64_
         const RootD r = root_d(yy[k]);
         const double zeta = root_d(zz[k]).root, e = __dsub_rn(r.root, zeta), rd = recip_d(r.root, r.inv);
         const double ti = state(ai, om_i(zeta), zeta, e), tj = state(aj[k], om_j(k, zeta), zeta, e);
+        odd |= !recip_in_range(r.root);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           fi[k][c] = quotient_d(__dmul_rn(ti, Y[c]), r.root, rd);
@@ -1321,7 +1322,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_FORCE_MINB) k_force_f64s(
                                                                const double4* __restrict__ ab64,
                                                                const double4* __restrict__ xv,
                                                                const double4* __restrict__ pt, EpiArgs E,
-                                                               const int64_t* __restrict__ soff) {
+                                                               const int64_t* __restrict__ soff, int builtin) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t i = g / 4;
   const int lane = threadIdx.x & 3;
@@ -1340,7 +1341,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_FORCE_MINB) k_force_f64s(
         const double b = (own_live ? ai.y : 0.0) + (part_live ? aj[k].y : 0.0);
         return fma(zeta, a, __dsub_rn(dY, zeta) * b) * yj[k].w;
       };
-      bool odd = false;
+      bool odd = builtin;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const double y2 = sq3_rn(__dsub_rn(yj[k].x, yi.x), __dsub_rn(yj[k].y, yi.y), __dsub_rn(yj[k].z, yi.z));
@@ -1348,6 +1349,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_FORCE_MINB) k_force_f64s(
         yy[k] = (d[k] & kDummyBond) ? 1.0 : y2;
         odd |= !root_in_range(zz[k]) || !root_in_range(yy[k]);
         const RootD ry = root_d(yy[k]);
+        odd |= !recip_in_range(ry.root);
         w[k] = quotient_d(weight(k, root_d(zz[k]).root, ry.root), ry.root, recip_d(ry.root, ry.inv));
       }
       if (odd)
@@ -2104,7 +2106,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_verlet_small_fp64(SmallArgs A) {
     }
     sz[t * T] = zeta, sv[t * T] = V, sj[t * T] = j, sd[t * T] = d;
   }
-  const bool m_in = root_in_range(p.x);
+  const bool m_in = divisor_in_range(p.x);
   const double rm = __drcp_rn(p.x);
   const double s_c = A.damage_on ? A.sc[ic] : -1.0;
   const double gate = A.damage_on ? A.s_gate : INFINITY;
@@ -2202,6 +2204,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_verlet_small_fp64(SmallArgs A) {
         const double e = __dsub_rn(r.root, zeta[k]), rd = recip_d(r.root, r.inv);
         const double ti = __dadd_rn(__dmul_rn(ai.w, zeta[k]), __dmul_rn(ai.z, e));
         const double tj = __dadd_rn(__dmul_rn(aj[k].w, zeta[k]), __dmul_rn(aj[k].z, e));
+        odd |= !recip_in_range(r.root);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           fi[k][c] = quotient_d(__dmul_rn(ti, Y[k][c]), r.root, rd);
@@ -2585,7 +2588,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
     auto* kf = pair ? &k_force_f64s<true> : &k_force_f64s<false>;
     kf<<<grid_split(c->n, 4), kSplitBlock, 0, c->stream>>>(c->n, c->sell_col.p, c->sell_dmg.p, c->bx64.p,
                                                            c->st[c->cur].p, c->ab64.p, c->xv.p, c->pt.p, E,
-                                                           c->sell_off.p);
+                                                           c->sell_off.p, sp.builtin);
     if (ev) cudaEventRecord(ev[2], c->stream);
     return cudaGetLastError();
   }
@@ -2664,7 +2667,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
                     ipair);
   } else {
     PD_DISPATCH_TPO_ONE(tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->pt.p,
-                    c->sc.p, c->hp.p, c->influence, sp.damage_on, c->sc_gate64, c->ab64.p, c->theta.p, c->node_damage.p, ipair);
+                    c->sc.p, c->hp.p, c->influence, sp.damage_on, c->sc_gate64, c->ab64.p, c->theta.p, c->node_damage.p, ipair, sp.builtin);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -2714,7 +2717,7 @@ cudaError_t launch_eval(pd_ctx* c, const StepParams& sp, uint8_t* dmg, bool* hos
                     c->pt.p, c->hp.p, c->influence, E);
   } else {
     PD_DISPATCH_TPO_ONE(tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, dmg, c->xv.p, c->st[c->cur].p, c->ab64.p,
-                    c->pt.p, c->hp.p, c->influence, E);
+                    c->pt.p, c->hp.p, c->influence, E, sp.builtin);
   }
   if (ev) cudaEventRecord(ev[2], c->stream);
   return cudaGetLastError();
@@ -2873,7 +2876,7 @@ cudaError_t launch_fp64_eval_at(pd_ctx* c, const double4* y4, double4* ab, doubl
   if (c->n == 0) return cudaSuccess;
   const unsigned grid = grid_for(c->n, c->tpo);
   PD_DISPATCH_TPO_ONE(c->tpo, k_dilatation_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, c->pt.p,
-                      c->sc.p, c->hp.p, c->influence, 0, c->sc_gate64, ab, theta, nd, 0);
+                      c->sc.p, c->hp.p, c->influence, 0, c->sc_gate64, ab, theta, nd, 0, 0);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   EpiArgs E{};
@@ -2881,7 +2884,7 @@ cudaError_t launch_fp64_eval_at(pd_ctx* c, const double4* y4, double4* ab, doubl
   E.f_out = f_out;
   E.status = c->status.p;
   PD_DISPATCH_TPO_ONE(c->tpo, k_force_fp64, grid, c->n, c->row.p, c->col.p, c->dmg.p, c->xv.p, y4, ab, c->pt.p, c->hp.p,
-                  c->influence, E);
+                  c->influence, E, 0);
   return cudaGetLastError();
 }
 

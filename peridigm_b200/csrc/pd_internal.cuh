@@ -73,6 +73,7 @@ struct StepParams {
   // host coordinates [3n] to evaluate at, uploaded through f_out (which then
   // receives the force density), overlapped with the dilatation where it can be
   const double* y_host = nullptr;
+  int builtin = 0;  // FP64: roots and quotients by the built-in functions alone (fp64_math.cuh)
 };
 
 // EVAL_ONLY: evaluation (force out) with no integration; EVAL_ADVANCE: finish
