@@ -719,9 +719,11 @@ __global__ void __launch_bounds__(kCgSmallBlock, 1) k_cg_small(CgSmallArgs A) {
   bool held = false;
   double r = 0.0, x = 0.0, p = 0.0;
   const double4 m = A.pt[ic];
-  const double s = 3.0 * (A.ab[ic].y / m.x), V = A.xv[ic].w, rho = m.w;
+  const double V = A.xv[ic].w, rho = m.w;
+  double s = 0.0;  // (a point without bonds has q/m = 0/0, which its empty slots must not see)
   {
     const int64_t b0 = A.row[ic], b1 = A.row[ic + 1];
+    if (b1 > b0) s = 3.0 * (A.ab[ic].y / m.x);
     for (int t = 0; t < S; ++t) {
       const int64_t b = b0 + lane + t * L;
       const bool in = valid && b < b1;

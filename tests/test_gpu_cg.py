@@ -71,3 +71,21 @@ def test_iteration_limit_and_convergence(precond, modes, n):
     r0 = (r0 * np.repeat(w["vol"], 3))[free]
     metric = lambda r: np.linalg.norm(r) + 20.0 * np.abs(r).max()  # noqa: E731
     assert metric(f[free]) <= 1.01e-9 * metric(r0)
+
+
+@pytest.mark.parametrize("n", [8, 18])
+def test_a_point_without_bonds_does_not_reach_the_solve(n):
+    """Nothing of its 0/0 owner constants enters a product: the load step is that
+    of the body alone (8^3: one launch; 18^3: launch by launch)."""
+    w = workloads.qs_cube(n=n, jitter=0.05, load_steps=4)
+    alone = np.concatenate([w["x"], w["x"].max() + np.array([1.0, 1.0, 1.0])])
+    got = []
+    for x in (w["x"], alone):
+        w2 = dict(w, x=x, vol=np.full(x.size // 3, w["vol"][0]), v0=np.zeros_like(x))
+        with Context(precision="fp64") as ctx:
+            workloads.setup_context(ctx, w2)
+            st, u = _step(ctx, "none", 4000, 20, -1e-9)
+            assert st.newton_iterations > 0
+            got.append((st.cg_iterations, u[:w["x"].size]))
+    assert np.isfinite(got[1][1]).all() and abs(got[0][0] - got[1][0]) <= 0.02 * got[0][0]
+    assert np.linalg.norm(got[0][1] - got[1][1]) <= 1e-7 * np.linalg.norm(got[0][1])
