@@ -286,7 +286,11 @@ int pd_expr_eval(const char* function, double x, double y, double z, double t, d
 int pd_clear_boundary_conditions(pd_ctx* ctx);
 /* Velocity-Verlet loop of Peridigm::executeExplicit (src/core/Peridigm.cpp:1290-1593):
  * initial evaluation at t0, then nsteps steps of size dt. State stays on the
- * device; read it with pd_get_field. stats may be NULL. */
+ * device; read it with pd_get_field. stats may be NULL. PD_ERR_TIMEOUT, here
+ * and in the stepping form, when a bounded device wait ran out: the stepping
+ * run is over, and steps and solves are refused (PD_ERR_STATE) until
+ * pd_set_state has set both displacement and velocity; the bond damage is some
+ * steps ahead and has to be set too where it matters. */
 int pd_verlet_run(pd_ctx* ctx, double dt, double t0, int64_t nsteps, pd_stats* stats);
 /* Stepping form of pd_verlet_run for hosts that act between steps, e.g. the
  * halo exchange of a domain decomposition (no counterpart in the reference,

@@ -109,6 +109,7 @@ int alloc_state(pd_ctx* c) {
     PD_CUDA_TRY(c, dzero(c, b->p, b->bytes()));
   c->cur = 0;
   c->state_init = false;
+  c->state_lost = false;
   return PD_OK;
 }
 
@@ -198,6 +199,12 @@ int ensure_ready(pd_ctx* c) {
   return PD_OK;
 }
 
+int state_kept(pd_ctx* c) {
+  if (!c->state_lost) return PD_OK;
+  return fail(c, PD_ERR_STATE, "a device wait ran out in the last time steps: set displacement and velocity (and the "
+                               "bond damage) before the next steps or solve");
+}
+
 // broke (may be null): whether a sliced pass broke a bond since the last check.
 int check_status(pd_ctx* c, bool* broke = nullptr) {
   int word[2] = {0, 0};
@@ -206,11 +213,16 @@ int check_status(pd_ctx* c, bool* broke = nullptr) {
   const int st = word[0];
   if (broke) *broke = word[1] != 0;
   if (st || word[1]) PD_CUDA_TRY(c, cudaMemsetAsync(c->status.p, 0, sizeof(word), c->stream));
+  if (st & ST_TIMEOUT) {  // (in the time steps: the solves look at their own)
+    c->vrun = false;
+    c->state_lost = true;
+    return fail(c, PD_ERR_TIMEOUT, "a bounded device wait ran out in the time steps: displacement, velocity and bond "
+                                   "damage are not of one step any more");
+  }
   // a non-finite prescribed value first: it makes the next forces non-finite too
   if (st & ST_NONFINITE_BC) return fail(c, PD_ERR_NONFINITE, "NaN returned by dirichlet increment BC evaluation");
   if (st & ST_NONFINITE_FORCE) return fail(c, PD_ERR_NONFINITE, "NaN returned by force evaluation");
   if (st & ST_NONFINITE_CONTACT) return fail(c, PD_ERR_NONFINITE, "NaN returned by contact force evaluation");
-  if (st & ST_TIMEOUT) return fail(c, PD_ERR_TIMEOUT, "a bounded device wait ran out");
   if (st & ST_BAD_INDEX) return fail(c, PD_ERR_ARG, "a point index was outside the context (ignored)");
   return PD_OK;
 }
@@ -644,6 +656,7 @@ int pd_critical_time_step(pd_ctx* c, double* dt_out) {
 int pd_set_state(pd_ctx* c, const double* u, const double* v) {
   CHECK_CTX(c);
   TRY(ensure_ready(c));
+  if (!u || !v) TRY(state_kept(c));  // (a field that is left as it is)
   const size_t bytes = 3 * (size_t)c->n * sizeof(double);
   if (u) PD_CUDA_TRY(c, h2d_user(c, c->u.p, u, bytes));
   else if (!c->state_init) PD_CUDA_TRY(c, dzero(c, c->u.p, bytes));
@@ -654,6 +667,7 @@ int pd_set_state(pd_ctx* c, const double* u, const double* v) {
     PD_CUDA_TRY(c, launch_sync_state(c));
     PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   }
+  c->state_lost = false;
   c->state_init = true;
   return PD_OK;
 }
@@ -712,6 +726,7 @@ int pd_verlet_run(pd_ctx* c, double dt, double t0, int64_t nsteps, pd_stats* sta
   CHECK_CTX(c);
   if (!(dt > 0.0) || nsteps < 0) return fail(c, PD_ERR_ARG, "pd_verlet_run: dt must be positive and nsteps >= 0");
   TRY(ensure_ready(c));
+  TRY(state_kept(c));
   if (!c->state_init) TRY(pd_set_state(c, nullptr, nullptr));
   const bool contact = c->contact != nullptr;
   cudaEvent_t e0, e1;
@@ -790,6 +805,7 @@ int pd_verlet_begin(pd_ctx* c, double dt, double t0) {
   CHECK_CTX(c);
   if (!(dt > 0.0)) return fail(c, PD_ERR_ARG, "pd_verlet_begin: dt must be positive");
   TRY(ensure_ready(c));
+  TRY(state_kept(c));
   if (!c->state_init) TRY(pd_set_state(c, nullptr, nullptr));
   StepParams sp = verlet_params(c, dt, t0);
   if (!c->vbeg) PD_CUDA_TRY(c, cudaEventCreate(&c->vbeg));
@@ -895,6 +911,7 @@ int pd_qs_load_step(pd_ctx* c, double t_prev, double t_cur, const pd_qs_options*
   if (!(t_cur > t_prev) || o->preconditioner < 0 || o->preconditioner > 3 || o->max_cg_iterations <= 0 ||
       o->max_newton_iterations < 0 || !(o->cg_relative_tolerance > 0.0))
     return fail(c, PD_ERR_ARG, "pd_qs_load_step: bad options");
+  TRY(state_kept(c));
   if (!c->state_init) TRY(pd_set_state(c, nullptr, nullptr));
   return qs_load_step(c, t_prev, t_cur, o, st);
 }
@@ -906,6 +923,7 @@ int pd_implicit_run(pd_ctx* c, double dt, double t0, int64_t nsteps, const pd_im
       !(o->cg_relative_tolerance > 0.0) || o->max_newton_iterations < 0 || o->max_cg_iterations <= 0 ||
       (o->preconditioner != PD_PRECOND_NONE && o->preconditioner != PD_PRECOND_BLOCK_JACOBI))
     return fail(c, PD_ERR_ARG, "pd_implicit_run: bad options");
+  TRY(state_kept(c));
   if (!c->state_init) TRY(pd_set_state(c, nullptr, nullptr));
   return implicit_run(c, dt, t0, nsteps, o, st);
 }

@@ -21,6 +21,7 @@ struct CgCtl {
   int state;              // CgState; every kernel of a later iteration returns at once when it is not 0
   unsigned int ticket[2];  // blocks finished, of the p.q sum and of the dot products (wrap to 0)
   CgReport* report;
+  int waits;  // ST_TIMEOUT when a block of the one-launch solve gave up waiting
 };
 
 // Block sums of NV values per thread (T threads), a fixed tree: warp shuffles,

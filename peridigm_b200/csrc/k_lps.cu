@@ -2782,7 +2782,7 @@ cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, i
     c->sell_gen = c->dmg_gen;
   }
   if (c->small_bar.count < 1) TRY_CUDA(c->small_bar.alloc(1));
-  TRY_CUDA(dzero(c, c->small_bar.p, sizeof(unsigned int)));
+  TRY_CUDA(cudaMemsetAsync(c->small_bar.p, c->bar_fill, sizeof(unsigned int), c->stream));
   SmallArgs A{};
   A.n = c->n;
   A.row = c->row.p;

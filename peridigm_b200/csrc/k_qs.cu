@@ -1183,7 +1183,7 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   QsState* s = c->qs;
   TRY_RC(qs_geometry(c));
   if (c->small_bar.count < 1) PD_CUDA_TRY(c, c->small_bar.alloc(1));
-  PD_CUDA_TRY(c, dzero(c, c->small_bar.p, sizeof(unsigned int)));
+  PD_CUDA_TRY(c, cudaMemsetAsync(c->small_bar.p, c->bar_fill, sizeof(unsigned int), c->stream));
   PD_CUDA_TRY(c, dzero(c, s->ctl.p, s->ctl.bytes()));
   CgSmallArgs A{};
   A.n = c->n;
@@ -1207,7 +1207,7 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   A.max_it = max_it;
   A.ctl = s->ctl.p;
   A.bar = c->small_bar.p;
-  A.status = c->status.p;
+  A.status = &s->ctl.p->waits;
   void* args[] = {&A};
   PD_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void*)&k_cg_small,
                                              dim3((unsigned)((c->n * kCgLanes + threads - 1) / threads)), dim3(threads),
@@ -1216,15 +1216,15 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   PD_CUDA_TRY(c, d2h(c, &h, s->ctl.p, sizeof(h)));
   *iters = (int)h.it;
   *rel_out = h.rel;
+  if (h.waits & ST_TIMEOUT) {  // (whatever the others found: not every point has its x)
+    c->err = "a bounded device wait ran out in the CG solve";
+    return PD_ERR_TIMEOUT;
+  }
   switch (h.state) {
     case CG_CONVERGED:
     case CG_ZERO_RHS: return PD_OK;
-    case CG_MAX_ITERATIONS: return PD_ERR_NOT_CONVERGED;
     case CG_NONFINITE: c->err = "CG diverged (non-finite residual)"; return PD_ERR_NONFINITE;
-    default:
-      PD_CUDA_TRY(c, dzero(c, c->status.p, sizeof(int)));
-      c->err = "a bounded device wait ran out";
-      return PD_ERR_TIMEOUT;
+    default: return PD_ERR_NOT_CONVERGED;
   }
 }
 

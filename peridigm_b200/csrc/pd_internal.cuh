@@ -234,6 +234,10 @@ struct pd_ctx {
   const int64_t* small_row = nullptr;
   int64_t small_nb = -1;
   pdb::DBuf<unsigned int> small_bar;  // its grid barrier
+  unsigned char bar_fill = 0;         // (a test's 0x80 makes its first wait run out, grid_sync.cuh)
+  // Such a wait ran out in the time steps: the records and the bond damage are
+  // some steps ahead of u and v. No step or solve until both are set again.
+  bool state_lost = false;
 
   // boundary conditions
   std::vector<uint8_t> h_bc_mask;
