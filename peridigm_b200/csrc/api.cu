@@ -752,14 +752,9 @@ int pd_verlet_run(pd_ctx* c, double dt, double t0, int64_t nsteps, pd_stats* sta
   PD_CUDA_TRY(c, cudaEventRecord(e0, c->stream));
   PD_CUDA_TRY(c, launch_eval(c, sp, c->dmg_trial.p));
   if (nsteps > 0) c->cur ^= 1;
-  int64_t first = 1;
-  if (small_steps(c))
-    for (; first <= nsteps;) {
-      const int k = (int)std::min<int64_t>(kSmallSteps, nsteps - first + 1);
-      PD_CUDA_TRY(c, launch_small_steps(c, sp, first, k, first + k > nsteps));
-      first += k;
-    }
-  for (int64_t s = first; s <= nsteps; ++s) {
+  int64_t done = 0;
+  PD_CUDA_TRY(c, run_small_steps(c, sp, 1, nsteps, true, &done));
+  for (int64_t s = done + 1; s <= nsteps; ++s) {
     sp.step = s;
     const bool last = s == nsteps;
     sp.mode = last ? EVAL_LAST : EVAL_ADVANCE;
@@ -837,13 +832,8 @@ int pd_verlet_step(pd_ctx* c, int64_t nsteps) {
   if (nsteps < 0) return fail(c, PD_ERR_ARG, "pd_verlet_step: nsteps must be >= 0");
   StepParams sp = verlet_params(c, c->vdt, c->vt0);
   int64_t done = 0;
-  if (small_steps(c))
-    for (; done < nsteps;) {
-      const int k = (int)std::min<int64_t>(kSmallSteps, nsteps - done);
-      PD_CUDA_TRY(c, launch_small_steps(c, sp, c->vstep + 1, k, false));
-      c->vstep += k;
-      done += k;
-    }
+  PD_CUDA_TRY(c, run_small_steps(c, sp, c->vstep + 1, nsteps, false, &done));
+  c->vstep += done;
   for (int64_t k = done; k < nsteps; ++k) {
     sp.step = ++c->vstep;
     sp.mode = EVAL_ADVANCE;

@@ -2730,12 +2730,14 @@ static const void* small_kernel(const pd_ctx* c, bool pair, int threads) {
   return pair ? (const void*)&k_verlet_small_split<true> : (const void*)&k_verlet_small_split<false>;
 }
 
+constexpr int kSmallSteps = 1024;  // steps per launch
+
 // Whether steps of this context run as one cooperative launch: LPS with
 // omega = 1 on the default lane counts, nothing between the passes (contact,
 // prescribed functions, kernel timing, phantom halves), and one block per SM
 // with its bonds in shared memory (split: to about 13,000 points of 110 bonds,
 // FP64: to about 4,700).
-bool small_steps(pd_ctx* c) {
+static bool small_steps(pd_ctx* c) {
   if (c->n == 0 || c->material_model != PD_MATERIAL_LPS || c->influence != PD_INFLUENCE_ONE || c->contact ||
       c->n_bc_expr || c->ktime || c->phantoms)
     return false;
@@ -2773,8 +2775,11 @@ bool small_steps(pd_ctx* c) {
 }
 
 // Steps step0 .. step0 + nsteps - 1 (the last one of the run: last) from the
-// state of parity c->cur, on the committed damage; c->cur follows.
-cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int nsteps, bool last) {
+// state of parity c->cur, on the committed damage; c->cur follows. *taken: false
+// when the driver refuses the launch (the device can be shared in ways that the
+// queries before it do not show): nothing has run then.
+static cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int nsteps, bool last,
+                                      bool* taken) {
   const bool split = c->precision == PD_SPLIT_FP32, pair = c->sc_pair || c->dmg_asym;
   if (split && (c->sell_src != c->dmg.p || c->sell_gen != c->dmg_gen)) {
     k_sell_dmg<<<grid_for(c->n, 4), kBlock, 0, c->stream>>>(c->n, c->row.p, c->sell_off.p, c->dmg.p, c->sell_dmg.p);
@@ -2825,9 +2830,24 @@ cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, i
   const int lanes = split ? 4 : 16, T = c->small_threads;
   const void* k = small_kernel(c, pair, T);
   void* args[] = {&A};
-  TRY_CUDA(cudaLaunchCooperativeKernel(k, dim3((unsigned)((c->n * lanes + T - 1) / T)), dim3(T), args,
-                                       (size_t)c->small_bytes, c->stream));
-  c->cur ^= (nsteps - (last ? 1 : 0)) & 1;
+  *taken = cudaLaunchCooperativeKernel(k, dim3((unsigned)((c->n * lanes + T - 1) / T)), dim3(T), args,
+                                       (size_t)c->small_bytes, c->stream) == cudaSuccess;
+  if (!*taken) cudaGetLastError();  // (an earlier fault comes up again at the next call)
+  else c->cur ^= (nsteps - (last ? 1 : 0)) & 1;
+  return cudaSuccess;
+}
+
+// Of the steps step0 .. step0 + nsteps - 1 (ends: the last of them ends the run)
+// as many as run in cooperative launches, from the first on; *done says how many.
+cudaError_t run_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int64_t nsteps, bool ends, int64_t* done) {
+  *done = 0;
+  while (*done < nsteps && small_steps(c)) {
+    const int k = (int)std::min<int64_t>(kSmallSteps, nsteps - *done);
+    bool taken = false;
+    TRY_CUDA(launch_small_steps(c, sp, step0 + *done, k, ends && *done + k == nsteps, &taken));
+    if (taken) *done += k;
+    else c->small_threads = 0;  // the passes, for this bond set
+  }
   return cudaSuccess;
 }
 

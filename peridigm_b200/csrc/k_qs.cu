@@ -1175,11 +1175,14 @@ static int cg_small_threads(pd_ctx* c) {
     }
     s->small_threads = (int)threads;
     s->small_slots = (int)slots;
+    c->cg_bytes = (int)bytes;
   }
   return s->small_threads;
 }
 
-static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out, int threads) {
+// *taken: false when the driver refuses the launch; nothing has run then.
+static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int* iters, double* rel_out, int threads,
+                        bool* taken) {
   QsState* s = c->qs;
   TRY_RC(qs_geometry(c));
   if (c->small_bar.count < 1) PD_CUDA_TRY(c, c->small_bar.alloc(1));
@@ -1209,9 +1212,14 @@ static int cg_run_small(pd_ctx* c, int precond, double rel_tol, int max_it, int*
   A.bar = c->small_bar.p;
   A.status = &s->ctl.p->waits;
   void* args[] = {&A};
-  PD_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void*)&k_cg_small,
-                                             dim3((unsigned)((c->n * kCgLanes + threads - 1) / threads)), dim3(threads),
-                                             args, (size_t)threads * s->small_slots * kCgBond, c->stream));
+  *taken = cudaLaunchCooperativeKernel((const void*)&k_cg_small,
+                                       dim3((unsigned)((c->n * kCgLanes + threads - 1) / threads)), dim3(threads), args,
+                                       (size_t)c->cg_bytes, c->stream) == cudaSuccess;
+  if (!*taken) {
+    cudaGetLastError();  // (an earlier fault comes up again at the next call)
+    s->small_threads = 0;
+    return PD_OK;
+  }
   CgCtl h{};
   PD_CUDA_TRY(c, d2h(c, &h, s->ctl.p, sizeof(h)));
   *iters = (int)h.it;
@@ -1241,7 +1249,9 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
   const int use_bj = precond != PD_PRECOND_NONE;
   if (!coarse && every == 0) {
     const int threads = cg_small_threads(c);
-    if (threads) return cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, threads);
+    bool taken = false;
+    if (threads) TRY_RC(cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, threads, &taken));
+    if (taken) return PD_OK;
   }
   TRY_RC(qs_report(c));
   auto update = [&](bool first) -> int {

@@ -233,7 +233,8 @@ struct pd_ctx {
   int small_threads = -1, small_slots = 0, small_bytes = 0;
   const int64_t* small_row = nullptr;
   int64_t small_nb = -1;
-  pdb::DBuf<unsigned int> small_bar;  // its grid barrier
+  int cg_bytes = 0;                   // the same of the one-launch CG solve
+  pdb::DBuf<unsigned int> small_bar;  // the grid barrier of both
   unsigned char bar_fill = 0;         // (a test's 0x80 makes its first wait run out, grid_sync.cuh)
   // Such a wait ran out in the time steps: the records and the bond damage are
   // some steps ahead of u and v. No step or solve until both are set again.
@@ -307,9 +308,7 @@ cudaError_t launch_critical_dt_into(pd_ctx* c, double* partial, double* dt_out_d
 cudaError_t collect_kernel_times(pd_ctx* c);
 cudaError_t launch_fp64_eval_at(pd_ctx* c, const double4* y4, double4* ab, double* theta, double* nd, double* f_out);
 // Verlet steps of a small body in one cooperative launch (k_lps.cu).
-bool small_steps(pd_ctx* c);
-cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int nsteps, bool last);
-constexpr int kSmallSteps = 1024;  // steps per launch
+cudaError_t run_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int64_t nsteps, bool ends, int64_t* done);
 int ensure_ready_internal(pd_ctx* c);
 
 // quasi-static (k_qs.cu) and the learned preconditioner (k_mpnn.cu)

@@ -58,3 +58,8 @@ extern "C" int compare_fp64(int64_t n, const double* a, const double* c, unsigne
 // The arrivals of the kernels that loop in one launch are counted from one that
 // no wait's target is reached from, or from zero as ever.
 extern "C" void set_waits_run_out(pd_ctx* c, int on) { c->bar_fill = on ? 0x80 : 0; }
+
+// More shared memory than a block can have: the driver refuses the one launch
+// of the time steps and of the CG solve.
+extern "C" void ask_too_much(pd_ctx* c) { c->small_bytes = c->cg_bytes = 512 << 10; }
+extern "C" int small_step_threads(pd_ctx* c) { return c->small_threads; }

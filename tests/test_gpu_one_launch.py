@@ -1,10 +1,13 @@
-"""The bounded waits of the kernels that run a loop of a small body in one launch.
+"""What can go wrong with the kernels that run a loop of a small body in one launch.
 
-With the arrivals counted from a number that no target is reached from, the
-first wait of the time steps and of the CG solve runs out (within a second):
-the call says so, the blocks all leave, and nothing goes on with a state that is not of one step. After the
-state is set again the context steps and solves as a new one does, bit for
-bit.
+The bounded waits. With the arrivals counted from a number that no target is
+reached from, the first wait of the time steps and of the CG solve runs out
+(within a second): the call says so, the blocks all leave, and nothing goes on
+with a state that is not of one step. After the state is set again the context
+steps and solves as a new one does, bit for bit.
+
+The launch itself. Where the driver refuses it, the general passes and the
+general CG loop take the steps and the solve.
 """
 import ctypes as C
 
@@ -86,3 +89,46 @@ def test_a_solve_whose_wait_runs_out():
             assert np.array_equal(ctx.field("Displacement"), z)  # nothing of it was taken over
         _waits_run_out(ctx, 0)
         assert np.array_equal(step(ctx), want)
+
+
+@pytest.mark.parametrize("stepping", [False, True])
+@pytest.mark.parametrize("precision", ["split", "fp64"])
+def test_time_steps_whose_launch_is_refused(precision, stepping):
+    w = workloads.large_plate(30, 13, 7, pull=3.0)
+    lib = _internals.load()
+    got = []
+    for refuse in (False, True):
+        with Context(precision=precision) as ctx:
+            workloads.setup_context(ctx, w)
+            ctx.verlet_run(DT, 4)
+            assert lib.small_step_threads(ctx.h) > 0
+            if refuse:
+                lib.ask_too_much(ctx.h)
+            if stepping:
+                ctx.verlet_begin(DT)
+                ctx.verlet_step(9)
+                ctx.verlet_step(10)
+                ctx.verlet_finish()
+            else:
+                ctx.verlet_run(DT, 20)
+            assert (lib.small_step_threads(ctx.h) == 0) == refuse
+            got.append([ctx.field(k) for k in FIELDS])
+    for name, a, b in zip(FIELDS, *got):
+        assert np.array_equal(a, b), name
+
+
+@pytest.mark.parametrize("precond", ["none", "block_jacobi"])
+def test_a_solve_whose_launch_is_refused(precond):
+    w = workloads.qs_cube(n=10, jitter=0.05, load_steps=4)
+    lib = _internals.load()
+    got = []
+    for refuse in (False, True):
+        with Context(precision="fp64") as ctx:
+            workloads.setup_context(ctx, w)
+            ctx.qs_load_step(0.0, 0.25, newton_tolerance=-1e-9, preconditioner=precond, use_predictor=False)
+            if refuse:
+                lib.ask_too_much(ctx.h)
+            st = ctx.qs_load_step(0.25, 0.5, newton_tolerance=-1e-9, preconditioner=precond, use_predictor=False)
+            got.append((st.cg_iterations, ctx.field("Displacement")))
+    assert abs(got[0][0] - got[1][0]) <= 0.02 * got[0][0] + 1
+    assert np.linalg.norm(got[0][1] - got[1][1]) <= 1e-7 * np.linalg.norm(got[0][1])
