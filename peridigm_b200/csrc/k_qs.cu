@@ -92,6 +92,7 @@ struct QsState {
   DBuf<CgCtl> ctl;           // scalars and state of the running solve
   CgReport* report = nullptr;      // its progress, in a mapped page (made by the first solve that reports)
   CgReport* report_dev = nullptr;
+  bool no_report = false;          // (not to be had)
   // one-launch solve: threads per block (-1: not determined, 0: the general
   // loop) and bonds per lane, for rows of up to small_max_row bonds
   int small_threads = -1, small_slots = 0, small_max_row = -1;
@@ -874,30 +875,27 @@ static int qs_alloc(pd_ctx* c) {
   return PD_OK;
 }
 
-// The word a solve reports through. A page registered with the driver: 0.4 ms
-// for a context's first solve, where cudaHostAlloc took 1.9 to 2.6 ms; the
-// one-launch solve needs none.
-static int qs_report(pd_ctx* c) {
+// Whether there is a word for solves to report through. A page registered with
+// the driver: 0.4 ms for a context's first solve, where cudaHostAlloc took 1.9
+// to 2.6 ms; the one-launch solve needs none. Where the page cannot be had, the
+// host reads the solve's record after every iteration.
+static bool qs_report(pd_ctx* c) {
   QsState* s = c->qs;
-  if (s->report) return PD_OK;
+  if (s->report || s->no_report) return s->report != nullptr;
   constexpr size_t kPage = 4096;
   void* page = aligned_alloc(kPage, kPage);
-  if (!page) {
-    c->err = "no host memory for the CG report";
-    return PD_ERR_CUDA;
+  if (page && cudaHostRegister(page, kPage, cudaHostRegisterMapped) == cudaSuccess) {
+    if (cudaHostGetDevicePointer((void**)&s->report_dev, page, 0) == cudaSuccess) {
+      s->report = (CgReport*)page;
+      return true;
+    }
+    cudaHostUnregister(page);
   }
-  cudaError_t e = cudaHostRegister(page, kPage, cudaHostRegisterMapped);
-  if (e == cudaSuccess) {
-    e = cudaHostGetDevicePointer((void**)&s->report_dev, page, 0);
-    if (e != cudaSuccess) cudaHostUnregister(page);
-  }
-  if (e != cudaSuccess) {
-    free(page);
-    s->report_dev = nullptr;
-    PD_CUDA_TRY(c, e);
-  }
-  s->report = (CgReport*)page;
-  return PD_OK;
+  cudaGetLastError();
+  free(page);
+  s->report_dev = nullptr;
+  s->no_report = true;
+  return false;
 }
 
 const uint8_t* qs_fixed_mask(const pd_ctx* c) { return c->qs ? c->qs->fixed.p : nullptr; }
@@ -1150,6 +1148,14 @@ static int cg_wait(pd_ctx* c, long long it, CgReport* out) {
   }
 }
 
+// The same from the solve's record, after what is in the stream.
+static int cg_read(pd_ctx* c, CgReport* out) {
+  CgCtl h{};
+  PD_CUDA_TRY(c, d2h(c, &h, c->qs->ctl.p, sizeof(h)));
+  *out = (CgReport)h.it * 8 + h.state;
+  return PD_OK;
+}
+
 // Threads per block of the one-launch solve; 0 when the body's lanes are not
 // all resident with their geometry in shared memory (about 4,500 points of 110
 // bonds), or the device takes no cooperative launches.
@@ -1244,7 +1250,6 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
   QsState* s = c->qs;
   const int64_t n = c->n;
   const int every = mpnn_capture_every(c) && precond != PD_PRECOND_NONE ? mpnn_capture_every(c) : 0;
-  const int ahead = every > 0 ? 0 : kCgAhead;  // training pairs are taken at the reported iterate
   const bool coarse = s->coarse_on && precond == PD_PRECOND_TWO_LEVEL;
   const int use_bj = precond != PD_PRECOND_NONE;
   if (!coarse && every == 0) {
@@ -1253,7 +1258,8 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
     if (threads) TRY_RC(cg_run_small(c, precond, rel_tol, max_it, iters, rel_out, threads, &taken));
     if (taken) return PD_OK;
   }
-  TRY_RC(qs_report(c));
+  const bool follow = qs_report(c);
+  const int ahead = every > 0 || !follow ? 0 : kCgAhead;  // training pairs are taken at the reported iterate
   auto update = [&](bool first) -> int {
     if (coarse)
       return coarse_cg_update(c, s->w.p, s->q.p, s->x.p, s->r.p, s->z.p, s->dinv.p, s->fixed.p, s->partial.p, s->ctl.p,
@@ -1266,7 +1272,7 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
                                                             use_bj, s->partial.p, s->ctl.p);
     return PD_OK;
   };
-  *(volatile CgReport*)s->report = ~0ull;  // (no kernel of an earlier solve is in flight: each ends with a wait for the stream)
+  if (follow) *(volatile CgReport*)s->report = ~0ull;  // (no kernel of an earlier solve is in flight: each ends with a wait for the stream)
   PD_CUDA_TRY(c, cudaMemsetAsync(s->x.p, 0, s->x.bytes(), c->stream));
   k_cg_begin<<<1, 1, 0, c->stream>>>(s->ctl.p, rel_tol, max_it, s->report_dev);
   TRY_RC(update(true));
@@ -1278,12 +1284,12 @@ static int qs_cg_run(pd_ctx* c, int precond, double rel_tol, int max_it, int* it
     rc = qs_tangent(c);
     if (rc == PD_OK) rc = update(false);
     PD_CUDA_TRY(c, cudaGetLastError());
-    if (rc == PD_OK) rc = cg_wait(c, it - ahead, &at);
+    if (rc == PD_OK) rc = follow ? cg_wait(c, it - ahead, &at) : cg_read(c, &at);
     if (rc != PD_OK || (at & 7) != CG_RUNNING) break;
     if (every > 0 && it % every == 0) TRY_RC(mpnn_snapshot(c, s->r.p, s->x.p));
     k_cg_direction<<<g1(n), kQsBlock, 0, c->stream>>>(n, s->z.p, s->w.p, 0, s->ctl.p);
   }
-  if (rc == PD_OK && (at & 7) == CG_RUNNING) rc = cg_wait(c, max_it, &at);
+  if (rc == PD_OK && follow && (at & 7) == CG_RUNNING) rc = cg_wait(c, max_it, &at);
   // (the copy also ends the launches beyond the last iteration, which must not
   // reach into the next solve's report)
   const cudaError_t e = d2h(c, rel_out, &s->ctl.p->rel, sizeof(double));

@@ -8,6 +8,11 @@
   iterate: a second solve with the same limit repeats it bit for bit.
 * A converged load step leaves a force residual below the Newton tolerance.
 """
+import os
+import subprocess
+import sys
+import textwrap
+
 import numpy as np
 import pytest
 
@@ -89,3 +94,40 @@ def test_a_point_without_bonds_does_not_reach_the_solve(n):
             got.append((st.cg_iterations, u[:w["x"].size]))
     assert np.isfinite(got[1][1]).all() and abs(got[0][0] - got[1][0]) <= 0.02 * got[0][0]
     assert np.linalg.norm(got[0][1] - got[1][1]) <= 1e-7 * np.linalg.norm(got[0][1])
+
+
+def test_a_solve_without_a_page_to_report_through(tmp_path):
+    """The page cannot be had (an allocation that fails, preloaded): the host reads the solve's record instead."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    so = str(tmp_path / "no_page.so")
+    subprocess.run(["gcc", "-O1", "-fPIC", "-shared", os.path.join(here, "no_page.c"), "-o", so], check=True)
+    body = """
+        import os
+        import numpy as np
+        from peridigm_b200 import Context, PDError, workloads
+
+        w = workloads.qs_cube(n=18, jitter=0.05, load_steps=4)
+        for precond in ("none", "two_level"):
+            got = []
+            for page in (True, False):
+                os.environ.pop("PD_TEST_NO_PAGE", None)
+                with Context(precision="fp64") as ctx:
+                    workloads.setup_context(ctx, w)
+                    if not page:
+                        os.environ["PD_TEST_NO_PAGE"] = "1"
+                    st = ctx.qs_load_step(0.0, 0.25, newton_tolerance=-1e-9, preconditioner=precond,
+                                          use_predictor=False)
+                    its, u = st.cg_iterations, ctx.field("Displacement")
+                    try:  # a limit: exactly so many iterations
+                        ctx.qs_load_step(0.25, 0.5, newton_tolerance=-1e-12, max_newton=1, max_cg=7,
+                                         preconditioner=precond, use_predictor=False, stats=st)
+                    except PDError as e:
+                        assert "Newton" in str(e), e
+                    assert st.cg_iterations == its + 7
+                    got.append((its, u, ctx.field("Displacement")))
+            assert got[0][0] == got[1][0]
+            assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
+    """
+    r = subprocess.run([sys.executable, "-c", textwrap.dedent(body)], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(here), env=dict(os.environ, LD_PRELOAD=so))
+    assert r.returncode == 0, r.stdout + r.stderr
