@@ -2768,6 +2768,14 @@ static bool small_steps(pd_ctx* c) {
       return false;
     }
   }
+  // Steps that have to be taken at once for the launch to pay. It reads the
+  // whole stream into shared memory before its first step: FP64 wins from one
+  // step on (4000 points: 31.5 us against 34.1 of the passes). Split, us: one step
+  // loses (3200 points 38.4 against 33.0), two win (47.9 against 55.7), unless a
+  // block has a lot to read (11,200 points, 168 KB: 2 steps 66.4 against 60.7, 4
+  // 103.1 against 97.2, 5 117.1 against 119.6) or there is little to gain (6000
+  // points of 26 bonds: 2 steps 41.4 against 38.6, 3 43.9 against 53.7).
+  c->small_least = f64 ? 1 : bytes > 160000 ? 5 : slots < 16 && threads > 96 ? 3 : 2;
   c->small_threads = (int)threads;
   c->small_slots = (int)slots;
   c->small_bytes = (int)bytes;
@@ -2838,10 +2846,11 @@ static cudaError_t launch_small_steps(pd_ctx* c, const StepParams& sp, int64_t s
 }
 
 // Of the steps step0 .. step0 + nsteps - 1 (ends: the last of them ends the run)
-// as many as run in cooperative launches, from the first on; *done says how many.
+// as many as run in cooperative launches, from the first on; *done says how many
+// (a rest of few steps is the passes').
 cudaError_t run_small_steps(pd_ctx* c, const StepParams& sp, int64_t step0, int64_t nsteps, bool ends, int64_t* done) {
   *done = 0;
-  while (*done < nsteps && small_steps(c)) {
+  while (*done < nsteps && small_steps(c) && nsteps - *done >= c->small_least) {
     const int k = (int)std::min<int64_t>(kSmallSteps, nsteps - *done);
     bool taken = false;
     TRY_CUDA(launch_small_steps(c, sp, step0 + *done, k, ends && *done + k == nsteps, &taken));

@@ -233,6 +233,7 @@ struct pd_ctx {
   int small_threads = -1, small_slots = 0, small_bytes = 0;
   const int64_t* small_row = nullptr;
   int64_t small_nb = -1;
+  int small_least = 1;                // steps from which the launch pays
   int cg_bytes = 0;                   // the same of the one-launch CG solve
   pdb::DBuf<unsigned int> small_bar;  // the grid barrier of both
   unsigned char bar_fill = 0;         // (a test's 0x80 makes its first wait run out, grid_sync.cuh)
