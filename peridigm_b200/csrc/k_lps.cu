@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
 // Bound: latency of the gathers (64 B per bond here, 80 B in the force pass)
 // and of the FP64 chains, so resident warps count for more than bonds in
 // flight per lane: one bond per batch and 4 blocks per SM (64 registers) is the
-// fastest. 131x97x21 points, 27.5 M bonds: dilatation 318 -> 230 us, force
+// fastest. 131x97x21 points, 27.5 M bonds: dilatation 318 -> 224 us, force
 // 522 -> 293 us (2 bonds per batch 248 and 399 us; 5 blocks 255 and 396 us).
 #ifndef PD_F64_DIL_BATCH
 #define PD_F64_DIL_BATCH 1
@@ -770,6 +770,14 @@ __global__ void __launch_bounds__(kBlock, PD_F64_DIL_MINB) k_dilatation_fp64(
 #pragma unroll
       for (int k = 0; k < K; ++k) d[k] = dn[k], j[k] = jn[k];
       next(b + K * TPO);
+      // A broken bond gathers nothing (its byte is here already, read a batch
+      // ahead): 234 -> 224 us at 131x97x21 points, 94 -> 60 us where all bonds of
+      // 100,000 points are broken. Not in the force pass, whose gathers
+      // would wait for the byte: 301 -> 324 us.
+      if (K == 1 && (d[0] & 3) == 3) {
+        ++broken;
+        continue;
+      }
       double4 xj[K], yj[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) xj[k] = ld_f64x4_nc(xv + j[k]), yj[k] = ld_f64x4_nc(st + j[k]);
