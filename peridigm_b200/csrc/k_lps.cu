@@ -352,8 +352,13 @@ __device__ __forceinline__ Rec8 ld_rec_u(const Rec8* p) {
 // read-only path (no record written by the kernel), (2) slots 0-5 only.
 // Tells the host that a bond broke, once per warp that broke one and only
 // while nobody has (a store for each of 10 M bonds that broke at once took the
-// pass from 70 to 245 us). Every lane calls it.
-__device__ __forceinline__ void report_break(bool tore, int* broke) {
+// pass from 70 to 245 us). The lane's count of broken bonds carries the mark
+// (a flag of its own: full-bond dilatation 105 -> 114 us at the notched plate),
+// which is taken off. Every lane calls it.
+constexpr int kTore = 1 << 31;
+__device__ __forceinline__ void report_break(int& broken, int* broke) {
+  const bool tore = broken < 0;
+  broken &= ~kTore;
   if (__any_sync(0xffffffffu, tore) && (threadIdx.x & 31) == 0 && *(volatile int*)broke == 0) *(volatile int*)broke = 1;
 }
 
@@ -621,7 +626,6 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
   const bool valid = i < n;
   float th = 0.0f;
   int broken = 0;
-  bool tore = false;
   int len = 0;
   if (valid) {
     const int64_t b0 = row[i];
@@ -657,7 +661,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
         const uint8_t nd = (uint8_t)(d | (brk ? 1 : 0) | (brkp ? 2 : 0));
         *pdm = nd;
         if (SELL) cdm[r] = nd;  // the CSR copy stays canonical
-        tore = true;
+        broken |= kTore;
       }
       broken += ((d & 1) || brk) ? 1 : 0;
       float wv = uj.v[5];  // V_j
@@ -677,7 +681,7 @@ __global__ void __launch_bounds__(kSplitBlock, WEIGHT ? 5 : PD_DIL_MINB) k_dilat
     else
       csr_walk<TPO, kRec>(i, lane, b0, b0 + len, col, dmg, bx3, ur, body);
   }
-  report_break(tore, broke);
+  report_break(broken, broke);
   th = group_sum<TPO>(th);
   broken = group_sum<TPO>(broken);
   if (valid && lane == 0) {
@@ -1252,7 +1256,6 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
   const bool valid = i < n;
   double th = 0.0;
   int broken = 0;
-  bool tore = false;
   int len = 0;
   if (valid) {
     const int64_t b0 = row[i];
@@ -1302,7 +1305,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
             d[k] |= (brk ? 1 : 0) | (brkp ? 2 : 0);
             pdm[k * step] = (uint8_t)d[k];
             cdm[r + 4 * k] = (uint8_t)d[k];  // the CSR copy stays canonical
-            tore = true;
+            broken |= kTore;
           }
         }
       }
@@ -1314,7 +1317,7 @@ __global__ void __launch_bounds__(kSplitBlock, PD_F64S_DIL_MINB) k_dilatation_f6
     };
     sell_walk64<false>(i, lane, soff, col, dmg, bx, st, nullptr, body);
   }
-  report_break(tore, broke);
+  report_break(broken, broke);
   th = group_sum<4>(th);
   broken = group_sum<4>(broken);
   if (valid && lane == 0) {
