@@ -100,13 +100,15 @@ __global__ void k_sorted_positions(int64_t n, const int32_t* __restrict__ sorted
   if (s < n) pos_s[s] = pos[sorted_idx[s]];
 }
 
-// Eight lanes per point over the 9 rows of 3 cells around its own: the three
+// L lanes per point over the 9 rows of 3 cells around its own: the three
 // cells of a row are one run of the sorted points, read in order. FILL = false
 // counts, FILL = true writes the row (most points have no pair and leave at
 // once). A cell is little wider than the search radius and holds a few points:
 // a warp to a point, cell by cell, had 3 of 32 lanes at work (two bodies of
-// 814,000 points: count 3.33 -> 0.75 ms, fill 3.83 -> 0.04 ms).
-template <bool FILL>
+// 814,000 points, 8 lanes: count 3.33 -> 0.75 ms, fill 3.83 -> 0.04 ms). Few
+// points with long runs leave the chip idle while eight lanes walk them: 32
+// lanes there (contact_lanes).
+template <int L, bool FILL>
 __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4* __restrict__ pos,
                                                        const double4* __restrict__ pos_s, Grid g,
                                                        const int64_t* __restrict__ cell_start,
@@ -114,9 +116,10 @@ __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4
                                                        const int64_t* __restrict__ brow,
                                                        const int32_t* __restrict__ bcol, int64_t* __restrict__ counts,
                                                        const int64_t* __restrict__ crow, int32_t* __restrict__ ccol) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-  const int lane = threadIdx.x & 7, shift = threadIdx.x & 24;
-  const unsigned group = 0xffu << shift;
+  constexpr unsigned kAll = 0xffffffffu >> (32 - L);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int lane = threadIdx.x & (L - 1), shift = threadIdx.x & (32 - L);
+  const unsigned group = kAll << shift;
   if (i >= n) return;  // the lanes of a point leave together
   if (FILL && crow[i + 1] == crow[i]) return;
   const double4 pi = pos[i];
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4
     for (int yc = max(c1 - 1, 0); yc <= min(c1 + 1, g.dims[1] - 1); ++yc) {
       const int64_t q = ((int64_t)zc * g.dims[1] + yc) * g.dims[0];
       const int64_t s0 = cell_start[q + x0], s1 = cell_start[q + x1 + 1];
-      for (int64_t s = s0; s < s1; s += 8) {
+      for (int64_t s = s0; s < s1; s += L) {
         bool hit = false;
         int32_t j = -1;
         if (s + lane < s1) {
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4
             hit = j != i && !in_row(brow, bcol, i, j);
           }
         }
-        const unsigned m = (__ballot_sync(group, hit) >> shift) & 0xffu;
+        const unsigned m = (__ballot_sync(group, hit) >> shift) & kAll;
         if (FILL) {
           if (hit) ccol[base + __popc(m & ((1u << lane) - 1u))] = j;
           base += __popc(m);
@@ -151,11 +154,29 @@ __global__ void __launch_bounds__(256) k_contact_search(int64_t n, const double4
   if (!FILL && lane == 0) counts[i] = cnt;
 }
 
-// The points with a pair (their order does not matter to the force pass).
-__global__ void k_contact_active(int64_t n, const int64_t* __restrict__ crow, int32_t* __restrict__ active,
-                                 int* __restrict__ n_active) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && crow[i + 1] > crow[i]) active[atomicAdd(n_active, 1)] = (int32_t)i;
+// The points with a pair: those of a block's 1024 points in order, so that
+// threads beside each other in the force pass have neighbors in common (64,000
+// points of 140 pairs, a step: 190 us, 202 when each warp took its own place).
+__global__ void __launch_bounds__(1024) k_contact_active(int64_t n, const int64_t* __restrict__ crow,
+                                                         int32_t* __restrict__ active, int* __restrict__ n_active) {
+  __shared__ int start[33];
+  const int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool has = i < n && crow[i + 1] > crow[i];
+  const unsigned m = __ballot_sync(0xffffffffu, has);
+  if (lane == 0) start[w] = __popc(m);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int k = 0; k < 32; ++k) {
+      const int c = start[k];
+      start[k] = total;
+      total += c;
+    }
+    start[32] = total ? atomicAdd(n_active, total) : 0;
+  }
+  __syncthreads();
+  if (has) active[start[32] + start[w] + __popc(m & ((1u << lane) - 1u))] = (int32_t)i;
 }
 
 // Where the current coordinates come from: an array y [3n], the FP64 records,
@@ -273,6 +294,15 @@ __global__ void k_pos_from_y(int64_t n, const double* y, double4* pos) {
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+// Lanes per point of the search: 32 where eight leave lanes idle or walk long
+// runs. A search of 13,800 points at 2.2 spacings takes 226 us with eight and
+// 210 with 32, of 27,000 points 252 and 259; at 3.4 spacings (110 points to a run)
+// of 1700 points 372 and 262, of 64,000 points 824 and 747.
+static int contact_lanes(int64_t n, const Grid& g) {
+  const double cells = (double)g.dims[0] * g.dims[1] * g.dims[2];
+  return n < 20000 || 3.0 * (double)n >= 64.0 * cells ? 32 : 8;
+}
+
 static int contact_search(pd_ctx* c, const double4* pos) {
   ContactState* cs = c->contact;
   const int64_t n = c->n;
@@ -303,10 +333,14 @@ static int contact_search(pd_ctx* c, const double4* pos) {
   if (rc != PD_OK) return rc;
   PD_CUDA_TRY(c, counts.reserve(n + 1));
   PD_CUDA_TRY(c, cs->pos_s.reserve(n));
-  const unsigned g1 = (unsigned)((n + 255) / 256), gw = (unsigned)((n * 8 + 255) / 256);
+  const unsigned g1 = (unsigned)((n + 255) / 256);
+  const int L = contact_lanes(n, g);
+  const unsigned gw = (unsigned)((n * L + 255) / 256);
+  auto* count = L == 32 ? &k_contact_search<32, false> : &k_contact_search<8, false>;
+  auto* fill = L == 32 ? &k_contact_search<32, true> : &k_contact_search<8, true>;
   k_sorted_positions<<<g1, 256, 0, c->stream>>>(n, idx_s.p, pos, cs->pos_s.p);
-  k_contact_search<false><<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search,
-                                                     c->row.p, c->col.p, counts.p, nullptr, nullptr);
+  count<<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search, c->row.p, c->col.p,
+                                   counts.p, nullptr, nullptr);
   PD_CUDA_TRY(c, cudaGetLastError());
   if (cs->crow.count < (size_t)(n + 1)) PD_CUDA_TRY(c, cs->crow.alloc(n + 1));
   PD_CUDA_TRY(c, cudaMemsetAsync(counts.p + n, 0, sizeof(int64_t), c->stream));
@@ -320,12 +354,12 @@ static int contact_search(pd_ctx* c, const double4* pos) {
   PD_CUDA_TRY(c, cudaMemcpyAsync(&np, cs->crow.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
   PD_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if (cs->ccol.count < (size_t)std::max<int64_t>(np, 1)) PD_CUDA_TRY(c, cs->ccol.alloc((size_t)std::max<int64_t>(np, 1) * 5 / 4 + 16));
-  k_contact_search<true><<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search,
-                                                    c->row.p, c->col.p, nullptr, cs->crow.p, cs->ccol.p);
+  fill<<<gw, 256, 0, c->stream>>>(n, pos, cs->pos_s.p, g, cell_start.p, idx_s.p, cs->r_search, c->row.p, c->col.p,
+                                  nullptr, cs->crow.p, cs->ccol.p);
   PD_CUDA_TRY(c, cs->active.reserve(n));
   PD_CUDA_TRY(c, cs->n_active.reserve(1));
   PD_CUDA_TRY(c, dzero(c, cs->n_active.p, sizeof(int)));
-  k_contact_active<<<g1, 256, 0, c->stream>>>(n, cs->crow.p, cs->active.p, cs->n_active.p);
+  k_contact_active<<<(unsigned)((n + 1023) / 1024), 1024, 0, c->stream>>>(n, cs->crow.p, cs->active.p, cs->n_active.p);
   PD_CUDA_TRY(c, cudaGetLastError());
   cs->fc_follows = false;
   cs->npairs = np;
@@ -383,7 +417,10 @@ int contact_prepare(pd_ctx* c, int64_t step) {
 
 static void launch_contact_force(pd_ctx* c, const ContactCoords& Y, const double* v, double* fc) {
   const ContactState* cs = c->contact;
-  const unsigned g = (unsigned)std::min<int64_t>((c->n + 127) / 128, 4 * 148);
+  // no more points with a pair than pairs (a grid of four blocks per SM at most:
+  // 64,000 points with 140 pairs each, 159 us a step against 145)
+  const int64_t most = std::max<int64_t>(1, std::min(c->n, cs->npairs));
+  const unsigned g = (unsigned)((most + 127) / 128);
   k_contact_force<<<g, 128, 0, c->stream>>>(cs->n_active.p, cs->active.p, cs->crow.p, cs->ccol.p, Y, v, c->xv.p,
                                             cs->kappa.p, cs->r_contact, cs->friction, fc, c->status.p);
 }
@@ -397,7 +434,15 @@ int contact_eval(pd_ctx* c) {
     PD_CUDA_TRY(c, dzero(c, c->fc.p, 3 * (size_t)c->n * sizeof(double)));
     cs->fc_follows = true;
   }
-  launch_contact_force(c, ContactCoords{nullptr, split ? nullptr : c->st[c->cur].p, c->xv.p, c->u.p}, c->v.p, c->fc.p);
+  // Coordinates formed once, by a launch of its own, pay where there are millions
+  // of pairs to form them for (a step, formed in each pair and once: 5.6 M pairs
+  // 161 and 146 us, 9 M 191 and 181; 3.3 M 156 and 159, 0.7 M 46 and 50).
+  const bool once = split && cs->npairs >= 4000000;
+  if (once)
+    k_contact_positions<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->xv.p, c->u.p, nullptr, cs->pos.p,
+                                                                               cs->y.p);
+  launch_contact_force(c, ContactCoords{once ? cs->y.p : nullptr, split ? nullptr : c->st[c->cur].p, c->xv.p, c->u.p},
+                       c->v.p, c->fc.p);
   PD_CUDA_TRY(c, cudaGetLastError());
   return PD_OK;
 }

@@ -113,3 +113,33 @@ def test_contact_force_of_points_that_left_the_list_is_zero(precision):
         assert not ctx.contact_force(x, np.zeros_like(x)).any()  # apart: no pair
         ctx.verlet_step(1)
         assert not ctx.field("Contact_Force_Density").any()
+
+
+@pytest.mark.parametrize("precision", ["split", "fp64"])
+@pytest.mark.parametrize("dims,search", [((9, 8, 7), 1.5), ((9, 8, 7), 3.4), ((31, 29, 26), 2.2), ((31, 29, 26), 3.4),
+                                         ((36, 36, 36), 3.4)])
+def test_every_point_in_many_pairs(dims, search, precision):
+    """Points of one lattice bonded to their nearest neighbors alone: the pairs of either width of the search, few and
+    many points, short and long runs of cells, and enough pairs that the coordinates are formed once. The steps'
+    contact force is that of contact_force on the same coordinates, whose pairs a k-d tree counts."""
+    from scipy.spatial import cKDTree
+
+    h = 1.0e-3
+    x, vol = workloads.lattice(*dims, h, jitter=0.03, seed=1)
+    v = np.random.default_rng(2).normal(0.0, 1.0, x.size)
+    with Context(precision=precision) as ctx:
+        ctx.set_points(x, vol)
+        ctx.set_horizons([1.3 * h])
+        ctx.build_bonds()
+        ctx.material(130.0e9, 78.0e9, 7800.0)
+        ctx.contact(search * h, 0, search * h, 1.0, 0.2)
+        fc = ctx.contact_force(x, v)
+        ctx.set_state(np.zeros_like(x), v)
+        st = ctx.verlet_run(1.0e-9, 0)
+        pairs = 2 * len(cKDTree(x.reshape(-1, 3)).query_pairs(search * h))
+        assert st["contact_pairs"] == pairs - ctx.num_bonds()
+        assert np.linalg.norm(ctx.field("Contact_Force_Density") - fc) <= 1e-12 * np.linalg.norm(fc)
+        assert np.count_nonzero(np.abs(fc.reshape(-1, 3)).max(1)) == vol.size
+    # the sum of V f over all points vanishes: every pair's two halves are there
+    total = (fc.reshape(-1, 3) * vol[:, None]).sum(0)
+    assert np.abs(total).max() <= 1e-9 * (np.abs(fc.reshape(-1, 3)) * vol[:, None]).sum()
