@@ -9,7 +9,8 @@
 namespace pdb {
 
 // Polls of one wait (each a round trip to L2, about a second in all). After
-// that the kernel sets ST_TIMEOUT and every block leaves.
+// that the block sets ST_TIMEOUT and leaves, and so do those that wait for it. (A
+// constant: with a limit from a kernel argument each barrier took 75 ns more.)
 constexpr unsigned kGridSpin = 1u << 20;
 
 // bar: blocks arrived since the launch, zero then; target: of the next barrier,

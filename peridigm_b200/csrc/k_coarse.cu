@@ -1175,7 +1175,7 @@ int coarse_build(pd_ctx* c, const double4* y, const double4* ab, const uint8_t* 
   return PD_OK;
 }
 
-// z += scale P0 Ac^-1 P0^T r on the free dofs (r double or float).
+// zc = Ac^-1 rc (ctl may be null, see k_coarse_symv).
 static void launch_symv(pd_ctx* c, const CgCtl* ctl) {
   CoarseState* s = c->coarse;
   const int nt = (s->nc + kSyT - 1) / kSyT;
@@ -1183,6 +1183,7 @@ static void launch_symv(pd_ctx* c, const CgCtl* ctl) {
   k_coarse_symv_sum<<<(unsigned)((s->nc + 31) / 32), 256, 0, c->stream>>>(s->nc, s->sypart.p, s->zc.p, ctl);
 }
 
+// z += scale P0 Ac^-1 P0^T r on the free dofs (r double or float).
 template <typename T>
 static int co_apply(pd_ctx* c, const T* r, double* z, const uint8_t* fixed, double scale) {
   CoarseState* s = c->coarse;

@@ -212,7 +212,7 @@ struct pd_ctx {
   bool sc_pair = false;
   bool dmg_asym = false;
   float sc_min = 0.0f;  // smallest critical stretch >= 0 of the points (FP32; +inf when none)
-  double sc_gate64 = 0.0;  // FP64 sliced path: the smallest s_c >= 0 times (1 - 1e-12) (+inf when none)
+  double sc_gate64 = 0.0;  // FP64 passes: the smallest s_c >= 0 times (1 - 1e-12) (+inf when none)
 
   // state
   pdb::DBuf<double4> st[2];   // FP64 path gathered coordinates

@@ -1,12 +1,13 @@
 """The conjugate-gradient loop that keeps its scalars on the device.
 
-* Tangent products of both lane counts (32 lanes per point up to 16384 points,
-  8 above) against the oracle's linearization: 1e-11 relative, the bound of
-  the tangent tests.
+* Tangent products of both lane counts (32 lanes per point up to 4096 points,
+  8 above: 16^3 is the last of the one, 17x31x8 = 4216 is of the other) against
+  the oracle's linearization: 1e-11 relative, the bound of the tangent tests.
 * The iteration limit: CG stops at exactly max_cg iterations although the host
   runs ahead of the device, and the solution is the limited one, not a later
   iterate: a second solve with the same limit repeats it bit for bit.
 * A converged load step leaves a force residual below the Newton tolerance.
+* A point without bonds, and a page that cannot be had, change nothing.
 """
 import os
 import subprocess
